@@ -7,16 +7,17 @@
 // device table of per-case descriptors (the case's HydroParams, its IBM
 // arguments, force slots and per-step series) and launches
 //
-//   side stream:  prep -> (interp -> spread -> diag) x sweeps -> commit -> forced cells
-//   main stream:  full-grid sweep of every case (lean TRT kernel)
-//   join:         cached-field refresh (fprev = fcur)
+//   direct forcing: one cluster per case (ibm_chain)
+//   side stream:    forced cells, then the cached-field refresh (fprev = fcur)
+//   main stream:    full-grid sweep of every case (lean TRT kernel), started
+//                   as soon as every cluster runs
 //
-// per step, each over the concatenation of all cases' cells, slots or
-// markers. A block never straddles two cases: each family has a table of
+// per step, the last three over the concatenation of all cases' cells or
+// slots. A block never straddles two cases: each family has a table of
 // per-case block offsets, and a block finds its case by binary search. The
-// per-case IBM early exit, the diagnostics reduction (last block of the
-// case) and the step counters are per case, so every case follows exactly
-// the sequence it would follow alone.
+// per-case IBM early exit, the diagnostics reduction and the step counters
+// are per case, so every case follows exactly the sequence it would follow
+// alone.
 #pragma once
 #include "hydro_lean.cuh"
 #include "ibm.cuh"
@@ -24,7 +25,7 @@
 namespace lbmb {
 
 constexpr int BATCH_BLOCK = 128;
-static_assert(BATCH_BLOCK == LEAN_BLOCK && BATCH_BLOCK == IBM_BLOCK, "one block size for every family");
+static_assert(BATCH_BLOCK == LEAN_BLOCK, "one block size for the cell families");
 
 struct BatchCase {
   HydroParams<float> hp;
@@ -35,7 +36,6 @@ struct BatchCase {
   Vec4<float>* fcur;
   Vec4<float>* fprev;
   IbmArgs ibm;
-  double gx, gy, gz;
   double* series_torque;  // per step
   int64_t* counter;
 };
@@ -70,44 +70,34 @@ static __global__ void __launch_bounds__(BATCH_BLOCK) batch_cells_kernel(const B
   forced_cell<Q, S, COLL_TRT, ODD>(b.hp, uint32_t(b.slot_cell[i]));
 }
 
-// u_now over the slots; the runner clears the force field before the IBM,
-// so the field at call time is zero and the new field starts from zero.
+// The direct forcing of every case, cluster k working on case k; the runner
+// clears the force field before it, so the field at call time is zero.
+// Small blocks (64 registers a thread), so that the clusters of many cases run at once: the sweep starts when the last
+// of them has.
+constexpr int BATCH_IBM_THREADS = 256;
 template <int Q, class S>
-static __global__ void __launch_bounds__(BATCH_BLOCK)
-    batch_prep_kernel(const BatchCase* cs, const int32_t* off, int ncase, int parity) {
-  const int k = batch_case(off, ncase, blockIdx.x);
-  const BatchCase& b = cs[k];
-  const int64_t i = int64_t(int(blockIdx.x) - __ldg(off + k)) * BATCH_BLOCK + threadIdx.x;
-  ibm_prep_body<Q, S>(b.ibm, i, static_cast<const S*>(b.hp.f), int64_t(b.hp.plane), b.slot_cell, b.hp.flags,
-                      b.hp.nbr, b.nx, b.ny, b.nz, parity, b.fcur, 0, b.gx, b.gy, b.gz);
-  if (i < b.ibm.ns) b.fcur[b.ibm.bslot[i]] = Vec4<float>{0.f, 0.f, 0.f, 0.f};
-}
-
-static __global__ void __launch_bounds__(BATCH_BLOCK)
-    batch_interp_kernel(const BatchCase* cs, const int32_t* off, int ncase, int sweep) {
-  const int k = batch_case(off, ncase, blockIdx.x);
-  const BatchCase& b = cs[k];
-  ibm_interp_body(b.ibm, int64_t(int(blockIdx.x) - __ldg(off + k)) * BATCH_BLOCK + threadIdx.x, sweep);
-}
-
-static __global__ void __launch_bounds__(BATCH_BLOCK) batch_spread_kernel(const BatchCase* cs, const int32_t* off, int ncase) {
-  const int k = batch_case(off, ncase, blockIdx.x);
-  ibm_spread_body(cs[k].ibm, int(blockIdx.x) - __ldg(off + k));
-}
-
-static __global__ void __launch_bounds__(BATCH_BLOCK)
-    batch_diag_kernel(const BatchCase* cs, const int32_t* off_m, const int32_t* off_s, int ncase, int sweep) {
-  const int k = batch_case(off_m, ncase, blockIdx.x);
-  const int b0 = __ldg(off_m + k), nblk = __ldg(off_m + k + 1) - b0;
-  const int nblk_spread = __ldg(off_s + k + 1) - __ldg(off_s + k);
-  ibm_diag_body(cs[k].ibm, sweep, nblk_spread, unsigned(int(blockIdx.x) - b0), unsigned(nblk));
-}
-
-static __global__ void __launch_bounds__(BATCH_BLOCK) batch_commit_kernel(const BatchCase* cs, const int32_t* off, int ncase) {
-  const int k = batch_case(off, ncase, blockIdx.x);
-  const BatchCase& b = cs[k];
-  ibm_commit_body<float>(b.ibm, int64_t(int(blockIdx.x) - __ldg(off + k)) * BATCH_BLOCK + threadIdx.x, b.fcur,
-                         b.series_torque, nullptr, nullptr, b.counter);
+static __global__ void __launch_bounds__(BATCH_IBM_THREADS, 4) batch_ibm_kernel(const BatchCase* cs, int parity, int sweeps) {
+  release_dependents();
+  int rank, ncta;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
+  const BatchCase& b = cs[int(blockIdx.x) / ncta];
+  IbmRun<S> r = {};
+  r.fb = static_cast<const S*>(b.hp.f);
+  r.pl = int64_t(b.hp.plane);
+  r.nbr = b.hp.nbr;
+  r.nx = b.nx;
+  r.ny = b.ny;
+  r.nz = b.nz;
+  r.parity = parity;
+  r.fcur = b.fcur;
+  r.nslots = b.nslots;
+  r.clear = 1;
+  r.sweeps = sweeps;
+  r.series_torque = b.series_torque;
+  r.step_counter = b.counter;
+  const IbmArgs a = b.ibm;
+  ibm_chain<Q, S, 4>(a, r, rank, ncta);
 }
 
 static __global__ void __launch_bounds__(BATCH_BLOCK) batch_fprev_kernel(const BatchCase* cs, const int32_t* off, int ncase) {

@@ -88,8 +88,9 @@ struct BodyState {
   double center[3] = {0, 0, 0}, omega[3] = {0, 0, 0};
   double scale = 1.0;
   int radius = 0;  // radius the device stencils were built for (0: none)
-  DevBuf<double> d_pos, d_weight, st_w, st_cks, cs_w, imp, mob, rmf, part_spread, part_diag;
+  DevBuf<double> d_pos, d_weight, st_w, st_cks, wsum, cs_w, imp, mob, rmf, part_spread, part_diag;
   DevBuf<int32_t> st_off, st_slot, bslot, cs_off, cs_marker;
+  DevBuf<int2> brec;
   int64_t ns = 0;
   bool empty_stencil = false;
 };
@@ -204,6 +205,7 @@ struct Engine final : EngineBase {
   DevBuf<int64_t> slot_cell;
   DevBuf<Vec4<A>> fprev, fcur;
   DevBuf<double> s_rho, s_unow, s_du, s_spread;
+  DevBuf<double4> s_urec;
   bool field_present = false;
   bool fprev_stale = false;
   // IBM
@@ -223,11 +225,11 @@ struct Engine final : EngineBase {
   int n_pair_tiles = 0;
   TileDirs tile_dirs[2];
   int tile_grid[2] = {0, 0};
-  // persistent window-kernel grid per (parity, concurrent with the IBM chain)
-  int window_grid[4] = {0, 0, 0, 0};
+  // resident blocks per SM of the window sweep per parity
+  int window_per_sm[2] = {0, 0};
   int tma_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  // persistent cp.async grid per (parity, collision, concurrent with the IBM chain)
-  int async_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  // resident blocks per SM of the cp.async sweep per (parity, collision)
+  int async_per_sm[4] = {0, 0, 0, 0};
   // reductions
   DevBuf<double> red_part, red_out;
   int red_blocks = 0;
@@ -314,7 +316,6 @@ struct Engine final : EngineBase {
 
   ~Engine() override {
     if (step_graph) cudaGraphExecDestroy(step_graph);
-    for (auto& e : apply_cache) cudaGraphExecDestroy(e.exec);
     for (auto& e : fused_cache) cudaGraphExecDestroy(e.exec);
     for (auto& g : run_graphs)
       if (g) cudaGraphExecDestroy(g);
@@ -391,8 +392,6 @@ struct Engine final : EngineBase {
       CK(cudaGraphExecDestroy(step_graph));
       step_graph = nullptr;
     }
-    for (auto& e : apply_cache) CK(cudaGraphExecDestroy(e.exec));
-    apply_cache.clear();
     drop_fused_graphs();
     drop_run_graphs();
   }
@@ -421,6 +420,7 @@ struct Engine final : EngineBase {
     grow(s_rho, size_t(slot_cap), size_t(cap));
     grow(s_unow, size_t(3 * slot_cap), size_t(3 * cap));
     grow(s_du, size_t(3 * slot_cap), size_t(3 * cap));
+    grow(s_urec, size_t(slot_cap), size_t(cap));
     grow(s_spread, size_t(3 * slot_cap), size_t(3 * cap));
     slot_cap = cap;
     invalidate_graphs();
@@ -513,27 +513,31 @@ struct Engine final : EngineBase {
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TMA_TILE, smem));
       tma_grid[slot] = int(std::max<int64_t>(1, std::min<int64_t>(ntiles, int64_t(sm_count) * std::max(per_sm, 1))));
     }
-    kern<<<unsigned(tma_grid[slot]), TMA_TILE, smem, s>>>(p, n, int(ntiles), d_err.p, omega_ptr(), wait_limit);
-    CK(cudaGetLastError());
+    launch_sweep(kern, dim3(unsigned(tma_grid[slot])), TMA_TILE, smem, s, p, n, int(ntiles), d_err.p, omega_ptr(),
+                 wait_limit);
   }
 
   // Per-thread cp.async pipeline (persistent grid). `concurrent`: the sweep
-  // of a runner step, running while the IBM chain runs on the side stream;
-  // its grid leaves async_reserve block slots free for that chain.
+  // of a runner step, running beside the direct forcing.
   template <int COLL, bool ODD, int MINB, int STAGES>
   void launch_async_mb(const HydroParams<A>& p, cudaStream_t s, bool concurrent) {
     auto kern = hydro_async_kernel<Q, S, COLL, ODD, STAGES, MINB>;
     const size_t smem = async_smem_bytes<Q, S, STAGES>();
-    const int slot = (ODD ? 1 : 0) + (COLL == COLL_CM ? 2 : 0) + (concurrent ? 4 : 0);
-    if (async_grid[slot] == 0) {
+    const int slot = (ODD ? 1 : 0) + (COLL == COLL_CM ? 2 : 0);
+    if (async_per_sm[slot] == 0) {
       CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-      int per_sm = 0;
-      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ASYNC_TILE, smem));
-      const int64_t slots = int64_t(sm_count) * std::max(per_sm, 1) - (concurrent ? async_reserve : 0);
-      async_grid[slot] = int(std::max<int64_t>(1, std::min<int64_t>(ntiles, slots)));
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&async_per_sm[slot], kern, ASYNC_TILE, smem));
+      async_per_sm[slot] = std::max(async_per_sm[slot], 1);
     }
-    kern<<<unsigned(async_grid[slot]), ASYNC_TILE, smem, s>>>(p, n, int(ntiles));
-    CK(cudaGetLastError());
+    launch_sweep(kern, dim3(persistent_grid(ntiles, async_per_sm[slot], concurrent)), ASYNC_TILE, smem, s, p, n,
+                 int(ntiles));
+  }
+  // Blocks of a persistent sweep over `work` block tiles with `per_sm`
+  // resident blocks; concurrent: beside the direct forcing, which has
+  // IBM_CLUSTER SMs to itself (and then the forced cells on them).
+  unsigned persistent_grid(int64_t work, int per_sm, bool concurrent) const {
+    const int64_t slots = int64_t(sm_count - (concurrent ? IBM_CLUSTER : 0)) * per_sm;
+    return unsigned(std::max<int64_t>(1, std::min<int64_t>(work, slots)));
   }
   template <int COLL, bool ODD>
   void launch_async(const HydroParams<A>& p, cudaStream_t s, bool concurrent) {
@@ -569,13 +573,6 @@ struct Engine final : EngineBase {
   // blocks per SM (4 = 128 registers with a 3-tile ring, 5 = 96 with 3,
   // 6 = 80 with 2); the persistent grid fills every resident slot.
   int async_minb[2] = {4, 4};
-  // Block slots the persistent cp.async grid of a runner step leaves free
-  // (out of sm_count x blocks per SM): the latency-bound IBM chain on the
-  // side stream runs in them while the sweep is resident, instead of
-  // waiting for the whole sweep (128^3 central-moment tank on B200: 227 ->
-  // 192 us per runner step with 32).
-  const int async_reserve = 32;
-
   void set_sweep_variant(int even, int odd) override {
     if (kernel_mode == LBMB_SWEEP_ASYNC) {
       auto ok = [](int v) { return v >= 4 && v <= 6; };
@@ -585,7 +582,7 @@ struct Engine final : EngineBase {
         throw Error(LBMB_ERR_UNSUPPORTED, "sweep variant: the fp64 cp.async sweep has one register budget (4)");
       async_minb[0] = even;
       async_minb[1] = odd;
-      for (int& g : async_grid) g = 0;
+      for (int& g : async_per_sm) g = 0;
       invalidate_graphs();
       return;
     }
@@ -606,7 +603,7 @@ struct Engine final : EngineBase {
         throw Error(LBMB_ERR_INVALID, "sweep variant: window resident blocks per SM must be 2, 3 or 4");
       window_minb[0] = even;
       window_minb[1] = odd;
-      for (int& g : window_grid) g = 0;
+      for (int& g : window_per_sm) g = 0;
       invalidate_graphs();
       return;
     }
@@ -632,8 +629,8 @@ struct Engine final : EngineBase {
   template <bool ODD, int MINB>
   void launch_lean_mb(const HydroParams<A>& p, cudaStream_t s) {
     if constexpr (std::is_same<A, float>::value) {
-      hydro_lean_kernel<Q, S, ODD, MINB><<<unsigned(ceil_div(n, LEAN_BLOCK)), LEAN_BLOCK, 0, s>>>(p, uint32_t(n));
-      CK(cudaGetLastError());
+      launch_sweep(hydro_lean_kernel<Q, S, ODD, MINB>, dim3(unsigned(ceil_div(n, LEAN_BLOCK))), LEAN_BLOCK, 0, s, p,
+                   uint32_t(n));
     }
   }
 
@@ -713,21 +710,14 @@ struct Engine final : EngineBase {
       constexpr int STAGES = window_stages<Q, S, MINB>();
       auto kern = hydro_window_kernel<Q, S, ODD, STAGES, COLL, MINB>;
       const size_t smem = window_smem_bytes<Q, S, STAGES>();
-      const int slot = (ODD ? 1 : 0) + (concurrent ? 2 : 0);
-      if (window_grid[slot] == 0) {
+      if (window_per_sm[ODD] == 0) {
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        int per_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TILE_CELLS, smem));
-        // in a runner step, leave the same thread slots free for the IBM
-        // chain as the cp.async grid does
-        const int64_t reserve = concurrent ? int64_t(async_reserve) * ASYNC_TILE / TILE_CELLS : 0;
-        const int64_t slots = int64_t(sm_count) * std::max(per_sm, 1) - reserve;
-        window_grid[slot] = int(std::max<int64_t>(1, std::min<int64_t>(n_tiles_active, slots)));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&window_per_sm[ODD], kern, TILE_CELLS, smem));
+        window_per_sm[ODD] = std::max(window_per_sm[ODD], 1);
       }
       if (n_tiles_active == 0) return;
-      kern<<<unsigned(window_grid[slot]), TILE_CELLS, smem, s>>>(p, tile_list.p, n_tiles_active, tile_dirs[ODD],
-                                                                 omega_ptr());
-      CK(cudaGetLastError());
+      launch_sweep(kern, dim3(persistent_grid(n_tiles_active, window_per_sm[ODD], concurrent)), TILE_CELLS, smem, s, p,
+                   tile_list.p, n_tiles_active, tile_dirs[ODD], omega_ptr());
     }
   }
   template <int COLL, bool ODD>
@@ -753,8 +743,8 @@ struct Engine final : EngineBase {
         tile_grid[ODD] = int(std::max<int64_t>(1, std::min<int64_t>(n_tiles_active, int64_t(sm_count) * std::max(per_sm, 1))));
       }
       if (n_tiles_active == 0) return;
-      kern<<<unsigned(tile_grid[ODD]), TILE_THREADS, smem, s>>>(p, tile_list.p, n_tiles_active, tile_dirs[ODD]);
-      CK(cudaGetLastError());
+      launch_sweep(kern, dim3(unsigned(tile_grid[ODD])), TILE_THREADS, smem, s, p, tile_list.p, n_tiles_active,
+                   tile_dirs[ODD]);
     }
   }
 
@@ -786,16 +776,13 @@ struct Engine final : EngineBase {
   void launch_pair_mb(const HydroParams<A>& p, cudaStream_t s, bool concurrent) {
     if constexpr (std::is_same<A, float>::value && (COLL == COLL_TRT || Q == 27)) {
       if (n_pair_tiles == 0) return;
-      // persistent warps: every resident block slot, less async_reserve in
-      // the sweep of a runner step, where the IBM chain runs beside it
+      // persistent warps: every resident block slot, less what the direct
+      // forcing takes beside the sweep of a runner step
       const int64_t need = ceil_div(n_pair_tiles, PAIR_BLOCK / 32);
       const int resident = STAGED ? std::min(MINB, pair_staged_per_sm<ODD, COLL, MINB>()) : MINB;
-      const int64_t slots = int64_t(sm_count) * resident - (concurrent ? async_reserve : 0);
-      const unsigned blocks = unsigned(std::max<int64_t>(1, std::min(need, slots)));
       const size_t smem = STAGED ? pair_staged_smem_bytes<Q>() : 0;
-      hydro_pair_kernel<Q, S, ODD, MINB, COLL, STAGED><<<blocks, PAIR_BLOCK, smem, s>>>(p, pair_list.p, n_pair_tiles,
-                                                                                         uint32_t(n));
-      CK(cudaGetLastError());
+      launch_sweep(hydro_pair_kernel<Q, S, ODD, MINB, COLL, STAGED>, dim3(persistent_grid(need, resident, concurrent)),
+                   PAIR_BLOCK, smem, s, p, pair_list.p, n_pair_tiles, uint32_t(n));
     }
   }
   template <bool ODD, int COLL>
@@ -845,12 +832,11 @@ struct Engine final : EngineBase {
         if constexpr (sizeof(S) >= 4) launch_async<COLL, ODD>(p, s, !cells);
       } else {
         const int bx = nx >= 128 ? 128 : int(ceil_div(nx, 32) * 32);
-        dim3 block(bx), grid(unsigned(ceil_div(nx, bx)), unsigned(ny), unsigned(nz));
+        const dim3 grid(unsigned(ceil_div(nx, bx)), unsigned(ny), unsigned(nz));
         if (p.uniform_force)
-          hydro_aa_kernel<Q, S, COLL, ODD, true><<<grid, block, 0, s>>>(p, omega_ptr());
+          launch_sweep(hydro_aa_kernel<Q, S, COLL, ODD, true>, grid, unsigned(bx), 0, s, p, omega_ptr());
         else
-          hydro_aa_kernel<Q, S, COLL, ODD, false><<<grid, block, 0, s>>>(p, omega_ptr());
-        CK(cudaGetLastError());
+          launch_sweep(hydro_aa_kernel<Q, S, COLL, ODD, false>, grid, unsigned(bx), 0, s, p, omega_ptr());
       }
     }
     if (cells && !p.uniform_force && nslots > 0) {
@@ -1090,12 +1076,12 @@ struct Engine final : EngineBase {
       if (cd.kind == LBMB_SWEEP_ASYNC) {
         async_minb[0] = cd.ev;
         async_minb[1] = cd.od;
-        for (int& g : async_grid) g = 0;
+        for (int& g : async_per_sm) g = 0;
       }
       if (cd.kind == LBMB_SWEEP_WINDOW) {
         window_minb[0] = cd.ev;
         window_minb[1] = cd.od;
-        for (int& g : window_grid) g = 0;
+        for (int& g : window_per_sm) g = 0;
       }
       if (cd.kind == LBMB_SWEEP_PAIR) {
         pair_minb[0] = cd.ev;
@@ -1176,8 +1162,8 @@ struct Engine final : EngineBase {
       pair_minb[0] = pe0;
       pair_minb[1] = po0;
     }
-    for (int& g : async_grid) g = 0;
-    for (int& g : window_grid) g = 0;
+    for (int& g : async_per_sm) g = 0;
+    for (int& g : window_per_sm) g = 0;
     CK(cudaMemcpyAsync(f_alloc.p, save.p, fbytes, cudaMemcpyDeviceToDevice, st));
     CK(cudaStreamSynchronize(st));
     parity = par0;
@@ -1718,7 +1704,7 @@ struct Engine final : EngineBase {
     bs->imp.alloc(size_t(3 * nm));
     bs->mob.alloc(size_t(nm));
     bs->rmf.alloc(size_t(3 * nm));
-    bs->part_diag.alloc(size_t(9 * ceil_div(nm, IBM_BLOCK)));
+    bs->part_diag.alloc(size_t(2 * 9 * ceil_div(nm, IBM_CHUNK)));
     CK(cudaStreamSynchronize(st));
     bodies[b] = std::move(bs);
     invalidate_graphs();
@@ -1797,18 +1783,25 @@ struct Engine final : EngineBase {
         fill[l]++;
         cks[l] += st_w[k];  // cell_kernel_sum in marker order (solver.rs:3107-3116)
       }
+    std::vector<double> wsum(size_t(B.nm), 0.0);
+    for (int64_t m = 0; m < B.nm; ++m)
+      for (int32_t k = st_off[m]; k < st_off[m + 1]; ++k) wsum[size_t(m)] += st_w[size_t(k)];
     std::vector<double> st_cks(st_slot.size());
     for (size_t k = 0; k < st_slot.size(); ++k) st_cks[k] = cks[local[st_slot[k]]];
     B.st_off.upload(st_off, st);
     B.st_slot.upload(st_slot, st);
     B.st_w.upload(st_w, st);
     B.st_cks.upload(st_cks, st);
+    B.wsum.upload(wsum, st);
+    std::vector<int2> brec(bslot.size());
+    for (size_t i = 0; i < bslot.size(); ++i) brec[i] = make_int2(bslot[i], int(slot_cell_h[size_t(bslot[i])]));
     B.bslot.upload(bslot, st);
+    B.brec.upload(brec, st);
     B.cs_off.upload(cs_off, st);
     B.cs_marker.upload(cs_marker, st);
     B.cs_w.upload(cs_w, st);
     B.ns = ns;
-    B.part_spread.alloc(size_t(3 * std::max<int64_t>(1, ceil_div(ns, IBM_BLOCK))));
+    B.part_spread.alloc(size_t(2 * 3 * std::max<int64_t>(1, ceil_div(ns, IBM_CHUNK))));
     B.radius = radius;
     CK(cudaStreamSynchronize(st));
   }
@@ -1822,14 +1815,17 @@ struct Engine final : EngineBase {
     a.st_slot = B.st_slot.p;
     a.st_w = B.st_w.p;
     a.st_cks = B.st_cks.p;
+    a.wsum = B.wsum.p;
     a.ns = B.ns;
     a.bslot = B.bslot.p;
+    a.brec = B.brec.p;
     a.cs_off = B.cs_off.p;
     a.cs_marker = B.cs_marker.p;
     a.cs_w = B.cs_w.p;
     a.rho = s_rho.p;
     a.u_now = s_unow.p;
     a.du = s_du.p;
+    a.urec = s_urec.p;
     a.spread = s_spread.p;
     a.imp = B.imp.p;
     a.mob = B.mob.p;
@@ -1869,60 +1865,86 @@ struct Engine final : EngineBase {
     size_t ns3, nm;
   };
 
+  // The direct forcing of one call: one cluster of IBM_CLUSTER blocks.
+  // clear: the current field is zeroed first (the call then sees no field).
   void enqueue_ibm(BodyState& B, const lbmb_ibm_config& c, double* s_torque, double* s_ff, int32_t* s_it,
-                   int64_t* counter, bool field_at_call, cudaStream_t s_ = nullptr, const IbmSave* sv = nullptr) {
-    cudaStream_t sx = s_ ? s_ : st;
-    IbmArgs a = ibm_args(B, c);
-    const unsigned gs = unsigned(std::max<int64_t>(1, ceil_div(B.ns, IBM_BLOCK)));
-    const unsigned gm = unsigned(std::max<int64_t>(1, ceil_div(B.nm, IBM_BLOCK)));
-    const uint8_t* fl = flags.p;
-    const uint32_t* nb = nbr.p;
-    const Vec4<A>* fc = fcur.p;
-    launch_pdl(ibm_prep_kernel<Q, S>, gs, sx, a, static_cast<const S*>(fp), plane,
-               static_cast<const int64_t*>(slot_cell.p), fl, nb, nx, ny, nz, parity, fc, field_at_call ? 1 : 0,
-               double(A(cfg.force[0])), double(A(cfg.force[1])), double(A(cfg.force[2])));
-    for (int s = 0; s < c.max_iterations; ++s) {
-      if (sv && nslots)
-        CK(cudaMemcpyAsync(sv->du + size_t(s) * sv->ns3 * 3, s_du.p, size_t(nslots) * 3 * sizeof(double),
-                           cudaMemcpyDeviceToDevice, sx));
-      launch_pdl(ibm_interp_kernel, gm, sx, a, s);
-      if (sv && B.nm)
-        CK(cudaMemcpyAsync(sv->imp + size_t(s) * sv->nm * 3, B.imp.p, size_t(B.nm) * 3 * sizeof(double),
-                           cudaMemcpyDeviceToDevice, sx));
-      launch_pdl(ibm_spread_kernel, gs, sx, a);
-      launch_pdl(ibm_diag_kernel, gm, sx, a, s, int(gs));
-    }
+                   int64_t* counter, bool field_at_call, bool clear, cudaStream_t s_ = nullptr,
+                   const IbmSave* sv = nullptr) {
+    const IbmArgs a = ibm_args(B, c);
+    IbmRun<S> r = {};
+    r.fb = fp;
+    r.pl = plane;
+    r.nbr = nbr.p;
+    r.nx = nx;
+    r.ny = ny;
+    r.nz = nz;
+    r.parity = parity;
+    r.fcur = fcur.p;
+    r.nslots = nslots;
+    r.field_at_call = field_at_call ? 1 : 0;
+    r.clear = clear ? 1 : 0;
+    r.sweeps = c.max_iterations;
+    r.gx = double(A(cfg.force[0]));
+    r.gy = double(A(cfg.force[1]));
+    r.gz = double(A(cfg.force[2]));
+    r.series_torque = s_torque;
+    r.series_ff = s_ff;
+    r.series_iters = s_it;
+    r.step_counter = counter;
     if (sv) {
-      if (nslots) {
-        CK(cudaMemcpyAsync(sv->rho, s_rho.p, size_t(nslots) * sizeof(double), cudaMemcpyDeviceToDevice, sx));
-        CK(cudaMemcpyAsync(sv->u, s_unow.p, size_t(nslots) * 3 * sizeof(double), cudaMemcpyDeviceToDevice, sx));
-      }
-      if (B.nm) CK(cudaMemcpyAsync(sv->mob, B.mob.p, size_t(B.nm) * sizeof(double), cudaMemcpyDeviceToDevice, sx));
+      r.sv_rho = sv->rho;
+      r.sv_u = sv->u;
+      r.sv_mob = sv->mob;
+      r.sv_du = sv->du;
+      r.sv_imp = sv->imp;
+      r.sv_slots = int64_t(sv->ns3);
     }
-    CK(cudaGetLastError());
-    launch_pdl(ibm_commit_kernel<A>, gs, sx, a, fcur.p, s_torque, s_ff, s_it, counter);
+    cudaStream_t sx = s_ ? s_ : st;
+    // one round of up to 8 x 512 entries with 8 gathers in flight, else 8 x
+    // 1024 threads with 4 (T = 128 tank: 6,186 slots)
+    if (std::max(B.ns, B.nm) <= int64_t(IBM_CLUSTER) * 512)
+      launch_cluster(ibm_chain_kernel<Q, S, 512, 8>, 1, 512, sx, a, r);
+    else
+      launch_cluster(ibm_chain_kernel<Q, S, 1024, 4>, 1, 1024, sx, a, r);
   }
 
-  // One IBM-chain kernel of IBM_BLOCK threads with programmatic stream
-  // serialization (the kernel waits for its predecessor with pdl_wait).
+  // n clusters of IBM_CLUSTER blocks.
   template <class... KArgs, class... Args>
-  void launch_pdl(void (*kernel)(KArgs...), unsigned grid, cudaStream_t s, Args... args) {
+  static void launch_cluster(void (*kernel)(KArgs...), unsigned n, unsigned threads, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(grid);
-    lc.blockDim = dim3(IBM_BLOCK);
-    lc.dynamicSmemBytes = 0;
+    lc.gridDim = dim3(n * IBM_CLUSTER);
+    lc.blockDim = dim3(threads);
     lc.stream = s;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = IBM_CLUSTER;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
     lc.attrs = at;
     lc.numAttrs = 1;
     CK(cudaLaunchKernelEx(&lc, kernel, static_cast<KArgs>(args)...));
   }
 
-  // The IBM launch sequence of apply_rotating_ibm, captured once and
-  // replayed while every kernel argument is unchanged (the key holds all of
-  // them): one graph launch instead of 2 + 3 x sweeps kernel launches.
+  // A sweep kernel, as the programmatic dependent of the direct forcing
+  // launched before it on the same stream when after_ibm is set: it starts
+  // once the cluster's blocks run (it shares no data with them).
+  bool after_ibm = false;
+  template <class... KArgs, class... Args>
+  void launch_sweep(void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid;
+    lc.blockDim = dim3(threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = after_ibm ? 1 : 0;
+    CK(cudaLaunchKernelEx(&lc, kernel, static_cast<KArgs>(args)...));
+  }
+
+  // What a captured runner step was captured with.
   struct ApplyKey {
     IbmArgs a;
     const void* f;
@@ -1931,51 +1953,10 @@ struct Engine final : EngineBase {
     int64_t parity, field_at_call, sweeps;
     double force[3];
   };
-  // Instantiated IBM graphs by key. A runner alternates between the two AA
-  // parities (and a caller may alternate bodies), so a single cached graph
-  // would be captured and instantiated again on every call.
-  struct ApplyEntry {
-    ApplyKey key;
-    cudaGraphExec_t exec;
-  };
-  std::vector<ApplyEntry> apply_cache;
-  static constexpr size_t APPLY_CACHE = 8;
-
-  // The instantiated IBM graph of one apply (captured on the main stream at
-  // first use; launched on either stream).
-  cudaGraphExec_t apply_exec(BodyState& B, const lbmb_ibm_config& c) {
-    ApplyKey k;
-    std::memset(&k, 0, sizeof(k));
-    k.a = ibm_args(B, c);
-    k.f = fp;
-    k.slots = slot_cell.p;
-    k.field = fcur.p;
-    k.parity = parity;
-    k.field_at_call = field_present ? 1 : 0;
-    k.sweeps = c.max_iterations;
-    for (int i = 0; i < 3; ++i) k.force[i] = cfg.force[i];
-    cudaGraphExec_t exec = nullptr;
-    for (auto& e : apply_cache)
-      if (std::memcmp(&k, &e.key, sizeof(k)) == 0) exec = e.exec;
-    if (!exec) {
-      if (apply_cache.size() >= APPLY_CACHE) {
-        CK(cudaGraphExecDestroy(apply_cache.front().exec));
-        apply_cache.erase(apply_cache.begin());
-      }
-      cudaGraph_t g;
-      CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      enqueue_ibm(B, c, nullptr, nullptr, nullptr, nullptr, field_present);
-      CK(cudaStreamEndCapture(st, &g));
-      CK(cudaGraphInstantiate(&exec, g, 0));
-      CK(cudaGraphDestroy(g));
-      apply_cache.push_back({k, exec});
-    }
-    return exec;
-  }
 
   void ibm_apply(int b, const lbmb_ibm_config& c, lbmb_ibm_diag* out) override {
     BodyState& B = body_for(b, c);
-    CK(cudaGraphLaunch(apply_exec(B, c), st));
+    enqueue_ibm(B, c, nullptr, nullptr, nullptr, nullptr, field_present, false);
     field_present = true;
     fprev_stale = true;
     IbmDiagDev d;
@@ -2013,17 +1994,19 @@ struct Engine final : EngineBase {
     fused_cache.clear();
   }
 
-  // The step's device work: the clear (captured form), fork, the full-grid
-  // sweep on the main stream and on the side stream the IBM apply, the
-  // diagnostics copy, the forced cells and the refresh; join. (Measured: the
-  // clear and the marker upload on the side stream instead made the
-  // per-call loop 6% slower.)
+  // The step's device work: the direct forcing (with the clear of the field
+  // in the captured form: the steady state has fprev = fcur, so a field that
+  // the clear finds uniformly zero needs no reset of the cached moments'
+  // one; with a slot on every cell the uniform check runs first), then the
+  // full-grid sweep on the main stream beside the diagnostics copy, the
+  // forced cells and the refresh on the side stream; join.
   void enqueue_runner_step(BodyState& B, const lbmb_ibm_config& c, bool captured) {
-    if (captured) enqueue_clear_device();
+    const bool full = nslots == n;
+    if (captured && full) enqueue_clear_device();
+    enqueue_ibm(B, c, nullptr, nullptr, nullptr, nullptr, false, captured && !full);
     CK(cudaEventRecord(ev_fork, st));
     CK(cudaStreamWaitEvent(st2, ev_fork, 0));
-    launch_hydro(parity, st, true, false);
-    enqueue_ibm(B, c, nullptr, nullptr, nullptr, nullptr, false, st2);
+    sweep_beside_ibm();
     CK(cudaMemcpyAsync(h_diag, d_diag.p, sizeof(IbmDiagDev), cudaMemcpyDeviceToHost, st2));
     // inside a graph, an external record node: the host waits on it
     CK(cudaEventRecordWithFlags(ev_diag, st2, captured ? cudaEventRecordExternal : cudaEventRecordDefault));
@@ -2519,20 +2502,20 @@ struct Engine final : EngineBase {
     if (k >= 0) fill_nan(run_cv.p, steps);
     int64_t launches = 0;
     auto one_step = [&](int64_t step_index) {
-      // Fork: the IBM chain (clear -> direct forcing -> forced-cell hydro)
-      // runs on the high-priority side stream while the full-grid sweep of
-      // every other cell runs on the main stream; the two touch disjoint
-      // population slots (each cell's AA read/write set is its own).
-      CK(cudaEventRecord(ev_fork, st));
-      CK(cudaStreamWaitEvent(st2, ev_fork, 0));
+      // The direct forcing (with the clear) starts first; the full-grid
+      // sweep follows on the main stream once its blocks are resident, and
+      // the forced cells wait for it on the high-priority side stream. The
+      // two touch disjoint population slots (each cell's AA read/write set
+      // is its own).
       // Solver::clear_body_force_field: the IBM field is non-uniform, so the
       // cached moments keep it (F_prev) while the new field starts at zero.
-      if (nslots) CK(cudaMemsetAsync(fcur.p, 0, size_t(nslots) * sizeof(Vec4<A>), st2));
-      enqueue_ibm(B, c, run_torque.p, run_ff.p, run_it.p, run_counter.p, false, st2);
+      enqueue_ibm(B, c, run_torque.p, run_ff.p, run_it.p, run_counter.p, false, true);
+      CK(cudaEventRecord(ev_fork, st));
+      CK(cudaStreamWaitEvent(st2, ev_fork, 0));
       field_present = true;
       fprev_stale = true;
       launch_hydro(parity, st2, false, true);
-      launch_hydro(parity, st, true, false);
+      sweep_beside_ibm();
       // cached-moment field refresh on the side stream behind the forced
       // cells, hidden by the full-grid sweep
       if (nslots) CK(cudaMemcpyAsync(fprev.p, fcur.p, size_t(nslots) * sizeof(Vec4<A>), cudaMemcpyDeviceToDevice, st2));
@@ -2682,18 +2665,30 @@ struct Engine final : EngineBase {
   // side stream, full-grid sweep on the main stream, field refresh), eager.
   void enqueue_runner_step(BodyState& B, const lbmb_ibm_config& c, double* s_torque, int64_t* counter,
                            const IbmSave* sv = nullptr) {
+    enqueue_ibm(B, c, s_torque, nullptr, nullptr, counter, false, true, st, sv);
     CK(cudaEventRecord(ev_fork, st));
     CK(cudaStreamWaitEvent(st2, ev_fork, 0));
-    if (nslots) CK(cudaMemsetAsync(fcur.p, 0, size_t(nslots) * sizeof(Vec4<A>), st2));
-    enqueue_ibm(B, c, s_torque, nullptr, nullptr, counter, false, st2, sv);
     field_present = true;
     launch_hydro(parity, st2, false, true);
-    launch_hydro(parity, st, true, false);
+    sweep_beside_ibm();
     CK(cudaEventRecord(ev_join, st2));
     CK(cudaStreamWaitEvent(st, ev_join, 0));
     parity ^= 1;
     if (nslots) CK(cudaMemcpyAsync(fprev.p, fcur.p, size_t(nslots) * sizeof(Vec4<A>), cudaMemcpyDeviceToDevice, st));
     fprev_stale = false;
+  }
+
+  // The full-grid sweep of a runner step, launched on the main stream right
+  // behind the direct forcing.
+  void sweep_beside_ibm() {
+    after_ibm = true;
+    try {
+      launch_hydro(parity, st, true, false);
+    } catch (...) {
+      after_ibm = false;
+      throw;
+    }
+    after_ibm = false;
   }
 
   void snapshot(S* out) {
@@ -2872,8 +2867,8 @@ struct Engine final : EngineBase {
     cleanup.ss = {sb, sb2};
     cleanup.es = {e_fork, e_join, e_rec[0], e_rec[1], e_bwd[0], e_bwd[1]};
     const IbmArgs a0 = ibm_args(B, c);
-    const unsigned gs = unsigned(std::max<int64_t>(1, ceil_div(B.ns, IBM_BLOCK)));
-    const unsigned gm = unsigned(std::max<int64_t>(1, ceil_div(B.nm, IBM_BLOCK)));
+    const unsigned gs = unsigned(std::max<int64_t>(1, ceil_div(B.ns, ADJ_BLOCK)));
+    const unsigned gm = unsigned(std::max<int64_t>(1, ceil_div(B.nm, ADJ_BLOCK)));
     const unsigned gc = unsigned(ceil_div(n, ADJ_BLOCK));
     // recomputation of len steps from the restored checkpoint into b
     auto recompute = [&](SegBuf& b, int64_t len) {
@@ -3093,8 +3088,8 @@ struct Batch final : BatchBase {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_fork = nullptr, ev_join = nullptr;
   std::vector<BatchCase> cases_h;
   DevBuf<BatchCase> cases;
-  DevBuf<int32_t> off_cells, off_bslots, off_slots, off_markers;
-  int nb_cells = 0, nb_bslots = 0, nb_slots = 0, nb_markers = 0;
+  DevBuf<int32_t> off_cells, off_slots;
+  int nb_cells = 0, nb_slots = 0;
   DevBuf<double> d_torque;
   DevBuf<int64_t> d_counter;
 
@@ -3128,23 +3123,16 @@ struct Batch final : BatchBase {
     CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
     CK(cudaEventCreate(&ev0));
     CK(cudaEventCreate(&ev1));
-    std::vector<int32_t> oc(1, 0), ob(1, 0), os(1, 0), om(1, 0);
+    std::vector<int32_t> oc(1, 0), os(1, 0);
     for (int k = 0; k < ncase; ++k) {
       E* e = eng[k];
-      BodyState& B = *bod[k];
       oc.push_back(oc.back() + int32_t(ceil_div(e->n, BATCH_BLOCK)));
-      ob.push_back(ob.back() + int32_t(std::max<int64_t>(1, ceil_div(B.ns, BATCH_BLOCK))));
       os.push_back(os.back() + int32_t(std::max<int64_t>(1, ceil_div(e->nslots, BATCH_BLOCK))));
-      om.push_back(om.back() + int32_t(std::max<int64_t>(1, ceil_div(B.nm, BATCH_BLOCK))));
     }
     nb_cells = oc.back();
-    nb_bslots = ob.back();
     nb_slots = os.back();
-    nb_markers = om.back();
     off_cells.upload(oc, st);
-    off_bslots.upload(ob, st);
     off_slots.upload(os, st);
-    off_markers.upload(om, st);
     cases_h.resize(size_t(ncase));
     for (int k = 0; k < ncase; ++k) {
       E* e = eng[k];
@@ -3159,7 +3147,6 @@ struct Batch final : BatchBase {
       b.fcur = e->fcur.p;
       b.fprev = e->fprev.p;
       b.ibm = e->ibm_args(*bod[size_t(k)], cfg);
-      b.gx = b.gy = b.gz = 0.0;
       b.series_torque = nullptr;
       b.counter = nullptr;
     }
@@ -3180,7 +3167,8 @@ struct Batch final : BatchBase {
 
   template <bool ODD, int MB>
   void hydro_mb() {
-    batch_hydro_kernel<Q, S, ODD, MB><<<unsigned(nb_cells), BATCH_BLOCK, 0, st>>>(cases.p, off_cells.p, ncase);
+    eng[0]->launch_sweep(batch_hydro_kernel<Q, S, ODD, MB>, dim3(unsigned(nb_cells)), BATCH_BLOCK, 0, st, cases.p,
+                         off_cells.p, ncase);
   }
   template <bool ODD>
   void hydro_par() {
@@ -3198,27 +3186,21 @@ struct Batch final : BatchBase {
 
   // One runner step of every case (runner.rs:1079-1129 per case).
   void one_step() {
+    E::launch_cluster(batch_ibm_kernel<Q, S>, unsigned(ncase), BATCH_IBM_THREADS, st, cases.p, parity,
+                      int(cfg.max_iterations));
     CK(cudaEventRecord(ev_fork, st));
     CK(cudaStreamWaitEvent(st2, ev_fork, 0));
-    batch_prep_kernel<Q, S><<<unsigned(nb_bslots), BATCH_BLOCK, 0, st2>>>(cases.p, off_bslots.p, ncase, parity);
-    for (int s = 0; s < cfg.max_iterations; ++s) {
-      batch_interp_kernel<<<unsigned(nb_markers), BATCH_BLOCK, 0, st2>>>(cases.p, off_markers.p, ncase, s);
-      batch_spread_kernel<<<unsigned(nb_bslots), BATCH_BLOCK, 0, st2>>>(cases.p, off_bslots.p, ncase);
-      batch_diag_kernel<<<unsigned(nb_markers), BATCH_BLOCK, 0, st2>>>(cases.p, off_markers.p, off_bslots.p, ncase,
-                                                                         s);
-    }
-    batch_commit_kernel<<<unsigned(nb_bslots), BATCH_BLOCK, 0, st2>>>(cases.p, off_bslots.p, ncase);
     if (parity) batch_cells_kernel<Q, S, true><<<unsigned(nb_slots), BATCH_BLOCK, 0, st2>>>(cases.p, off_slots.p, ncase);
     else batch_cells_kernel<Q, S, false><<<unsigned(nb_slots), BATCH_BLOCK, 0, st2>>>(cases.p, off_slots.p, ncase);
+    batch_fprev_kernel<<<unsigned(nb_slots), BATCH_BLOCK, 0, st2>>>(cases.p, off_slots.p, ncase);
     CK(cudaGetLastError());
+    eng[0]->after_ibm = true;
     hydro(parity);
+    eng[0]->after_ibm = false;
     CK(cudaEventRecord(ev_join, st2));
     CK(cudaStreamWaitEvent(st, ev_join, 0));
-    batch_fprev_kernel<<<unsigned(nb_slots), BATCH_BLOCK, 0, st>>>(cases.p, off_slots.p, ncase);
-    CK(cudaGetLastError());
     parity ^= 1;
   }
-
   void run(int64_t steps, double* torque, double* device_ms) override {
     if (steps < 0) invalid("steps must be >= 0");
     for (E* e : eng) e->sync();

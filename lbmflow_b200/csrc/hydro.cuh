@@ -390,18 +390,21 @@ __device__ __forceinline__ void hydro_cell(const HydroParams<typename Codec<S>::
     if (!ODD) {
       f[q] = CD::ld(fb + (q * pl + cell));
     } else {
+      // source solid: bounce-back (own slot q), or under a free-slip top
+      // the mirrored population of the partner x - (cx, cy, 0) = x +
+      // (-cx, -cy, 0); the addresses are selected, so the Q loads stay one
+      // batch
       const int o = opp(q);
-      if (GENERIC && ((mask >> o) & 1u)) {
-        // source solid: bounce-back (own slot q), or under a free-slip top
-        // the mirrored population of the partner x - (cx, cy, 0)
-        const int d = planar<Q>(o);  // x - (cx, cy, 0) = x + (-cx, -cy, 0)
-        if ((mask & NBR_SLIP) && L::cz(q) == -1 && d > 0 && !((mask >> d) & 1u))
-          f[q] = CD::ld(fb + (opp(mirror_z<Q>(q)) * pl + nidx(-L::cx(q), -L::cy(q), 0)));
-        else
-          f[q] = CD::ld(fb + (q * pl + cell));
-      } else {
-        f[q] = CD::ld(fb + (o * pl + nidx(-L::cx(q), -L::cy(q), -L::cz(q))));
+      uint32_t e = o * pl + nidx(-L::cx(q), -L::cy(q), -L::cz(q));
+      if (GENERIC) {
+        const bool wall = (mask >> o) & 1u;
+        e = wall ? q * pl + cell : e;
+        if (slips_in<Q>(q)) {
+          const bool slip = wall && (mask & NBR_SLIP) && !((mask >> planar<Q>(o)) & 1u);
+          e = slip ? opp(mirror_z<Q>(q)) * pl + nidx(-L::cx(q), -L::cy(q), 0) : e;
+        }
       }
+      f[q] = CD::ld(fb + e);
     }
   }
   // Moments (kernels.rs:627-668): rho = 1 + sum f, m = sum c f.
@@ -459,12 +462,9 @@ __device__ __forceinline__ void hydro_cell(const HydroParams<typename Codec<S>::
       const A cu = (A(L::cx(o)) * wu.x + A(L::cy(o)) * wu.y) + A(L::cz(o)) * wu.z;
       v = v + ((A(6) * A(L::w(o))) * rho) * cu;
     }
-    if (ODD && slip)
-      CD::st(fb + (mirror_z<Q>(q) * pl + nidx(L::cx(q), L::cy(q), 0)), v);
-    else if (!ODD || wall)
-      CD::st(fb + (o * pl + cell), v);
-    else
-      CD::st(fb + (q * pl + nidx(L::cx(q), L::cy(q), L::cz(q))), v);
+    uint32_t e = !ODD || wall ? o * pl + cell : q * pl + nidx(L::cx(q), L::cy(q), L::cz(q));
+    if (GENERIC && ODD && slips_out<Q>(q)) e = slip ? mirror_z<Q>(q) * pl + nidx(L::cx(q), L::cy(q), 0) : e;
+    CD::st(fb + e, v);
   }
 }
 

@@ -1,43 +1,58 @@
 // Direct-forcing IBM on the device (crates/lbm-core/src/solver.rs:3016-3282).
 //
 // The reference runs this on the host over full-grid f64 arrays. Here only
-// the stencil cells ("slots") are touched:
-//   ibm_prep_kernel    per slot:   rho, u_now from the populations
-//   ibm_interp_kernel  per marker: um, mobility, impulse, represented force
-//   ibm_spread_kernel  per slot:   spread / du gathered in marker order
-//   ibm_diag_kernel    per marker: slip statistics; the last block reduces
-//                                  all partials in block order and decides
-//                                  the early exit on the device
-//   ibm_commit_kernel  per slot:   force field += spread (storage precision)
-// Every kernel of a sweep returns at once when an earlier sweep converged,
-// so a fixed launch sequence reproduces the reference's early exit without
-// a host round trip (and can be captured in a CUDA graph).
+// the stencil cells ("slots") are touched, and one call is one kernel of one
+// thread-block cluster per body (ibm_chain), whose phases are separated by
+// hardware cluster barriers:
+//   prep     per slot:   rho, u_now from the populations (and the cleared field)
+//   impulse  per marker: um, mobility, impulse, represented force
+//   spread   per slot:   spread / du gathered in marker order
+//   slip     per marker: slip statistics of the sweep, and the impulse of the
+//                        next one (it interpolates the same velocity)
+//   commit   per slot:   force field += spread (storage precision)
+// A sweep is spread + slip; every block reduces the largest slip by itself
+// and takes the reference's early exit, so no host round trip and no launch
+// of a sweep that is not run.
+//
+// What bounds it: latency. The data (a few MB) sits in L2 and each phase is
+// two or three dependent gathers, so the time is the number of phases times
+// (gathers + barrier). Per runner step on B200, as 2 + 3 x sweeps dependent
+// kernels -> in this form: 46.3 -> 21.7 us (48 x 48 x 60 tank, 1,139 slots;
+// 20 us of it the call), 69.0 -> 36.4 us (96 x 96 x 120), 131.6 -> 86.7 us
+// (128 x 128 x 160, D3Q19); where the sweep hides it, 121.2 -> 123.1 us
+// (128 x 128 x 160, D3Q27) and 408 -> 399 us (256 x 256 x 320, fp16).
 //
 // Summation order: per slot the contributions are gathered in ascending
 // marker order (the reference's loop order), so spread, du and the cell
 // kernel sum are bit-identical to the reference; the global diagnostics
-// are fixed-order tree sums (deterministic run to run).
+// are fixed-order tree sums over 32-entry chunks (independent of the block
+// size, deterministic run to run).
 #pragma once
 #include "common.cuh"
 #include "lattice.cuh"
 
 namespace lbmb {
 
-constexpr int IBM_BLOCK = 128;
+// Blocks of a body's cluster. A block takes all registers of its SM where one
+// body is forced beside a full-grid sweep: next to the sweep's own blocks the
+// phases' gathers wait behind its accesses (128 x 128 x 160 tank: 80-100 us
+// for the call with 16 blocks of 256 threads among the sweep's).
+constexpr int IBM_CLUSTER = 8;
+// Entries per partial sum of the global diagnostics.
+constexpr int IBM_CHUNK = 32;
+// Threads of the first block that reduce the partials.
+constexpr int IBM_REDUCE = 256;
 
-// The chain's kernels are launched with programmatic stream serialization:
-// a kernel may be scheduled while its predecessor finishes, and waits here,
-// before touching any memory, until the predecessor grid has completed and
-// its writes are visible.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// All threads of the cluster; writes before it are visible after it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
 
 struct IbmDiagDev {
   double slip_max, slip_rms, slip_max_rel, slip_rms_rel;
   double torque[3], fluid_force[3], marker_force[3];
   double momentum_error_rel;
   int iterations;
-  int converged;
-  unsigned int ticket;
   int pad;
 };
 
@@ -50,9 +65,11 @@ struct IbmArgs {
   const int32_t* st_slot;  // active (non-solid) stencil points -> global slot
   const double* st_w;
   const double* st_cks;    // cell kernel sum of the point's cell (this body)
+  const double* wsum;      // nm: sum of the marker's weights
   // slots touched by this body
   int64_t ns;
   const int32_t* bslot;    // body slot -> global slot
+  const int2* brec;        // body slot -> {global slot, cell}
   const int32_t* cs_off;   // ns + 1, contributions in marker order
   const int32_t* cs_marker;
   const double* cs_w;
@@ -60,14 +77,15 @@ struct IbmArgs {
   double* rho;       // cached density (f64 view)
   double* u_now;     // x3
   double* du;        // x3
+  double4* urec;     // {u_now + du, 1 / rho}: what a marker gathers from a slot
   double* spread;    // x3
   // per marker state
   double* imp;       // x3
-  double* mob;
+  double* mob;       // relaxation / mobility (0: none)
   double* rmf;       // x3 represented marker force of this sweep
   // partials
-  double* part_spread;  // gridDim(spread) x 3
-  double* part_diag;    // gridDim(diag) x 9
+  double* part_spread;  // 2 x ceil(ns / IBM_CHUNK) x 3 (two sweeps in flight)
+  double* part_diag;    // 2 x ceil(nm / IBM_CHUNK) x 9 (8 sums, then the maxima)
   IbmDiagDev* diag;
   double center[3], omega[3];
   double scale, relax, tol;
@@ -80,6 +98,24 @@ __device__ __forceinline__ void ibm_target(const IbmArgs& a, int64_t m, double t
   t[0] = a.omega[1] * r[2] - a.omega[2] * r[1];
   t[1] = a.omega[2] * r[0] - a.omega[0] * r[2];
   t[2] = a.omega[0] * r[1] - a.omega[1] * r[0];
+}
+
+// Where post-stream population q of a cell sits in the swapped AA layout
+// (parity 1), as an element offset. A select of addresses and no branch: with
+// a load behind a branch per direction the Q loads of a cell follow each
+// other (19 x ~700 cycles in the direct forcing's first phase, measured with
+// the clock register; ~3,000 in all as one batch).
+template <int Q>
+__device__ __forceinline__ int64_t post_stream_offset(int64_t pl, int64_t cell, const Nbr& nb, uint32_t mask, int q) {
+  using L = Lat<Q>;
+  const int o = opp(q);
+  const bool wall = (mask >> o) & 1u;
+  int64_t e = wall ? q * pl + cell : o * pl + nb.at(-L::cx(q), -L::cy(q), -L::cz(q));
+  if (slips_in<Q>(q)) {
+    const bool slip = wall && (mask & NBR_SLIP) && !((mask >> planar<Q>(o)) & 1u);
+    e = slip ? opp(mirror_z<Q>(q)) * pl + nb.at(-L::cx(q), -L::cy(q), 0) : e;
+  }
+  return e;
 }
 
 // Post-stream populations of one cell in the AA layout of the given parity
@@ -95,135 +131,8 @@ __device__ __forceinline__ void load_post_stream(const S* fb, int64_t pl, int64_
   } else {
     const Nbr nb(x, y, z, nx, ny, nz);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const int o = opp(q);
-      if ((mask >> o) & 1u) {
-        const int d = planar<Q>(o);
-        if ((mask & NBR_SLIP) && L::cz(q) == -1 && d > 0 && !((mask >> d) & 1u))
-          f[q] = Codec<S>::ld(fb + opp(mirror_z<Q>(q)) * pl + nb.at(-L::cx(q), -L::cy(q), 0));
-        else
-          f[q] = Codec<S>::ld(fb + q * pl + cell);
-      } else {
-        f[q] = Codec<S>::ld(fb + o * pl + nb.at(-L::cx(q), -L::cy(q), -L::cz(q)));
-      }
-    }
+    for (int q = 0; q < Q; ++q) f[q] = Codec<S>::ld(fb + post_stream_offset<Q>(pl, cell, nb, mask, q));
   }
-}
-
-// u_now over the body's slots (solver.rs:3036-3087): cached rho (storage
-// arithmetic: 1 + sum f) and (sum c f + F/2) / rho in f64 with the force
-// field current at call time.
-template <int Q, class S>
-__device__ __forceinline__ void ibm_prep_body(const IbmArgs& a, int64_t i, const S* fb, int64_t pl,
-                                              const int64_t* slot_cell, const uint8_t* flags, const uint32_t* nbr,
-                                              int nx, int ny, int nz, int parity,
-                                              const Vec4<typename Codec<S>::A>* fcur, int field_present, double gx,
-                                              double gy, double gz) {
-  using A = typename Codec<S>::A;
-  using L = Lat<Q>;
-  if (i == 0) {
-    IbmDiagDev* d = a.diag;
-    d->slip_max = d->slip_rms = d->slip_max_rel = d->slip_rms_rel = 0.0;
-    for (int k = 0; k < 3; ++k) d->torque[k] = d->fluid_force[k] = d->marker_force[k] = 0.0;
-    d->momentum_error_rel = 0.0;
-    d->iterations = 0;
-    d->converged = 0;
-    d->ticket = 0;
-  }
-  if (i >= a.ns) return;
-  const int32_t g = a.bslot[i];
-  const int64_t cell = slot_cell[g];
-  const int64_t nxy = int64_t(nx) * ny;
-  const int z = int(cell / nxy);
-  const int y = int((cell - int64_t(z) * nxy) / nx);
-  const int x = int(cell - int64_t(z) * nxy - int64_t(y) * nx);
-  const uint32_t mask = (flags[cell] & F_BOUNDARY) ? nbr[cell] : 0u;
-  A f[Q];
-  load_post_stream<Q, S>(fb, pl, cell, x, y, z, nx, ny, nz, mask, parity, f);
-  A dr = A(0);
-  double mom[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    dr = dr + f[q];
-    const double fq = double(f[q]);
-    mom[0] += double(L::cx(q)) * fq;
-    mom[1] += double(L::cy(q)) * fq;
-    mom[2] += double(L::cz(q)) * fq;
-  }
-  const double rho = double(A(1) + dr);
-  double force[3] = {gx, gy, gz};
-  if (field_present) {
-    const Vec4<A> fc = fcur[g];
-    force[0] += double(fc.x);
-    force[1] += double(fc.y);
-    force[2] += double(fc.z);
-  }
-  const double inv_rho = 1.0 / fmax(rho, 1.0e-30);
-  a.rho[g] = rho;
-  for (int k = 0; k < 3; ++k) {
-    a.u_now[3 * g + k] = (mom[k] + 0.5 * force[k]) * inv_rho;
-    a.du[3 * g + k] = 0.0;
-    a.spread[3 * g + k] = 0.0;
-  }
-}
-
-template <int Q, class S>
-__global__ void ibm_prep_kernel(IbmArgs a, const S* fb, int64_t pl, const int64_t* slot_cell,
-                                const uint8_t* flags, const uint32_t* nbr, int nx, int ny, int nz,
-                                int parity, const Vec4<typename Codec<S>::A>* fcur, int field_present,
-                                double gx, double gy, double gz) {
-  pdl_wait();
-  ibm_prep_body<Q, S>(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x, fb, pl, slot_cell, flags, nbr, nx, ny, nz,
-                      parity, fcur, field_present, gx, gy, gz);
-}
-
-// Impulse per marker from the current du (solver.rs:3118-3173).
-__device__ __forceinline__ void ibm_interp_body(const IbmArgs& a, int64_t m, int sweep) {
-  if (m >= a.nm) return;
-  if (a.diag->converged) return;
-  double t[3], r[3];
-  ibm_target(a, m, t, r);
-  double um[3] = {0.0, 0.0, 0.0};
-  const int32_t k0 = a.st_off[m], k1 = a.st_off[m + 1];
-  double mobility = 0.0;
-  for (int32_t k = k0; k < k1; ++k) {
-    const int32_t s = a.st_slot[k];
-    const double w = a.st_w[k];
-    um[0] += w * (a.u_now[3 * s + 0] + a.du[3 * s + 0]);
-    um[1] += w * (a.u_now[3 * s + 1] + a.du[3 * s + 1]);
-    um[2] += w * (a.u_now[3 * s + 2] + a.du[3 * s + 2]);
-  }
-  if (sweep == 0) {
-    for (int32_t k = k0; k < k1; ++k) {
-      const int32_t s = a.st_slot[k];
-      mobility += a.st_w[k] * a.st_cks[k] / fmax(a.rho[s], 1.0e-30);
-    }
-    a.mob[m] = mobility;
-  } else {
-    mobility = a.mob[m];
-  }
-  double imp[3] = {0.0, 0.0, 0.0};
-  if (mobility != 0.0) {
-    imp[0] = a.relax * (t[0] - um[0]) / mobility;
-    imp[1] = a.relax * (t[1] - um[1]) / mobility;
-    imp[2] = a.relax * (t[2] - um[2]) / mobility;
-  }
-  double rmf[3] = {0.0, 0.0, 0.0};
-  for (int32_t k = k0; k < k1; ++k) {
-    const double w = a.st_w[k];
-    rmf[0] += imp[0] * w;
-    rmf[1] += imp[1] * w;
-    rmf[2] += imp[2] * w;
-  }
-  for (int c = 0; c < 3; ++c) {
-    a.imp[3 * m + c] = imp[c];
-    a.rmf[3 * m + c] = rmf[c];
-  }
-}
-
-static __global__ void ibm_interp_kernel(IbmArgs a, int sweep) {
-  pdl_wait();
-  ibm_interp_body(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x, sweep);
 }
 
 template <int N>
@@ -244,176 +153,354 @@ __device__ __forceinline__ void block_sum(double (&v)[N], double* sh) {
     }
 }
 
-// Spread the impulses into the slots, in marker order (solver.rs:3174-3209).
-// bid: block index within this body's spread grid (its partial slot).
-__device__ __forceinline__ void ibm_spread_body(const IbmArgs& a, int64_t bid) {
-  __shared__ double sh[3 * (IBM_BLOCK / 32)];
-  if (a.diag->converged) return;
-  const int64_t i = bid * blockDim.x + threadIdx.x;
-  double ff[3] = {0.0, 0.0, 0.0};
-  if (i < a.ns) {
-    const int32_t g = a.bslot[i];
-    double sp[3], d[3];
+// What one apply_rotating_ibm call works on besides the body.
+template <class S>
+struct IbmRun {
+  using A = typename Codec<S>::A;
+  const S* fb;
+  int64_t pl;
+  const uint32_t* nbr;
+  int nx, ny, nz, parity;
+  Vec4<A>* fcur;       // force field by global slot
+  int64_t nslots;
+  int field_at_call;   // fcur counts in u_now
+  int clear;           // fcur is zeroed first (only without field_at_call)
+  int sweeps;
+  double gx, gy, gz;   // uniform force
+  // per-step series (null: not recorded)
+  double* series_torque;
+  double* series_ff;
+  int32_t* series_iters;
+  int64_t* step_counter;
+  // where the adjoint keeps the intermediates of the step (null: not kept):
+  // rho, u_now (per slot), mobility (per marker), du at the start of each
+  // sweep (per slot, sv_slots rows) and each sweep's impulse (per marker)
+  double *sv_rho, *sv_u, *sv_mob, *sv_du, *sv_imp;
+  int64_t sv_slots;
+};
+
+// u_now over the body's slots (solver.rs:3036-3087): cached rho (storage
+// arithmetic: 1 + sum f) and (sum c f + F/2) / rho in f64 with the force
+// field current at call time.
+template <int Q, class S>
+__device__ __forceinline__ void ibm_prep_slot(const IbmArgs& a, const IbmRun<S>& r, int64_t i) {
+  using A = typename Codec<S>::A;
+  using L = Lat<Q>;
+  const int2 rec = a.brec[i];
+  const int32_t g = rec.x;
+  const int64_t cell = rec.y;
+  const uint32_t mask = r.nbr[cell];  // zero away from solids
+  const int64_t nxy = int64_t(r.nx) * r.ny;
+  const int z = int(cell / nxy);
+  const int y = int((cell - int64_t(z) * nxy) / r.nx);
+  const int x = int(cell - int64_t(z) * nxy - int64_t(y) * r.nx);
+  A f[Q];
+  load_post_stream<Q, S>(r.fb, r.pl, cell, x, y, z, r.nx, r.ny, r.nz, mask, r.parity, f);
+  A dr = A(0);
+  double mom[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    dr = dr + f[q];
+    const double fq = double(f[q]);
+    mom[0] += double(L::cx(q)) * fq;
+    mom[1] += double(L::cy(q)) * fq;
+    mom[2] += double(L::cz(q)) * fq;
+  }
+  const double rho = double(A(1) + dr);
+  double force[3] = {r.gx, r.gy, r.gz};
+  if (r.field_at_call) {
+    const Vec4<A> fc = r.fcur[g];
+    force[0] += double(fc.x);
+    force[1] += double(fc.y);
+    force[2] += double(fc.z);
+  }
+  const double inv_rho = 1.0 / fmax(rho, 1.0e-30);
+  a.rho[g] = rho;
+  if (r.sv_rho) r.sv_rho[g] = rho;
+  double u3[3];
+  for (int k = 0; k < 3; ++k) {
+    const double u = (mom[k] + 0.5 * force[k]) * inv_rho;
+    u3[k] = u;
+    a.u_now[3 * g + k] = u;
+    if (r.sv_u) r.sv_u[3 * g + k] = u;
+  }
+  a.urec[g] = make_double4(u3[0], u3[1], u3[2], inv_rho);
+}
+
+// Interpolated velocity of a marker from its stencil points [k0, k1) in
+// order, NB gathers in flight (points past the end repeat the last one with
+// weight 0), and, with MOB, its mobility (solver.rs:3131-3140).
+template <int NB, bool MOB>
+__device__ __forceinline__ void ibm_marker_velocity(const IbmArgs& a, int32_t k0, int32_t k1, double (&um)[3],
+                                                    double& mobility) {
+  um[0] = um[1] = um[2] = 0.0;
+  mobility = 0.0;
+  for (int32_t k = k0; k < k1; k += NB) {
+    double w[NB], n[NB];
+    double4 v[NB];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const bool in = k + j < k1;
+      const int32_t kk = in ? k + j : k1 - 1;
+      v[j] = a.urec[a.st_slot[kk]];
+      w[j] = in ? a.st_w[kk] : 0.0;
+      if (MOB) n[j] = a.st_cks[kk];
+    }
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      um[0] += w[j] * v[j].x;
+      um[1] += w[j] * v[j].y;
+      um[2] += w[j] * v[j].z;
+      if (MOB) mobility += w[j] * n[j] * v[j].w;
+    }
+  }
+}
+
+// Impulse of a marker from the interpolated velocity (solver.rs:3118-3173);
+// inv_mob = relaxation / mobility (0: no impulse).
+template <class S>
+__device__ __forceinline__ void ibm_impulse(const IbmArgs& a, const IbmRun<S>& r, int64_t m, const double (&t)[3],
+                                            const double (&um)[3], double inv_mob, int sweep) {
+  const double ws = a.wsum[m];
+  for (int c = 0; c < 3; ++c) {
+    const double imp = (t[c] - um[c]) * inv_mob;
+    a.imp[3 * m + c] = imp;
+    a.rmf[3 * m + c] = imp * ws;
+    if (r.sv_imp) r.sv_imp[(int64_t(sweep) * a.nm + m) * 3 + c] = imp;
+  }
+}
+
+// Spread the impulses into slot i, in marker order (solver.rs:3174-3209);
+// ff: the slot's share of the fluid force.
+template <int NB, class S>
+__device__ __forceinline__ void ibm_spread_slot(const IbmArgs& a, const IbmRun<S>& r, int64_t i, int sweep,
+                                                double (&ff)[3]) {
+  const int32_t g = a.brec[i].x;
+  const int32_t k0 = a.cs_off[i], k1 = a.cs_off[i + 1];
+  double sp[3] = {0.0, 0.0, 0.0}, d[3] = {0.0, 0.0, 0.0};
+  const double inv_rho = a.urec[g].w;
+  if (sweep > 0)
     for (int c = 0; c < 3; ++c) {
       sp[c] = a.spread[3 * g + c];
       d[c] = a.du[3 * g + c];
     }
-    const double inv_rho = 1.0 / fmax(a.rho[g], 1.0e-30);
-    for (int32_t k = a.cs_off[i]; k < a.cs_off[i + 1]; ++k) {
-      const int32_t m = a.cs_marker[k];
-      const double w = a.cs_w[k];
+  if (r.sv_du)
+    for (int c = 0; c < 3; ++c) r.sv_du[(int64_t(sweep) * r.sv_slots + g) * 3 + c] = d[c];
+  const double un[3] = {a.u_now[3 * g], a.u_now[3 * g + 1], a.u_now[3 * g + 2]};
+  for (int32_t k = k0; k < k1; k += NB) {
+    double w[NB], v[NB][3];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const bool in = k + j < k1;
+      const int32_t kk = in ? k + j : k1 - 1;
+      const double* im = a.imp + 3 * int64_t(a.cs_marker[kk]);
+      w[j] = in ? a.cs_w[kk] : 0.0;
+      v[j][0] = im[0];
+      v[j][1] = im[1];
+      v[j][2] = im[2];
+    }
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+#pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const double cf = a.imp[3 * m + c] * w;
+        const double cf = v[j][c] * w[j];
         sp[c] += cf;
         d[c] += cf * inv_rho;
         ff[c] += cf;
       }
-    }
-    for (int c = 0; c < 3; ++c) {
-      a.spread[3 * g + c] = sp[c];
-      a.du[3 * g + c] = d[c];
-    }
   }
-  block_sum<3>(ff, sh);
-  if (threadIdx.x == 0)
-    for (int c = 0; c < 3; ++c) a.part_spread[3 * bid + c] = ff[c];
-}
-
-static __global__ void __launch_bounds__(IBM_BLOCK) ibm_spread_kernel(IbmArgs a) {
-  pdl_wait();
-  ibm_spread_body(a, blockIdx.x);
-}
-
-// Slip statistics and the sweep's global reduction (solver.rs:3211-3253).
-// bid / nblk: block index and block count of this body's diag grid.
-__device__ __forceinline__ void ibm_diag_body(const IbmArgs& a, int sweep, int nblk_spread, unsigned int bid,
-                                              unsigned int nblk) {
-  __shared__ double sh[9 * (IBM_BLOCK / 32)];
-  __shared__ double smax_sh[IBM_BLOCK / 32];
-  __shared__ bool last;
-  if (a.diag->converged) return;
-  const int64_t m = int64_t(bid) * blockDim.x + threadIdx.x;
-  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // ssq, wsum, mf[3], tq[3]
-  double smax = 0.0;
-  if (m < a.nm) {
-    double t[3], r[3];
-    ibm_target(a, m, t, r);
-    const int32_t k0 = a.st_off[m], k1 = a.st_off[m + 1];
-    if (k1 > k0) {
-      double um[3] = {0.0, 0.0, 0.0};
-      for (int32_t k = k0; k < k1; ++k) {
-        const int32_t s = a.st_slot[k];
-        const double w = a.st_w[k];
-        um[0] += w * (a.u_now[3 * s + 0] + a.du[3 * s + 0]);
-        um[1] += w * (a.u_now[3 * s + 1] + a.du[3 * s + 1]);
-        um[2] += w * (a.u_now[3 * s + 2] + a.du[3 * s + 2]);
-      }
-      const double sl[3] = {t[0] - um[0], t[1] - um[1], t[2] - um[2]};
-      const double mag = sqrt(sl[0] * sl[0] + sl[1] * sl[1] + sl[2] * sl[2]);
-      smax = mag;
-      v[0] = a.weight[m] * mag * mag;
-      v[1] = a.weight[m];
-    }
-    const double* f = a.rmf + 3 * m;
-    v[2] = f[0];
-    v[3] = f[1];
-    v[4] = f[2];
-    v[5] = r[1] * f[2] - r[2] * f[1];
-    v[6] = r[2] * f[0] - r[0] * f[2];
-    v[7] = r[0] * f[1] - r[1] * f[0];
-  }
-  for (int o = 16; o > 0; o >>= 1) smax = fmax(smax, __shfl_down_sync(0xffffffffu, smax, o));
-  if ((threadIdx.x & 31) == 0) smax_sh[threadIdx.x >> 5] = smax;
-  block_sum<8>(v, sh);
-  if (threadIdx.x == 0) {
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) smax = fmax(smax, smax_sh[w]);
-    double* p = a.part_diag + 9 * bid;
-    p[0] = smax;
-    for (int k = 0; k < 8; ++k) p[1 + k] = v[k];
-    __threadfence();
-    const unsigned int t = atomicAdd(&a.diag->ticket, 1u);
-    last = (t == nblk - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // The last block reduces every partial: thread t takes blocks t, t + B,
-  // ... in order, then a fixed tree (deterministic run to run).
-  double acc[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // 8 diag sums, 3 spread sums
-  double amax = 0.0;
-  for (unsigned int b = threadIdx.x; b < nblk; b += blockDim.x) {
-    const volatile double* p = a.part_diag + 9 * b;
-    amax = fmax(amax, p[0]);
-    for (int k = 0; k < 8; ++k) acc[k] += p[1 + k];
-  }
-  for (int b = threadIdx.x; b < nblk_spread; b += blockDim.x)
-    for (int c = 0; c < 3; ++c) acc[8 + c] += ((const volatile double*)a.part_spread)[3 * b + c];
-  __syncthreads();
-  for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_down_sync(0xffffffffu, amax, o));
-  if ((threadIdx.x & 31) == 0) smax_sh[threadIdx.x >> 5] = amax;
-  __shared__ double sh2[11 * (IBM_BLOCK / 32)];
-  block_sum<11>(acc, sh2);
-  if (threadIdx.x != 0) return;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) amax = fmax(amax, smax_sh[w]);
-  double tot[9];
-  tot[0] = amax;
-  for (int k = 0; k < 8; ++k) tot[1 + k] = acc[k];
-  const double ffs[3] = {acc[8], acc[9], acc[10]};
-  IbmDiagDev* d = a.diag;
   for (int c = 0; c < 3; ++c) {
-    d->fluid_force[c] += ffs[c];
-    d->marker_force[c] += tot[3 + c];
-    d->torque[c] -= tot[6 + c];
+    a.spread[3 * g + c] = sp[c];
+    a.du[3 * g + c] = d[c];
   }
-  d->iterations = sweep + 1;
-  d->slip_max = tot[0];
-  d->slip_rms = tot[2] > 0.0 ? sqrt(tot[1] / tot[2]) : 0.0;
-  d->slip_max_rel = d->slip_max / a.scale;
-  d->slip_rms_rel = d->slip_rms / a.scale;
-  const double e0 = d->fluid_force[0] - d->marker_force[0];
-  const double e1 = d->fluid_force[1] - d->marker_force[1];
-  const double e2 = d->fluid_force[2] - d->marker_force[2];
-  const double mf = sqrt(d->marker_force[0] * d->marker_force[0] + d->marker_force[1] * d->marker_force[1] +
-                         d->marker_force[2] * d->marker_force[2]);
-  d->momentum_error_rel = sqrt(e0 * e0 + e1 * e1 + e2 * e2) / fmax(mf, 1.0e-12);
-  if (d->slip_max_rel <= a.tol) d->converged = 1;
-  d->ticket = 0;
+  a.urec[g] = make_double4(un[0] + d[0], un[1] + d[1], un[2] + d[2], inv_rho);
 }
 
-static __global__ void __launch_bounds__(IBM_BLOCK) ibm_diag_kernel(IbmArgs a, int sweep, int nblk_spread) {
-  pdl_wait();
-  ibm_diag_body(a, sweep, nblk_spread, blockIdx.x, gridDim.x);
+__device__ __forceinline__ double warp_sum(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ double warp_max(double v) {
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
+  return v;
 }
 
-// force field += spread in the storage arithmetic (solver.rs:3256-3279),
-// and optionally record the diagnostics of this call into per-step series.
-template <class A>
-__device__ __forceinline__ void ibm_commit_body(const IbmArgs& a, int64_t i, Vec4<A>* fcur, double* series_torque,
-                                                double* series_ff, int32_t* series_iters, int64_t* step_counter) {
-  if (i < a.ns) {
-    const int32_t g = a.bslot[i];
-    Vec4<A> v = fcur[g];
+// One apply_rotating_ibm call of one body by one cluster; rank: block in the
+// cluster, ncta: its blocks; NB: gathers in flight per thread. Every barrier
+// is reached by every thread: the sweep loop's exit is decided from the same
+// value in every block.
+template <int Q, class S, int NB>
+__device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, int rank, int ncta) {
+  using A = typename Codec<S>::A;
+  __shared__ double sh[11 * (IBM_REDUCE / 32)];
+  __shared__ double tot[11];
+  const int lane = int(threadIdx.x) & 31, warp = int(threadIdx.x) >> 5;
+  const int64_t nthr = int64_t(ncta) * blockDim.x;
+  const int64_t tid = (int64_t(warp) * ncta + rank) * 32 + lane;  // few entries spread over the blocks
+  const int64_t nc_m = (a.nm + IBM_CHUNK - 1) / IBM_CHUNK, nc_s = (a.ns + IBM_CHUNK - 1) / IBM_CHUNK;
+  for (int64_t i = tid; i < a.ns; i += nthr) ibm_prep_slot<Q, S>(a, r, i);
+  if (r.clear)
+    for (int64_t s = tid; s < r.nslots; s += nthr) r.fcur[s] = Vec4<A>{A(0), A(0), A(0), A(0)};
+  cluster_sync();
+  for (int64_t m = tid; m < a.nm; m += nthr) {
+    double t[3], x[3], um[3], mob;
+    ibm_target(a, m, t, x);
+    ibm_marker_velocity<NB, true>(a, a.st_off[m], a.st_off[m + 1], um, mob);
+    const double inv = mob != 0.0 ? a.relax / mob : 0.0;
+    a.mob[m] = inv;
+    if (r.sv_mob) r.sv_mob[m] = mob;
+    ibm_impulse(a, r, m, t, um, inv, 0);
+  }
+  cluster_sync();
+  // block 0: running sums of the call (thread k of the first warp holds sum k:
+  // 0..1 slip, 2..4 marker force, 5..7 marker torque, 8..10 fluid force)
+  double run = 0.0, slip_max = 0.0, ssq = 0.0, wsum = 0.0;
+  int done = 0;
+  for (int s = 0; s < r.sweeps; ++s) {
+    double* const ps = a.part_spread + (s & 1) * 3 * nc_s;
+    double* const pd = a.part_diag + (s & 1) * 9 * nc_m;
+    double* const px = pd + 8 * nc_m;
+    for (int64_t i0 = tid - lane; i0 < a.ns; i0 += nthr) {
+      double ff[3] = {0.0, 0.0, 0.0};
+      if (i0 + lane < a.ns) ibm_spread_slot<NB>(a, r, i0 + lane, s, ff);
+      for (int c = 0; c < 3; ++c) {
+        const double v = warp_sum(ff[c]);
+        if (lane == 0) ps[3 * (i0 / IBM_CHUNK) + c] = v;
+      }
+    }
+    cluster_sync();
+    // slip statistics (solver.rs:3211-3253) and the next sweep's impulse
+    for (int64_t m0 = tid - lane; m0 < a.nm; m0 += nthr) {
+      const int64_t m = m0 + lane;
+      double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // ssq, wsum, mf[3], tq[3]
+      double smax = 0.0;
+      if (m < a.nm) {
+        double t[3], x[3], um[3], none;
+        const double* f = a.rmf + 3 * m;
+        const double f0 = f[0], f1 = f[1], f2 = f[2], wt = a.weight[m], inv = a.mob[m];
+        ibm_target(a, m, t, x);
+        const int32_t k0 = a.st_off[m], k1 = a.st_off[m + 1];
+        ibm_marker_velocity<NB, false>(a, k0, k1, um, none);
+        if (k1 > k0) {
+          const double sl[3] = {t[0] - um[0], t[1] - um[1], t[2] - um[2]};
+          const double s2 = sl[0] * sl[0] + sl[1] * sl[1] + sl[2] * sl[2];
+          const double mag = sqrt(s2);
+          smax = fmax(mag, 0.0);  // a diverged state (NaN) has no slip
+          v[0] = wt * mag * mag;
+          v[1] = wt;
+        }
+        v[2] = f0;
+        v[3] = f1;
+        v[4] = f2;
+        v[5] = x[1] * f2 - x[2] * f1;
+        v[6] = x[2] * f0 - x[0] * f2;
+        v[7] = x[0] * f1 - x[1] * f0;
+        if (s + 1 < r.sweeps) ibm_impulse(a, r, m, t, um, inv, s + 1);
+      }
+      smax = warp_max(smax);
+      if (lane == 0) px[m0 / IBM_CHUNK] = smax;
+      double* const p = pd + 8 * (m0 / IBM_CHUNK);
+      for (int k = 0; k < 8; ++k) {
+        const double y = warp_sum(v[k]);
+        if (lane == 0) p[k] = y;
+      }
+    }
+    cluster_sync();
+    // the largest slip, by every warp
+    double amax = 0.0;
+    for (int64_t c = lane; c < nc_m; c += 32) amax = fmax(amax, px[c]);
+    amax = __shfl_sync(0xffffffffu, warp_max(amax), 0);
+    if (rank == 0) {
+      // the first block sums the partials: IBM_REDUCE threads, chunks
+      // t, t + IBM_REDUCE, ... in order, then a fixed tree
+      double acc[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // 8 slip sums, 3 spread sums
+      if (threadIdx.x < IBM_REDUCE) {
+        for (int64_t c = threadIdx.x; c < nc_m; c += IBM_REDUCE)
+          for (int k = 0; k < 8; ++k) acc[k] += pd[8 * c + k];
+        for (int64_t c = threadIdx.x; c < nc_s; c += IBM_REDUCE)
+          for (int k = 0; k < 3; ++k) acc[8 + k] += ps[3 * c + k];
+        for (int k = 0; k < 11; ++k) {
+          const double y = warp_sum(acc[k]);
+          if (lane == 0) sh[k * (IBM_REDUCE / 32) + warp] = y;
+        }
+      }
+      __syncthreads();
+      if (threadIdx.x < 11) {
+        double y = 0.0;
+        for (int w = 0; w < IBM_REDUCE / 32; ++w) y += sh[int(threadIdx.x) * (IBM_REDUCE / 32) + w];
+        run += y;
+        if (threadIdx.x < 2) tot[threadIdx.x] = y;
+      }
+      __syncthreads();  // sh is written again by the next sweep
+      slip_max = amax;
+      ssq = tot[0];
+      wsum = tot[1];
+    }
+    done = s + 1;
+    if (!r.sv_imp && amax / a.scale <= a.tol) break;  // the adjoint records a fixed number of sweeps
+  }
+  // force field += spread in the storage arithmetic (solver.rs:3256-3279);
+  // each slot's spread was written by this thread
+  for (int64_t i = tid; i < a.ns; i += nthr) {
+    const int32_t g = a.brec[i].x;
+    Vec4<A> v = r.fcur[g];
     v.x = v.x + A(a.spread[3 * g + 0]);
     v.y = v.y + A(a.spread[3 * g + 1]);
     v.z = v.z + A(a.spread[3 * g + 2]);
-    fcur[g] = v;
+    r.fcur[g] = v;
   }
-  if (i == 0 && step_counter) {
-    const int64_t s = *step_counter;
-    if (series_torque) series_torque[s] = -a.diag->torque[2];
-    if (series_ff)
-      for (int c = 0; c < 3; ++c) series_ff[3 * s + c] = a.diag->fluid_force[c];
-    if (series_iters) series_iters[s] = a.diag->iterations;
-    *step_counter = s + 1;
+  if (rank == 0 && warp == 0) {
+    // lane k holds sum k (see above); the torque on the body is minus the
+    // marker torque
+    IbmDiagDev* d = a.diag;
+    const double sgn = lane >= 5 && lane < 8 ? -run : run;
+    const double e = __shfl_sync(0xffffffffu, run, lane < 3 ? lane + 8 : 0) -
+                     __shfl_sync(0xffffffffu, run, lane < 3 ? lane + 2 : 0);
+    const double f = __shfl_sync(0xffffffffu, run, lane < 3 ? lane + 2 : 0);
+    const double e0 = __shfl_sync(0xffffffffu, e, 0), e1 = __shfl_sync(0xffffffffu, e, 1),
+                 e2 = __shfl_sync(0xffffffffu, e, 2);
+    const double f0 = __shfl_sync(0xffffffffu, f, 0), f1 = __shfl_sync(0xffffffffu, f, 1),
+                 f2 = __shfl_sync(0xffffffffu, f, 2);
+    const int64_t st = r.step_counter ? *r.step_counter : 0;
+    __syncwarp();
+    if (lane >= 2 && lane < 5) d->marker_force[lane - 2] = run;
+    if (lane >= 5 && lane < 8) d->torque[lane - 5] = sgn;
+    if (lane >= 8 && lane < 11) d->fluid_force[lane - 8] = run;
+    if (r.step_counter) {
+      if (lane == 7 && r.series_torque) r.series_torque[st] = -sgn;
+      if (lane >= 8 && lane < 11 && r.series_ff) r.series_ff[3 * st + lane - 8] = run;
+    }
+    if (lane == 0) {
+      d->slip_max = slip_max;
+      d->slip_max_rel = slip_max / a.scale;
+      d->iterations = done;
+      if (r.step_counter) {
+        if (r.series_iters) r.series_iters[st] = done;
+        *r.step_counter = st + 1;
+      }
+    }
+    if (lane == 1) {
+      const double rms = wsum > 0.0 ? sqrt(ssq / wsum) : 0.0;
+      d->slip_rms = rms;
+      d->slip_rms_rel = rms / a.scale;
+    }
+    if (lane == 11)
+      d->momentum_error_rel =
+          sqrt(e0 * e0 + e1 * e1 + e2 * e2) / fmax(sqrt(f0 * f0 + f1 * f1 + f2 * f2), 1.0e-12);
   }
 }
 
-template <class A>
-__global__ void ibm_commit_kernel(IbmArgs a, Vec4<A>* fcur, double* series_torque, double* series_ff,
-                                  int32_t* series_iters, int64_t* step_counter) {
-  pdl_wait();
-  ibm_commit_body<A>(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x, fcur, series_torque, series_ff,
-                     series_iters, step_counter);
+// The sweep of the unforced cells is launched as this kernel's programmatic
+// dependent: it starts once every block of the cluster runs, so that the
+// cluster is resident before the sweep fills the chip.
+__device__ __forceinline__ void release_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// NT threads per block and NB gathers in flight: 512 and 8 (128 registers a
+// thread) or 1024 and 4 (64).
+template <int Q, class S, int NT, int NB>
+__global__ void __launch_bounds__(NT, 1) ibm_chain_kernel(IbmArgs a, IbmRun<S> r) {
+  release_dependents();
+  ibm_chain<Q, S, NB>(a, r, int(blockIdx.x), int(gridDim.x));
 }
 
 }  // namespace lbmb

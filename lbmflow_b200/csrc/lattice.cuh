@@ -86,4 +86,15 @@ __host__ __device__ constexpr int planar(int q) {
   return find_dir<Q>(Lat<Q>::cx(q), Lat<Q>::cy(q), 0);
 }
 
+// Directions of a free-slip reflection: on the odd step link q with c_z = -1
+// comes from the mirrored population of the in-plane partner.
+template <int Q>
+__host__ __device__ constexpr bool slips_in(int q) {
+  return Lat<Q>::cz(q) == -1 && planar<Q>(opp(q)) > 0;
+}
+template <int Q>
+__host__ __device__ constexpr bool slips_out(int q) {
+  return Lat<Q>::cz(q) == 1 && planar<Q>(q) > 0;
+}
+
 }  // namespace lbmb

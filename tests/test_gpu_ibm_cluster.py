@@ -1,0 +1,54 @@
+"""Direct forcing as one cluster kernel: marker and slot counts at the edges.
+
+The kernel works in chunks of 32 markers and slots, in one of two forms (up
+to 4,096 entries, and above), and leaves its sweep loop early. Each count is
+compared with the oracle on the same f64 populations: diagnostics to 1e-10
+(sums of at most 1e5 terms, n eps = 2e-11), field to 1e-12 of its largest
+value (the spread sums in the reference's marker order).
+"""
+import numpy as np
+import pytest
+
+import lbmflow_b200 as lb
+from cases import cavity, seeded_state
+from test_gpu_ibm import assert_diag_close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nm", [1, 31, 32, 33, 1025, 4096, 4097, 9000])
+@pytest.mark.parametrize("radius,tol", [(1, 1e-2), (2, 0.0)])
+def test_marker_counts_match_oracle(nm, radius, tol):
+    from oracle import oracle as o
+    dims, solid, wall_u, nu = cavity(34)
+    rng = np.random.default_rng(nm)
+    pos = rng.uniform(0.6, 32.4, (nm, 3))  # some stencils reach the walls
+    w = rng.uniform(0.2, 0.8, nm)
+    body = lb.RotatingBody([16.5, 16.5, 16.5], [0.0, 0.001, 0.002], pos, w)
+    g = lb.Solver(dims, lattice=19, storage="f64", nu=nu, solid=solid, wall_u=wall_u)
+    c = o.OracleSolver(dims, q=19, real_bits=64, nu=nu, solid=solid, wall_u=wall_u)
+    f = seeded_state(19, g.n, 5)
+    f[:, solid != 0] = 0.0
+    g.stage_in(f)
+    c.stage_in(f)
+    for _ in range(2):  # the second application sees the first one's field
+        dg = g.apply_rotating_ibm(body, lb.DirectForcingConfig(3, tol, radius, 0.9))
+        do = c.ibm_apply(body.positions, body.weights, body.center, body.omega, 3, tol, radius, 0.9)
+        assert_diag_close(dg, do, 1e-10)
+        fg, fc = g.force_field(), c.force_field()
+        assert np.abs(fg - fc).max() <= 1e-12 * np.abs(fc).max()
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+def test_runner_loop_repeats_bitwise(storage):
+    # the phases of one call are ordered by cluster barriers only: a missing
+    # one shows as a difference between two runs
+    from lbmflow_b200 import sweep
+    ref = None
+    for _ in range(4):
+        g, body = sweep.build_case(sweep.TankCase(32, 0.05, 600.0), storage=storage)
+        r = g.run_impeller(body, 40)
+        got = (r["torque_lu"], r["ibm_iterations"], g.stage_out())
+        if ref is not None:
+            assert all(np.array_equal(a, b) for a, b in zip(ref, got))
+        ref = got
