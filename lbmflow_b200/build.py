@@ -26,7 +26,7 @@ def units():
 
 
 def headers():
-    hs = [os.path.join(SRC, f) for f in os.listdir(SRC) if f.endswith((".cuh", ".h"))]
+    hs = [os.path.join(SRC, f) for f in os.listdir(SRC) if f.endswith((".cuh", ".h", ".hpp"))]
     return hs + [os.path.join(HERE, "..", "include", "lbmb.h"), __file__]
 
 

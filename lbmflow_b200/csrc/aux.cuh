@@ -16,15 +16,17 @@ __device__ __forceinline__ void cell_xyz(int64_t cell, int nx, int ny, int& x, i
   x = int(r - int64_t(y) * nx);
 }
 
-// Logical post-stream populations -> f64 q-major host layout (stage_out).
+// Logical post-stream populations of cells [c0, c1) -> f64, direction q at
+// out + q * stride (stage_out).
 // Solid cells report their raw own slots (the reference leaves solid
 // populations unspecified: streaming never writes them).
 template <int Q, class S>
 __global__ void stage_out_kernel(const S* fb, int64_t pl, const uint8_t* flags, const uint32_t* nbr,
-                                 int nx, int ny, int nz, int parity, double* out, int64_t n) {
+                                 int nx, int ny, int nz, int parity, double* out, int64_t stride, int64_t c0,
+                                 int64_t c1) {
   using A = typename Codec<S>::A;
-  const int64_t cell = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (cell >= n) return;
+  const int64_t cell = c0 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (cell >= c1) return;
   const uint8_t fl = flags[cell];
   A f[Q];
   if (fl & F_SOLID) {
@@ -37,7 +39,7 @@ __global__ void stage_out_kernel(const S* fb, int64_t pl, const uint8_t* flags, 
     load_post_stream<Q, S>(fb, pl, cell, x, y, z, nx, ny, nz, mask, parity, f);
   }
 #pragma unroll
-  for (int q = 0; q < Q; ++q) out[q * n + cell] = double(f[q]);
+  for (int q = 0; q < Q; ++q) out[q * stride + (cell - c0)] = double(f[q]);
 }
 
 // f64 q-major host layout -> normal (parity 0) storage layout (stage_in).
@@ -99,19 +101,30 @@ __global__ void unpack_padded_kernel(S* fb, int64_t pl, const T* img, int nx, in
 }
 
 // Moments of the current state (kernels.rs:627-668) with the force field
-// that is inside the cached moments (fprev). Solid cells are skipped.
+// that is inside the cached moments (fprev), cells [c0, c1), cell c0 at the
+// outputs' element 0. Solid cells: rho 1 and u 0 with fill_solid, else
+// skipped.
 template <int Q, class S>
 __global__ void moments_kernel(const S* fb, int64_t pl, const uint8_t* flags, const uint32_t* nbr,
                                int nx, int ny, int nz, int parity, const int32_t* fslot,
                                const Vec4<typename Codec<S>::A>* fprev, typename Codec<S>::A gx,
                                typename Codec<S>::A gy, typename Codec<S>::A gz, double* rho,
-                               double* ux, double* uy, double* uz, int64_t n) {
+                               double* ux, double* uy, double* uz, int fill_solid, int64_t c0, int64_t c1) {
   using A = typename Codec<S>::A;
   using L = Lat<Q>;
-  const int64_t cell = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (cell >= n) return;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t cell = c0 + i;
+  if (cell >= c1) return;
   const uint8_t fl = flags[cell];
-  if (fl & F_SOLID) return;
+  if (fl & F_SOLID) {
+    if (fill_solid) {
+      if (rho) rho[i] = 1.0;
+      if (ux) ux[i] = 0.0;
+      if (uy) uy[i] = 0.0;
+      if (uz) uz[i] = 0.0;
+    }
+    return;
+  }
   int x, y, z;
   cell_xyz(cell, nx, ny, x, y, z);
   const uint32_t mask = (fl & F_BOUNDARY) ? nbr[cell] : 0u;
@@ -137,10 +150,10 @@ __global__ void moments_kernel(const S* fb, int64_t pl, const uint8_t* flags, co
   }
   const A r = A(1) + dr;
   const A inv = A(1) / r;
-  if (rho) rho[cell] = double(r);
-  if (ux) ux[cell] = double((m0 + A(0.5) * Fx) * inv);
-  if (uy) uy[cell] = double((m1 + A(0.5) * Fy) * inv);
-  if (uz) uz[cell] = double((m2 + A(0.5) * Fz) * inv);
+  if (rho) rho[i] = double(r);
+  if (ux) ux[i] = double((m0 + A(0.5) * Fx) * inv);
+  if (uy) uy[i] = double((m1 + A(0.5) * Fy) * inv);
+  if (uz) uz[i] = double((m2 + A(0.5) * Fz) * inv);
 }
 
 // Per-block f64 partials of the backend reductions (backend.rs:920-970):

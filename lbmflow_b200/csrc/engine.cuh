@@ -21,6 +21,7 @@
 
 #include "../../include/lbmb.h"
 #include "checkpoint.hpp"
+#include "readback.hpp"
 #include "aux.cuh"
 #include "hydro.cuh"
 #include "hydro_tma.cuh"
@@ -236,6 +237,7 @@ struct Engine final : EngineBase {
   // host mirrors
   std::vector<uint8_t> solid_h, flags_h;
   std::vector<double> init_rho_h, init_u_h;
+  bool init_is_rest = true;  // they hold rho = 1, u = 0 everywhere
   // device copy of init_u_h (the velocity the scalar equilibrium uses on
   // solid cells), refreshed when init_u_h changes
   DevBuf<double> d_init_u;
@@ -1196,14 +1198,21 @@ struct Engine final : EngineBase {
     invalidate_graphs();
   }
 
+  // Readback of per-cell fields through pinned slots (readback.hpp).
+  std::shared_ptr<StagePool> stage_pool = StagePool::get();
+  template <class Launch>
+  void read(const std::vector<ReadField>& fields, const Launch& launch) {
+    read_fields(cfg.device, st, *stage_pool, n, fields, launch, [](cudaError_t e) { CK(e); });
+  }
+
   void stage_out(double* fout) override {
-    DevBuf<double> tmp;
-    tmp.alloc(size_t(Q) * n);
-    stage_out_kernel<Q, S><<<unsigned(ceil_div(n, 128)), 128, 0, st>>>(fp, plane, flags.p, nbr.p, nx, ny, nz,
-                                                                       parity, tmp.p, n);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(fout, tmp.p, size_t(Q) * n * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    std::vector<ReadField> fields;
+    for (int q = 0; q < Q; ++q) fields.push_back({fout + size_t(q) * size_t(n), 1});
+    read(fields, [&](const std::vector<double*>& d, int64_t c0, int64_t c1) {
+      stage_out_kernel<Q, S><<<unsigned(ceil_div(c1 - c0, 128)), 128, 0, st>>>(fp, plane, flags.p, nbr.p, nx, ny, nz,
+                                                                               parity, d[0], c1 - c0, c0, c1);
+      CK(cudaGetLastError());
+    });
   }
 
   // Solver::init_with (solver.rs:2474-2605) on the host, in the arithmetic
@@ -1271,26 +1280,34 @@ struct Engine final : EngineBase {
           for (int k = 0; k < 3; ++k) init_u_h[3 * c + k] = double(u[k]);
           d_init_u_ok = false;
         }
+    init_is_rest = false;
     stage_in(fh.data());
   }
 
   void read_moments(double* rho, double* ux, double* uy, double* uz) override {
-    DevBuf<double> d;
-    d.alloc(size_t(4) * n);
-    moments_kernel<Q, S><<<unsigned(ceil_div(n, 128)), 128, 0, st>>>(
-        fp, plane, flags.p, nbr.p, nx, ny, nz, parity, fslot.p, fprev.p, A(cfg.force[0]), A(cfg.force[1]),
-        A(cfg.force[2]), d.p, d.p + n, d.p + 2 * n, d.p + 3 * n, n);
-    CK(cudaGetLastError());
-    std::vector<double> h(size_t(4) * n);
-    CK(cudaMemcpyAsync(h.data(), d.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    for (int64_t c = 0; c < n; ++c) {
-      const bool s = solid_h[c] != 0;
-      if (rho) rho[c] = s ? init_rho_h[c] : h[c];
-      if (ux) ux[c] = s ? init_u_h[3 * c] : h[n + c];
-      if (uy) uy[c] = s ? init_u_h[3 * c + 1] : h[2 * n + c];
-      if (uz) uz[c] = s ? init_u_h[3 * c + 2] : h[3 * n + c];
-    }
+    double* const out[4] = {rho, ux, uy, uz};
+    std::vector<ReadField> fields;
+    int at[4] = {-1, -1, -1, -1};
+    for (int k = 0; k < 4; ++k)
+      if (out[k]) {
+        at[k] = int(fields.size());
+        fields.push_back({out[k], 1});
+      }
+    read(fields, [&](const std::vector<double*>& d, int64_t c0, int64_t c1) {
+      auto to = [&](int k) { return at[k] < 0 ? nullptr : d[size_t(at[k])]; };
+      moments_kernel<Q, S><<<unsigned(ceil_div(c1 - c0, 128)), 128, 0, st>>>(
+          fp, plane, flags.p, nbr.p, nx, ny, nz, parity, fslot.p, fprev.p, A(cfg.force[0]), A(cfg.force[1]),
+          A(cfg.force[2]), to(0), to(1), to(2), to(3), 1, c0, c1);
+      CK(cudaGetLastError());
+    });
+    if (init_is_rest) return;
+    for (int64_t c = 0; c < n; ++c)  // solid cells report what they were initialised with
+      if (solid_h[c]) {
+        if (rho) rho[c] = init_rho_h[c];
+        if (ux) ux[c] = init_u_h[3 * c];
+        if (uy) uy[c] = init_u_h[3 * c + 1];
+        if (uz) uz[c] = init_u_h[3 * c + 2];
+      }
   }
 
   void reduce_all(double out[5]) override {
@@ -1374,15 +1391,15 @@ struct Engine final : EngineBase {
   }
 
   void strain_rate(double* s6, double* gamma) override {
-    DevBuf<double> d6, dg;
-    if (s6) d6.alloc(size_t(6) * n);
-    if (gamma) dg.alloc(size_t(n));
-    strain_rate_kernel<Q, S><<<unsigned(ceil_div(n, 128)), 128, 0, st>>>(strain_args(), s6 ? d6.p : nullptr,
-                                                                        gamma ? dg.p : nullptr, n);
-    CK(cudaGetLastError());
-    if (s6) CK(cudaMemcpyAsync(s6, d6.p, size_t(6) * n * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (gamma) CK(cudaMemcpyAsync(gamma, dg.p, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    std::vector<ReadField> fields;
+    if (s6) fields.push_back({s6, 6});
+    if (gamma) fields.push_back({gamma, 1});
+    const StrainArgs<S> a = strain_args();
+    read(fields, [&](const std::vector<double*>& d, int64_t c0, int64_t c1) {
+      strain_rate_kernel<Q, S><<<unsigned(ceil_div(c1 - c0, 128)), 128, 0, st>>>(
+          a, s6 ? d[0] : nullptr, gamma ? d[s6 ? 1 : 0] : nullptr, c0, c1);
+      CK(cudaGetLastError());
+    });
   }
 
   // ---- per-cell relaxation field and WALE (les.rs) -------------------------
@@ -1422,15 +1439,15 @@ struct Engine final : EngineBase {
   }
 
   void velocity_gradient(double* g9) override {
-    DevBuf<double> u3, dg;
+    DevBuf<double> u3;
     velocity_moments(u3);
-    dg.alloc(size_t(9) * n);
-    wale_kernel<Q, S><<<unsigned(ceil_div(n, 128)), 128, 0, st>>>(
-        strain_args(), u3.p, wall_u.p, cfg.periodic[0], cfg.periodic[1], cfg.periodic[2], A(cfg.nu), 0, A(0), dg.p,
-        nullptr, nullptr, nullptr, nullptr, n);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(g9, dg.p, size_t(9) * n * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    const StrainArgs<S> a = strain_args();
+    read({{g9, 9}}, [&](const std::vector<double*>& d, int64_t c0, int64_t c1) {
+      wale_kernel<Q, S><<<unsigned(ceil_div(c1 - c0, 128)), 128, 0, st>>>(
+          a, u3.p, wall_u.p, cfg.periodic[0], cfg.periodic[1], cfg.periodic[2], A(cfg.nu), 0, A(0), d[0], nullptr,
+          nullptr, nullptr, nullptr, c0, c1);
+      CK(cudaGetLastError());
+    });
   }
 
   // WaleLes::update (les.rs:120-211): nu_t and the omega+ field, installed
@@ -1447,20 +1464,25 @@ struct Engine final : EngineBase {
       if (A(tau_eff_max) < tau0) invalid("tau_eff_max must be at least the laminar tau for this solver");
       nu_t_max = (A(tau_eff_max) - tau0) / A(3.0);
     }
-    DevBuf<double> u3, dnu;
+    DevBuf<double> u3;
     DevBuf<unsigned long long> cnt;
     cnt.alloc(2);
     CK(cudaMemsetAsync(cnt.p, 0, 2 * sizeof(unsigned long long), st));
     velocity_moments(u3);
-    if (nu_t) dnu.alloc(size_t(n));
     if (omega_dev.n != size_t(n)) omega_dev.alloc(size_t(n));
-    wale_kernel<Q, S><<<unsigned(ceil_div(n, 128)), 128, 0, st>>>(
-        strain_args(), u3.p, wall_u.p, cfg.periodic[0], cfg.periodic[1], cfg.periodic[2], nu0, clip ? 1 : 0,
-        nu_t_max, nullptr, nu_t ? dnu.p : nullptr, omega_dev.p, cnt.p, cnt.p + 1, n);
-    CK(cudaGetLastError());
+    const StrainArgs<S> a = strain_args();
+    auto update = [&](double* nut, int64_t c0, int64_t c1) {
+      wale_kernel<Q, S><<<unsigned(ceil_div(c1 - c0, 128)), 128, 0, st>>>(
+          a, u3.p, wall_u.p, cfg.periodic[0], cfg.periodic[1], cfg.periodic[2], nu0, clip ? 1 : 0, nu_t_max, nullptr,
+          nut, omega_dev.p, cnt.p, cnt.p + 1, c0, c1);
+      CK(cudaGetLastError());
+    };
+    if (nu_t)
+      read({{nu_t, 1}}, [&](const std::vector<double*>& d, int64_t c0, int64_t c1) { update(d[0], c0, c1); });
+    else
+      update(nullptr, 0, n);
     unsigned long long hc[2] = {0, 0};
     CK(cudaMemcpyAsync(hc, cnt.p, sizeof(hc), cudaMemcpyDeviceToHost, st));
-    if (nu_t) CK(cudaMemcpyAsync(nu_t, dnu.p, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     omega_install();
     if (diag) {
@@ -1479,7 +1501,7 @@ struct Engine final : EngineBase {
     u3.alloc(size_t(3) * n);
     moments_kernel<Q, S><<<unsigned(ceil_div(n, 128)), 128, 0, st>>>(
         fp, plane, flags.p, nbr.p, nx, ny, nz, parity, fslot.p, fprev.p, A(cfg.force[0]), A(cfg.force[1]),
-        A(cfg.force[2]), nullptr, u3.p, u3.p + n, u3.p + 2 * n, n);
+        A(cfg.force[2]), nullptr, u3.p, u3.p + n, u3.p + 2 * n, 0, int64_t(0), n);
     CK(cudaGetLastError());
   }
   static void check_si(double dx, double dt, double mu) {
@@ -1490,19 +1512,22 @@ struct Engine final : EngineBase {
 
   void stress_field(double dx, double dt, double mu, double* s6, double* gamma, double* viscous) override {
     check_si(dx, dt, mu);
-    DevBuf<double> u3, d6, dg, dv;
+    DevBuf<double> u3;
     velocity_moments(u3);
-    if (s6) d6.alloc(size_t(6) * n);
-    if (gamma) dg.alloc(size_t(n));
-    if (viscous) dv.alloc(size_t(n));
-    stress_field_kernel<<<unsigned(ceil_div(n, 128)), 128, 0, st>>>(
-        u3.p, u3.p + n, u3.p + 2 * n, flags.p, nx, ny, nz, dx, dx / dt, mu, s6 ? d6.p : nullptr,
-        gamma ? dg.p : nullptr, viscous ? dv.p : nullptr, nullptr, nullptr, n);
-    CK(cudaGetLastError());
-    if (s6) CK(cudaMemcpyAsync(s6, d6.p, size_t(6) * n * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (gamma) CK(cudaMemcpyAsync(gamma, dg.p, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (viscous) CK(cudaMemcpyAsync(viscous, dv.p, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    std::vector<ReadField> fields;
+    const int i6 = s6 ? int(fields.size()) : -1;
+    if (s6) fields.push_back({s6, 6});
+    const int ig = gamma ? int(fields.size()) : -1;
+    if (gamma) fields.push_back({gamma, 1});
+    const int iv = viscous ? int(fields.size()) : -1;
+    if (viscous) fields.push_back({viscous, 1});
+    read(fields, [&](const std::vector<double*>& d, int64_t c0, int64_t c1) {
+      auto to = [&](int k) { return k < 0 ? nullptr : d[size_t(k)]; };
+      stress_field_kernel<<<unsigned(ceil_div(c1 - c0, 128)), 128, 0, st>>>(
+          u3.p, u3.p + n, u3.p + 2 * n, flags.p, nx, ny, nz, dx, dx / dt, mu, to(i6), to(ig), to(iv), nullptr, nullptr,
+          c0, c1);
+      CK(cudaGetLastError());
+    });
   }
 
   // runner.rs:1648-1690: percentile summaries of gamma_dot and mu gamma_dot
@@ -1524,7 +1549,7 @@ struct Engine final : EngineBase {
     velocity_moments(u3);
     stress_field_kernel<<<unsigned(ceil_div(n, 128)), 128, 0, st>>>(u3.p, u3.p + n, u3.p + 2 * n, flags.p, nx, ny,
                                                                     nz, dx, dx / dt, mu, nullptr, nullptr, nullptr,
-                                                                    key.p, cnt.p, n);
+                                                                    key.p, cnt.p, int64_t(0), n);
     CK(cudaGetLastError());
     CK(cub::DeviceRadixSort::SortKeys(tmp.p, tmp_bytes, key.p, sorted.p, int(n), 0, 64, st));
     unsigned long long k = 0;
@@ -2128,16 +2153,15 @@ struct Engine final : EngineBase {
   }
   void get_scalar(int k, double* c) override {
     auto& sc = scalar(k);
-    DevBuf<double> dc;
-    dc.alloc(size_t(n));
-    const unsigned g = unsigned(ceil_div(n, 128));
+    read({{c, 1}}, [&](const std::vector<double*>& d, int64_t c0, int64_t c1) { gather_scalar(sc, d[0], c0, c1); });
+  }
+  void gather_scalar(ScalarStateT<A>& sc, double* out, int64_t c0, int64_t c1) {
+    const unsigned g = unsigned(ceil_div(c1 - c0, 128));
     if (sc.q == 7)
-      scalar_gather_kernel<7, A><<<g, 128, 0, st>>>(sc.h.p, sc.hplane, flags.p, nbr.p, nx, ny, nz, sc.parity, dc.p, n);
+      scalar_gather_kernel<7, A><<<g, 128, 0, st>>>(sc.h.p, sc.hplane, flags.p, nbr.p, nx, ny, nz, sc.parity, out, c0, c1);
     else
-      scalar_gather_kernel<Q, A><<<g, 128, 0, st>>>(sc.h.p, sc.hplane, flags.p, nbr.p, nx, ny, nz, sc.parity, dc.p, n);
+      scalar_gather_kernel<Q, A><<<g, 128, 0, st>>>(sc.h.p, sc.hplane, flags.p, nbr.p, nx, ny, nz, sc.parity, out, c0, c1);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(c, dc.p, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
   }
   // ---- checkpoint/restart (Solver::save / restore, solver.rs:4536-5066) ----
   const lbmb_config& config() const override { return cfg; }
@@ -2311,6 +2335,7 @@ struct Engine final : EngineBase {
         init_rho_h[c] = mom[size_t(c)];
         for (int k = 0; k < 3; ++k) init_u_h[size_t(3 * c + k)] = mom[size_t((k + 1) * n + c)];
       }
+    init_is_rest = false;
     d_init_u_ok = false;
     for (size_t k = 0; k < v.scalars.size(); ++k) {
       const ckpt::ScalarView& x = v.scalars[k];
@@ -2376,10 +2401,7 @@ struct Engine final : EngineBase {
     a.density = a0.density ? de.p : nullptr;
     dc.alloc(size_t(n));
     const unsigned g = unsigned(ceil_div(n, 128));
-    if (sc.q == 7)
-      scalar_gather_kernel<7, A><<<g, 128, 0, st>>>(sc.h.p, sc.hplane, flags.p, nbr.p, nx, ny, nz, sc.parity, dc.p, n);
-    else
-      scalar_gather_kernel<Q, A><<<g, 128, 0, st>>>(sc.h.p, sc.hplane, flags.p, nbr.p, nx, ny, nz, sc.parity, dc.p, n);
+    gather_scalar(sc, dc.p, 0, n);
     const int64_t nb = ceil_div(n, OXY_BLOCK);
     part.alloc(size_t(2 * nb));
     err.alloc(1);

@@ -139,20 +139,22 @@ __device__ __forceinline__ A scalar_conc(const A* hb, int64_t hpl, int64_t cell,
   return c;
 }
 
+// Concentration of cells [c0, c1), cell c0 at out[0].
 template <int SQ, class A>
 __global__ void scalar_gather_kernel(const A* hb, int64_t hpl, const uint8_t* flags, const uint32_t* nbr, int nx,
-                                     int ny, int nz, int sparity, double* out, int64_t n) {
-  const int64_t cell = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (cell >= n) return;
+                                     int ny, int nz, int sparity, double* out, int64_t c0, int64_t c1) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t cell = c0 + i;
+  if (cell >= c1) return;
   const uint8_t fl = flags[cell];
   if (fl & F_SOLID) {
-    out[cell] = 0.0;
+    out[i] = 0.0;
     return;
   }
   int x, y, z;
   cell_xyz(cell, nx, ny, x, y, z);
   const uint32_t mask = (fl & F_BOUNDARY) ? nbr[cell] : 0u;
-  out[cell] = double(scalar_conc<SQ, A>(hb, hpl, cell, x, y, z, nx, ny, nz, mask, sparity));
+  out[i] = double(scalar_conc<SQ, A>(hb, hpl, cell, x, y, z, nx, ny, nz, mask, sparity));
 }
 
 // Checkpoint image of a scalar's populations (the SCALAR_FIELDS h planes,

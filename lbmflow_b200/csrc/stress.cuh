@@ -114,23 +114,24 @@ __device__ __forceinline__ void strain_cell(const StrainArgs<S>& a, int64_t cell
 }
 
 template <int Q, class S>
-__global__ void strain_rate_kernel(StrainArgs<S> a, double* s6, double* gamma, int64_t n) {
+__global__ void strain_rate_kernel(StrainArgs<S> a, double* s6, double* gamma, int64_t c0, int64_t c1) {
   using A = typename Codec<S>::A;
-  const int64_t cell = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (cell >= n) return;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t cell = c0 + i;
+  if (cell >= c1) return;
   if (a.flags[cell] & F_SOLID) {  // solid cells report zero strain
     if (s6)
-      for (int k = 0; k < 6; ++k) s6[6 * cell + k] = 0.0;
-    if (gamma) gamma[cell] = 0.0;
+      for (int k = 0; k < 6; ++k) s6[6 * i + k] = 0.0;
+    if (gamma) gamma[i] = 0.0;
     return;
   }
   A pi[6], u[3];
   strain_cell<Q, S>(a, cell, pi, u);
   if (s6)
-    for (int k = 0; k < 6; ++k) s6[6 * cell + k] = double(pi[k]);
+    for (int k = 0; k < 6; ++k) s6[6 * i + k] = double(pi[k]);
   if (gamma) {
     const A ss = pi[0] * pi[0] + pi[1] * pi[1] + pi[2] * pi[2] + A(2) * (pi[3] * pi[3] + pi[4] * pi[4] + pi[5] * pi[5]);
-    gamma[cell] = double(sqrt(A(2) * ss));
+    gamma[i] = double(sqrt(A(2) * ss));
   }
 }
 
@@ -200,17 +201,17 @@ __device__ __forceinline__ void vel_grad_cell(const StrainArgs<S>& a, const doub
 
 // Velocity gradient of every cell (g9, n x 9 row-major) and / or WALE
 // (les.rs:120-211, Cw 0.325, Delta 1): nu_t and the omega+ field for the
-// next collision; clip bound nu_t_max when clip != 0; counts[0] = clipped
+// next collision, cells [c0, c1) (g9 and nu_t start at cell c0); clip bound nu_t_max when clip != 0; counts[0] = clipped
 // cells, maxbits = bits of the largest nu_t before clipping (non-negative,
 // so integer order is value order).
 template <int Q, class S>
 __global__ void wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typename Codec<S>::A>* wall_u, int per_x,
                             int per_y, int per_z, typename Codec<S>::A nu0, int clip,
                             typename Codec<S>::A nu_t_max, double* g9, double* nu_t, typename Codec<S>::A* omega,
-                            unsigned long long* counts, unsigned long long* maxbits, int64_t n) {
+                            unsigned long long* counts, unsigned long long* maxbits, int64_t c0, int64_t c1) {
   using A = typename Codec<S>::A;
-  const int64_t cell = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (cell >= n) return;
+  const int64_t cell = c0 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (cell >= c1) return;
   A g[3][3];
   if (a.flags[cell] & F_SOLID) {
     for (int i = 0; i < 9; ++i) g[i / 3][i % 3] = A(0);
@@ -218,7 +219,7 @@ __global__ void wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typena
     vel_grad_cell<Q, S>(a, u3, wall_u, per_x, per_y, per_z, cell, g);
   }
   if (g9)
-    for (int i = 0; i < 9; ++i) g9[9 * cell + i] = double(g[i / 3][i % 3]);
+    for (int i = 0; i < 9; ++i) g9[9 * (cell - c0) + i] = double(g[i / 3][i % 3]);
   if (!omega) return;
   A sr[3][3], g2[3][3], sd[3][3];
   for (int i = 0; i < 3; ++i)
@@ -251,21 +252,23 @@ __global__ void wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typena
     atomicAdd(counts, 1ull);
     nut = nu_t_max;
   }
-  if (nu_t) nu_t[cell] = double(nut);
+  if (nu_t) nu_t[cell - c0] = double(nut);
   omega[cell] = A(1) / (A(3) * (nu0 + nut) + A(0.5));
 }
 
 // compute_stress_field on the cached velocity moments (lattice units, f64;
-// solid entries are never read). key[i]: gamma_dot of a fluid cell when
+// solid entries are never read), cells [c0, c1), outputs from cell c0.
+// key[i]: gamma_dot of a fluid cell when
 // finite, else +NaN (solid or non-finite), so that an ascending sort puts
 // the values the percentile summary keeps first; *nfinite counts them.
 static __global__ void stress_field_kernel(const double* ux, const double* uy, const double* uz, const uint8_t* flags,
                                     int nx, int ny, int nz, double dx, double vscale, double mu, double* s6,
                                     double* gamma, double* viscous, double* key, unsigned long long* nfinite,
-                                    int64_t n) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+                                    int64_t c0, int64_t c1) {
+  const int64_t o = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t i = c0 + o;
   int finite = 0;
-  if (i < n) {
+  if (i < c1) {
     double gd = __longlong_as_double(0x7ff8000000000000ll);
     if (!(flags[i] & F_SOLID)) {
       int x, y, z;
@@ -296,20 +299,20 @@ static __global__ void stress_field_kernel(const double* ux, const double* uy, c
       const double ss = s[0] * s[0] + s[1] * s[1] + s[2] * s[2] + 2.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5]);
       const double v = sqrt(2.0 * ss);
       if (s6)
-        for (int k = 0; k < 6; ++k) s6[6 * i + k] = s[k];
-      if (gamma) gamma[i] = v;
-      if (viscous) viscous[i] = mu * v;
+        for (int k = 0; k < 6; ++k) s6[6 * o + k] = s[k];
+      if (gamma) gamma[o] = v;
+      if (viscous) viscous[o] = mu * v;
       if (isfinite(v)) {
         gd = v;
         finite = 1;
       }
     } else {
       if (s6)
-        for (int k = 0; k < 6; ++k) s6[6 * i + k] = 0.0;
-      if (gamma) gamma[i] = 0.0;
-      if (viscous) viscous[i] = 0.0;
+        for (int k = 0; k < 6; ++k) s6[6 * o + k] = 0.0;
+      if (gamma) gamma[o] = 0.0;
+      if (viscous) viscous[o] = 0.0;
     }
-    if (key) key[i] = gd;
+    if (key) key[o] = gd;
   }
   if (nfinite) {
     const unsigned b = __ballot_sync(0xffffffffu, finite);
