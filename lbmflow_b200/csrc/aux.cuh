@@ -205,7 +205,6 @@ __global__ void __launch_bounds__(RED_BLOCK) reduce_kernel(const S* fb, int64_t 
     for (int k = 0; k < 5; ++k) part[5 * blockIdx.x + k] = v[k];
 }
 
-// Sum block partials in block order (single thread: deterministic).
 // clear_body_force_field on the device: *nonuniform |= any slot of the
 // field differs from the base value (slot 0 when the slots cover every
 // cell, else zero), compared component-wise like the host check.
@@ -229,13 +228,22 @@ __global__ void field_zero_if_uniform_kernel(Vec4<A>* f, int64_t nslots, const i
     f[s] = Vec4<A>{A(0), A(0), A(0), A(0)};
 }
 
-static __global__ void reduce_finish_kernel(const double* part, int nblk, int width, double* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int k = 0; k < width; ++k) {
-    double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += part[width * b + k];
-    out[k] = s;
-  }
+// Sum of the block partials of one component in a fixed order: thread t takes
+// partials t, t + RED_BLOCK, ..., then a tree. (One thread adding the 1,184
+// partials waits for each load: 1.1 ms per component at B200's latency.)
+__device__ __forceinline__ double sum_partials(const double* part, int nblk, int width, int k, double* sh) {
+  double v[1] = {0.0};
+  for (int b = threadIdx.x; b < nblk; b += RED_BLOCK) v[0] += part[width * b + k];
+  block_sum<1>(v, sh);
+  return v[0];  // thread 0
+}
+
+// One block of RED_BLOCK threads per component.
+static __global__ void __launch_bounds__(RED_BLOCK) reduce_finish_kernel(const double* part, int nblk, int width,
+                                                                         double* out) {
+  __shared__ double sh[RED_BLOCK / 32];
+  const double s = sum_partials(part, nblk, width, int(blockIdx.x), sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
 }  // namespace lbmb

@@ -1316,7 +1316,7 @@ struct Engine final : EngineBase {
                                                          double(A(cfg.force[1])), double(A(cfg.force[2])),
                                                          n, red_part.p);
     CK(cudaGetLastError());
-    reduce_finish_kernel<<<1, 32, 0, st>>>(red_part.p, red_blocks, 5, red_out.p);
+    reduce_finish_kernel<<<5, RED_BLOCK, 0, st>>>(red_part.p, red_blocks, 5, red_out.p);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, red_out.p, 5 * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -2451,7 +2451,7 @@ struct Engine final : EngineBase {
       else
         scalar_cv_kernel<Q, A><<<red_blocks, RED_BLOCK, 0, st>>>(sc.h.p, sc.hplane, flags.p, nbr.p, nx, ny, nz,
                                                                   sc.parity, n, pass, sc.stats.p, nfluid, sc.part.p);
-      scalar_cv_finish_kernel<<<1, 32, 0, st>>>(sc.part.p, red_blocks, pass, sc.stats.p, nfluid, out);
+      scalar_cv_finish_kernel<<<1, RED_BLOCK, 0, st>>>(sc.part.p, red_blocks, pass, sc.stats.p, nfluid, out);
     }
     CK(cudaGetLastError());
   }

@@ -263,11 +263,11 @@ __global__ void __launch_bounds__(RED_BLOCK) scalar_cv_kernel(const A* hb, int64
   if (threadIdx.x == 0) part[blockIdx.x] = v[0];
 }
 
-static __global__ void scalar_cv_finish_kernel(const double* part, int nblk, int pass, double* stats, double nfluid,
-                                        double* cv_out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s = 0.0;
-  for (int b = 0; b < nblk; ++b) s += part[b];
+static __global__ void __launch_bounds__(RED_BLOCK)
+    scalar_cv_finish_kernel(const double* part, int nblk, int pass, double* stats, double nfluid, double* cv_out) {
+  __shared__ double sh[RED_BLOCK / 32];
+  const double s = sum_partials(part, nblk, 1, 0, sh);
+  if (threadIdx.x != 0) return;
   if (pass == 0) {
     stats[0] = s;
     return;
