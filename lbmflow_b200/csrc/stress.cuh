@@ -9,9 +9,10 @@
 //   bioprocess runner calls it, runner.rs:1648-1690): f64 central
 //   differences of the SI velocity (lattice velocity x dx/dt), one-sided
 //   next to a solid or the domain edge, gamma_dot = sqrt(2 S:S), viscous
-//   stress mu gamma_dot. The percentile summary (stress.rs:84-100) sorts the
-//   finite fluid values on the device (cub radix sort) and interpolates
-//   between ranks on the host.
+//   stress mu gamma_dot. The percentile summary (stress.rs:84-100) selects
+//   the values of its few ranks on the device: a histogram of the values'
+//   leading 16 bits, the bins the ranks fall in, and a sort of those bins'
+//   values only; the host interpolates between ranks.
 // * Wall-shear proxy (stress.rs:102-294): fluid cells with a solid among
 //   their 26 in-domain neighbours, compacted in cell order on the device.
 #pragma once
@@ -111,6 +112,41 @@ __device__ __forceinline__ void strain_cell(const StrainArgs<S>& a, int64_t cell
   const A scale = -(A(1) / (A(2.0 / 3.0) * r * a.tau_eff));
 #pragma unroll
   for (int k = 0; k < 6; ++k) pi[k] = pi[k] * scale;
+}
+
+// Cached velocity of a fluid cell (the arithmetic of moments_kernel).
+template <int Q, class S>
+__device__ __forceinline__ void cell_velocity(const StrainArgs<S>& a, int64_t cell, double (&u)[3]) {
+  using A = typename Codec<S>::A;
+  using L = Lat<Q>;
+  const uint8_t fl = a.flags[cell];
+  int x, y, z;
+  cell_xyz(cell, a.nx, a.ny, x, y, z);
+  const uint32_t mask = (fl & F_BOUNDARY) ? a.nbr[cell] : 0u;
+  A f[Q];
+  load_post_stream<Q, S>(a.fb, a.pl, cell, x, y, z, a.nx, a.ny, a.nz, mask, a.parity, f);
+  A dr = A(0), m0 = A(0), m1 = A(0), m2 = A(0);
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    dr = dr + f[q];
+    if (L::cx(q) == 1) m0 = m0 + f[q];
+    if (L::cx(q) == -1) m0 = m0 - f[q];
+    if (L::cy(q) == 1) m1 = m1 + f[q];
+    if (L::cy(q) == -1) m1 = m1 - f[q];
+    if (L::cz(q) == 1) m2 = m2 + f[q];
+    if (L::cz(q) == -1) m2 = m2 - f[q];
+  }
+  A Fx = a.gx, Fy = a.gy, Fz = a.gz;
+  if (fl & F_FORCED) {
+    const Vec4<A> v = a.fprev[a.fslot[cell]];
+    Fx = Fx + v.x;
+    Fy = Fy + v.y;
+    Fz = Fz + v.z;
+  }
+  const A inv = A(1) / (A(1) + dr);
+  u[0] = double((m0 + A(0.5) * Fx) * inv);
+  u[1] = double((m1 + A(0.5) * Fy) * inv);
+  u[2] = double((m2 + A(0.5) * Fz) * inv);
 }
 
 template <int Q, class S>
@@ -256,18 +292,23 @@ __global__ void wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typena
   omega[cell] = A(1) / (A(3) * (nu0 + nut) + A(0.5));
 }
 
+// Bin of a finite non-negative value: its exponent and four leading mantissa
+// bits (such values order like their bits; -0 counts as 0).
+constexpr int VALUE_BINS = 1 << 15;
+__device__ __forceinline__ int value_bin(double v) {
+  return int((unsigned long long)__double_as_longlong(v + 0.0) >> 48) & (VALUE_BINS - 1);
+}
+
 // compute_stress_field on the cached velocity moments (lattice units, f64;
 // solid entries are never read), cells [c0, c1), outputs from cell c0.
-// key[i]: gamma_dot of a fluid cell when
-// finite, else +NaN (solid or non-finite), so that an ascending sort puts
-// the values the percentile summary keeps first; *nfinite counts them.
+// key[i]: gamma_dot of a fluid cell when finite, else NaN (solid or
+// non-finite); hist counts the finite ones by bin.
 static __global__ void stress_field_kernel(const double* ux, const double* uy, const double* uz, const uint8_t* flags,
                                     int nx, int ny, int nz, double dx, double vscale, double mu, double* s6,
-                                    double* gamma, double* viscous, double* key, unsigned long long* nfinite,
+                                    double* gamma, double* viscous, double* key, unsigned int* hist,
                                     int64_t c0, int64_t c1) {
   const int64_t o = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t i = c0 + o;
-  int finite = 0;
   if (i < c1) {
     double gd = __longlong_as_double(0x7ff8000000000000ll);
     if (!(flags[i] & F_SOLID)) {
@@ -304,7 +345,11 @@ static __global__ void stress_field_kernel(const double* ux, const double* uy, c
       if (viscous) viscous[o] = mu * v;
       if (isfinite(v)) {
         gd = v;
-        finite = 1;
+        if (hist) {  // one add per bin and warp (a fluid at rest has one bin)
+          const int bin = value_bin(v);
+          const unsigned same = __match_any_sync(__activemask(), bin);
+          if ((threadIdx.x & 31) == unsigned(__ffs(int(same)) - 1)) atomicAdd(hist + bin, unsigned(__popc(same)));
+        }
       }
     } else {
       if (s6)
@@ -314,35 +359,149 @@ static __global__ void stress_field_kernel(const double* ux, const double* uy, c
     }
     if (key) key[o] = gd;
   }
-  if (nfinite) {
-    const unsigned b = __ballot_sync(0xffffffffu, finite);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(nfinite, (unsigned long long)__popc(b));
+}
+
+// The ranks of a percentile summary (stress.rs:296-309): floor and ceiling
+// ranks of the quantiles 0.5, 0.9, 0.95, 0.99, and the maximum.
+constexpr int N_RANKS = 9;
+struct RankSelect {
+  unsigned long long count;          // finite values
+  unsigned long long rank[N_RANKS];  // wanted ranks, then their positions among the selected values
+  unsigned long long n_selected;     // values in the bins of the ranks
+  unsigned long long above[2];       // values above the thresholds
+  unsigned int mark[VALUE_BINS / 32];  // bins of the ranks
+};
+
+// One block: turns the histogram into ranks, marked bins and each rank's
+// position among the marked bins' values in ascending order.
+constexpr int SELECT_BLOCK = 1024;
+static __global__ void __launch_bounds__(SELECT_BLOCK) select_ranks_kernel(const unsigned int* hist, RankSelect* r) {
+  constexpr int PER = VALUE_BINS / SELECT_BLOCK;  // consecutive bins of a thread: one mark word
+  static_assert(PER == 32, "a thread's bins are one mark word");
+  __shared__ unsigned long long part[SELECT_BLOCK];
+  __shared__ unsigned int words[SELECT_BLOCK];
+  __shared__ unsigned long long rank[N_RANKS], pos[N_RANKS];
+  const int t = int(threadIdx.x);
+  unsigned long long own = 0;
+  for (int k = 0; k < PER; ++k) own += hist[t * PER + k];
+  part[t] = own;
+  words[t] = 0u;
+  __syncthreads();
+  for (int d = 1; d < SELECT_BLOCK; d <<= 1) {  // inclusive scan
+    const unsigned long long v = t >= d ? part[t - d] : 0ull;
+    __syncthreads();
+    part[t] += v;
+    __syncthreads();
+  }
+  const unsigned long long n = part[SELECT_BLOCK - 1];
+  if (t < N_RANKS && n > 0) {
+    const double q[4] = {0.50, 0.90, 0.95, 0.99};
+    const double x = t < 8 ? q[t >> 1] * double(n - 1) : double(n - 1);
+    rank[t] = (unsigned long long)(t < 8 ? ((t & 1) ? ceil(x) : floor(x)) : x);
+  }
+  __syncthreads();
+  if (n > 0) {
+    for (int j = 0; j < N_RANKS; ++j) {
+      unsigned long long lo = part[t] - own;
+      if (rank[j] < lo || rank[j] >= part[t]) continue;
+      for (int k = 0; k < PER; ++k) {
+        const unsigned long long h = hist[t * PER + k];
+        if (rank[j] < lo + h) {
+          words[t] |= 1u << k;
+          pos[j] = rank[j] - lo;
+          break;
+        }
+        lo += h;
+      }
+    }
+  }
+  __syncthreads();
+  // values of the marked bins before each thread's
+  unsigned long long sel = 0;
+  for (int k = 0; k < PER; ++k)
+    if ((words[t] >> k) & 1u) sel += hist[t * PER + k];
+  const unsigned long long end = part[t];
+  __syncthreads();
+  part[t] = sel;
+  __syncthreads();
+  for (int d = 1; d < SELECT_BLOCK; d <<= 1) {
+    const unsigned long long v = t >= d ? part[t - d] : 0ull;
+    __syncthreads();
+    part[t] += v;
+    __syncthreads();
+  }
+  if (n > 0) {
+    for (int j = 0; j < N_RANKS; ++j) {
+      unsigned long long lo = end - own, before = part[t] - sel;
+      if (rank[j] < lo || rank[j] >= end) continue;
+      for (int k = 0; k < PER; ++k) {
+        const unsigned long long h = hist[t * PER + k];
+        if (rank[j] < lo + h) {
+          r->rank[j] = before + pos[j];
+          break;
+        }
+        lo += h;
+        if ((words[t] >> k) & 1u) before += h;
+      }
+    }
+  }
+  r->mark[t] = words[t];
+  if (t == 0) {
+    r->count = n;
+    r->n_selected = part[SELECT_BLOCK - 1];
   }
 }
 
-// Values of sorted[0, k) above t (scaled by mul first, as the reference
-// forms mu gamma_dot before it counts).
-static __global__ void count_above_kernel(const double* sorted, int64_t k, double mul, double t, unsigned long long* out) {
+// Values of the marked bins, in any order, and the counts above the
+// thresholds (values scaled first, as the reference forms mu gamma_dot before
+// it counts; thresholds +inf: none counted).
+static __global__ void select_values_kernel(const double* key, int64_t n, RankSelect* r, unsigned long long* cursor,
+                                            double* out, double t_gamma, double mu, double t_tau) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int above = (i < k) && (mul * sorted[i] > t);
-  const unsigned b = __ballot_sync(0xffffffffu, above);
-  if ((threadIdx.x & 31) == 0 && b) atomicAdd(out, (unsigned long long)__popc(b));
+  const double v = i < n ? key[i] : __longlong_as_double(0x7ff8000000000000ll);
+  const bool ok = isfinite(v);
+  const int lane = int(threadIdx.x) & 31;
+  const int bin = ok ? value_bin(v) : 0;
+  const bool take = ok && ((r->mark[bin >> 5] >> (bin & 31)) & 1u);
+  const unsigned b = __ballot_sync(0xffffffffu, take);
+  unsigned long long at = 0;
+  if (lane == 0 && b) at = atomicAdd(cursor, (unsigned long long)__popc(b));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (take) out[at + __popc(b & ((1u << lane) - 1u))] = v + 0.0;
+  const unsigned g = __ballot_sync(0xffffffffu, ok && v > t_gamma), w = __ballot_sync(0xffffffffu, ok && mu * v > t_tau);
+  if (lane == 0) {
+    if (g) atomicAdd(&r->above[0], (unsigned long long)__popc(g));
+    if (w) atomicAdd(&r->above[1], (unsigned long long)__popc(w));
+  }
 }
 
-// wall_shear_proxy per cell (dense): flag[i] = 1 for a fluid cell with a
-// solid among its 26 in-domain neighbours and a nonzero normal.
-template <class A>
-__global__ void wall_shear_kernel(const double* ux, const double* uy, const double* uz, const uint8_t* flags,
-                                  const Vec4<A>* wall_u, int nx, int ny, int nz, double dx, double vscale, double rho,
-                                  double mu, uint8_t* flag, double* tau, double* yplus, double* upar, double* normal,
-                                  int64_t n) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  flag[i] = 0;
+// The selected ranks' values from the sorted selection.
+static __global__ void rank_values_kernel(const double* sorted, const RankSelect* r, double* out) {
+  if (threadIdx.x < N_RANKS) out[threadIdx.x] = sorted[r->rank[threadIdx.x]];
+}
+
+// A cell of the wall-shear proxy: a fluid cell with a solid among its 26
+// in-domain neighbours and a nonzero wall normal (unit), and the number of
+// those solids.
+struct WallCell {
+  int64_t cell;
+  double normal[3];
+  double count;
+};
+
+// wall_shear_proxy's geometry per cell, which no step changes: flag[i] = 1
+// where the proxy has an entry (cells == null), or the entries of the listed
+// cells.
+static __global__ void wall_cells_kernel(const uint8_t* flags, int nx, int ny, int nz, uint8_t* flag,
+                                         const int64_t* cells, WallCell* out, int64_t n) {
+  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int64_t i = cells ? cells[t] : t;
+  if (!cells) flag[i] = 0;
   if (flags[i] & F_SOLID) return;
   int x, y, z;
   cell_xyz(i, nx, ny, x, y, z);
-  double nrm[3] = {0.0, 0.0, 0.0}, wu[3] = {0.0, 0.0, 0.0}, count = 0.0;
+  WallCell w = {i, {0.0, 0.0, 0.0}, 0.0};
   for (int dz = -1; dz <= 1; ++dz)
     for (int dy = -1; dy <= 1; ++dy)
       for (int dxo = -1; dxo <= 1; ++dxo) {
@@ -351,51 +510,71 @@ __global__ void wall_shear_kernel(const double* ux, const double* uy, const doub
         if (a < 0 || b < 0 || c < 0 || a >= nx || b >= ny || c >= nz) continue;
         const int64_t j = (int64_t(c) * ny + b) * nx + a;
         if (!(flags[j] & F_SOLID)) continue;
-        nrm[0] += double(dxo);
-        nrm[1] += double(dy);
-        nrm[2] += double(dz);
-        const Vec4<A> w = wall_u[j];
-        wu[0] += double(w.x) * vscale;
-        wu[1] += double(w.y) * vscale;
-        wu[2] += double(w.z) * vscale;
-        count += 1.0;
+        w.normal[0] += double(dxo);
+        w.normal[1] += double(dy);
+        w.normal[2] += double(dz);
+        w.count += 1.0;
       }
-  if (count == 0.0) return;
-  const double mag = sqrt(nrm[0] * nrm[0] + nrm[1] * nrm[1] + nrm[2] * nrm[2]);
+  if (w.count == 0.0) return;
+  const double mag = sqrt(w.normal[0] * w.normal[0] + w.normal[1] * w.normal[1] + w.normal[2] * w.normal[2]);
   if (mag == 0.0) return;
-  for (int k = 0; k < 3; ++k) {
-    nrm[k] /= mag;
-    wu[k] /= count;
+  if (!cells) {
+    flag[i] = 1;
+    return;
   }
-  const double u[3] = {ux[i] * vscale - wu[0], uy[i] * vscale - wu[1], uz[i] * vscale - wu[2]};
-  const double un = u[0] * nrm[0] + u[1] * nrm[1] + u[2] * nrm[2];
-  const double t[3] = {u[0] - un * nrm[0], u[1] - un * nrm[1], u[2] - un * nrm[2]};
+  for (int k = 0; k < 3; ++k) w.normal[k] /= mag;
+  out[t] = w;
+}
+
+// wall_shear_proxy (stress.rs:102-294) of entries [c0, c1) of the wall-cell
+// list, 8 values each in lbmb_wall_shear's layout; the velocity is computed
+// for the listed cells only.
+template <int Q, class S>
+__global__ void wall_shear_kernel(StrainArgs<S> g, const Vec4<typename Codec<S>::A>* wall_u, const WallCell* list,
+                                  double dx, double vscale, double rho, double mu, double* out, int64_t c0,
+                                  int64_t c1) {
+  const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (c0 + r >= c1) return;
+  const WallCell w = list[c0 + r];
+  const int64_t i = w.cell;
+  int x, y, z;
+  cell_xyz(i, g.nx, g.ny, x, y, z);
+  double wu[3] = {0.0, 0.0, 0.0};
+  for (int dz = -1; dz <= 1; ++dz)
+    for (int dy = -1; dy <= 1; ++dy)
+      for (int dxo = -1; dxo <= 1; ++dxo) {
+        if (!dxo && !dy && !dz) continue;
+        const int a = x + dxo, b = y + dy, c = z + dz;
+        if (a < 0 || b < 0 || c < 0 || a >= g.nx || b >= g.ny || c >= g.nz) continue;
+        const int64_t j = (int64_t(c) * g.ny + b) * g.nx + a;
+        if (!(g.flags[j] & F_SOLID)) continue;
+        const Vec4<typename Codec<S>::A> v = wall_u[j];
+        wu[0] += double(v.x) * vscale;
+        wu[1] += double(v.y) * vscale;
+        wu[2] += double(v.z) * vscale;
+      }
+  double u[3];
+  cell_velocity<Q, S>(g, i, u);
+  for (int k = 0; k < 3; ++k) u[k] = u[k] * vscale - wu[k] / w.count;
+  const double un = u[0] * w.normal[0] + u[1] * w.normal[1] + u[2] * w.normal[2];
+  const double t[3] = {u[0] - un * w.normal[0], u[1] - un * w.normal[1], u[2] - un * w.normal[2]};
   const double up = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
   const double y_m = 0.5 * dx;
   const double tw = mu * up / y_m;
-  flag[i] = 1;
-  tau[i] = tw;
-  yplus[i] = y_m * sqrt(tw / rho) / (mu / rho);
-  upar[i] = up;
-  for (int k = 0; k < 3; ++k) normal[3 * i + k] = nrm[k];
+  double* const o = out + 8 * r;
+  o[0] = __longlong_as_double(i);
+  o[1] = tw;
+  o[2] = y_m * sqrt(tw / rho) / (mu / rho);
+  o[3] = up;
+  o[4] = y_m;
+  o[5] = w.normal[0];
+  o[6] = w.normal[1];
+  o[7] = w.normal[2];
 }
 
 static __global__ void iota_kernel(int64_t* out, int64_t n) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) out[i] = i;
-}
-
-// Rows of the compacted wall cells: {tau_w, y+, |u_par|, normal x3}.
-static __global__ void gather_wall_kernel(const int64_t* sel, int64_t k, const double* tau, const double* yplus,
-                                   const double* upar, const double* normal, double* out) {
-  const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (r >= k) return;
-  const int64_t i = sel[r];
-  out[7 * r] = tau[i];
-  out[7 * r + 1] = yplus[i];
-  out[7 * r + 2] = upar[i];
-  for (int a = 0; a < 3; ++a) out[7 * r + 3 + a] = normal[3 * i + a];
-  out[7 * r + 6] = 0.0;
 }
 
 }  // namespace lbmb
