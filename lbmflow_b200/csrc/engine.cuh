@@ -1436,9 +1436,12 @@ struct Engine final : EngineBase {
   void omega_install() {
     if (cfg.smagorinsky_cs > 0.0)
       throw Error(LBMB_ERR_UNSUPPORTED, "a relaxation field and the Smagorinsky option cannot be combined");
+    // a field that replaces another one in the same array leaves every
+    // captured launch as it is
+    const bool same = omega_on && omega_kind_ok(kernel_mode);
     omega_on = true;
     if (!omega_kind_ok(kernel_mode)) kernel_mode = window_ok() ? LBMB_SWEEP_WINDOW : LBMB_SWEEP_DIRECT;
-    invalidate_graphs();
+    if (!same) invalidate_graphs();
   }
 
   void set_omega_field(const double* omega) override {
@@ -2528,6 +2531,29 @@ struct Engine final : EngineBase {
     run_graph = false;
   }
 
+  // The spans of a run of `steps` steps from step parity par: visit(gi) for a
+  // graph of RUN_G >> gi steps, visit(-1) for a single step; no span crosses
+  // a divergence check.
+  template <class Visit>
+  static void for_spans(int64_t steps, int par, bool graphs, const Visit& visit) {
+    int64_t done = 0;
+    while (done < steps) {
+      const int64_t stop = std::min(steps, (done / DIVERGE_EVERY + 1) * DIVERGE_EVERY);
+      while (done < stop) {
+        int gi = 0;
+        while (gi < RUN_NG && stop - done < (RUN_G >> gi)) ++gi;
+        if (graphs && par == 0 && gi < RUN_NG) {
+          visit(gi);
+          done += RUN_G >> gi;
+        } else {
+          visit(-1);
+          ++done;
+          par ^= 1;
+        }
+      }
+    }
+  }
+
   void run_reserve(int64_t steps) {
     if (steps <= run_cap && run_counter.p) return;
     const int64_t cap = std::max<int64_t>({steps, 2 * run_cap, int64_t(1024)});
@@ -2600,17 +2626,21 @@ struct Engine final : EngineBase {
         key.sc_par[i] = scalars[i]->parity ^ parity;
       }
       if (run_graph && std::memcmp(&key, &run_key, sizeof(key)) != 0) drop_run_graphs();
-      if (!run_graph) {
+      // the graph sizes that this call's spans use and that are not there yet
+      bool need[RUN_NG] = {false, false, false, false}, any = false;
+      for_spans(steps, parity, true, [&](int gi) {
+        if (gi >= 0 && !run_graphs[gi]) need[gi] = any = true;
+      });
+      if (any) {
         // capture from parity 0 with the scalar parities the graph will
         // start from, then put the host state back
         const int par0 = parity;
         std::vector<int> spar(scalars.size());
-        for (size_t i = 0; i < scalars.size(); ++i) {
-          spar[i] = scalars[i]->parity;
-          scalars[i]->parity = key.sc_par[i];
-        }
+        for (size_t i = 0; i < scalars.size(); ++i) spar[i] = scalars[i]->parity;
         const bool fpres = field_present, fstale = fprev_stale;
         for (int gi = 0; gi < RUN_NG; ++gi) {
+          if (!need[gi]) continue;
+          for (size_t i = 0; i < scalars.size(); ++i) scalars[i]->parity = key.sc_par[i];
           parity = 0;
           cudaGraph_t g;
           CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -2633,33 +2663,24 @@ struct Engine final : EngineBase {
     }
     CK(cudaEventRecord(ev0, st));
     int64_t done = 0;
-    while (done < steps) {
-      // next divergence check after step number `check` (1-based)
-      const int64_t check = (done / DIVERGE_EVERY + 1) * DIVERGE_EVERY;
-      const int64_t stop = std::min(steps, check);
-      while (done < stop) {
-        int gi = 0;
-        while (gi < RUN_NG && stop - done < (RUN_G >> gi)) ++gi;
-        if (use_graph && parity == 0 && gi < RUN_NG) {
-          CK(cudaGraphLaunch(run_graphs[gi], st));
-          done += RUN_G >> gi;
-          launches += RUN_G >> gi;
-          field_present = true;
-          fprev_stale = false;
-        } else {
-          one_step(done);
-          ++done;
-        }
+    for_spans(steps, parity, use_graph, [&](int gi) {
+      if (run_diverged) return;
+      if (gi >= 0) {
+        CK(cudaGraphLaunch(run_graphs[gi], st));
+        done += RUN_G >> gi;
+        launches += RUN_G >> gi;
+        field_present = true;
+        fprev_stale = false;
+      } else {
+        one_step(done);
+        ++done;
       }
-      if (done == check) {
+      if (done % DIVERGE_EVERY == 0) {
         double r[5];
         reduce_all(r);  // synchronizes the stream
-        if (!std::isfinite(r[0] + r[1])) {
-          run_diverged = true;
-          break;
-        }
+        run_diverged = !std::isfinite(r[0] + r[1]);
       }
-    }
+    });
     run_executed = done;
     CK(cudaEventRecord(ev1, st));
     CK(cudaEventSynchronize(ev1));
