@@ -152,6 +152,7 @@ struct EngineBase {
   virtual int enable_scalar(int q, double d) = 0;
   virtual void set_scalar(int k, const double* c) = 0;
   virtual void get_scalar(int k, double* c) = 0;
+  virtual double scalar_cv(int k) = 0;
   virtual void run_impeller(int b, const lbmb_ibm_config& cfg, int64_t steps, int k, int64_t probe_every,
                             double* torque, double* ff, double* cv, int32_t* iters) = 0;
   virtual void run_status(int64_t* executed, int32_t* diverged) = 0;
@@ -2487,6 +2488,17 @@ struct Engine final : EngineBase {
     CK(cudaGetLastError());
   }
 
+  // qoi::scalar_cv (qoi.rs:507-532): NaN without fluid cells or with a zero
+  // mean.
+  double scalar_cv(int k) override {
+    ScalarStateT<A>& sc = scalar(k);
+    enqueue_cv(sc, nullptr, double(n - solid_count()));
+    double cv = 0.0;
+    CK(cudaMemcpyAsync(&cv, sc.stats.p + 1, sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    return cv;
+  }
+
   // ---- runner loop ------------------------------------------------------
   // Series buffers of the runner (torque, fluid force, IBM iterations, CV,
   // step counter), kept on the handle and grown only when a longer run needs
@@ -2786,6 +2798,10 @@ struct Engine final : EngineBase {
     BodyState& B = body_for(ac.body, c);
     const int nsweep = c.max_iterations;
     const int64_t nseg = ceil_div(N, K);
+    // Whole segments replay as graphs where they repeat often enough: each
+    // buffer's graph is used every other segment, and capturing and
+    // instantiating one costs about two eager passes of its launches.
+    const bool graphs = nseg >= 6;
     const size_t fsz = size_t(Q) * size_t(plane);
     const size_t ns3 = size_t(std::max<int64_t>(nslots, 1));
     sync();
@@ -2824,7 +2840,7 @@ struct Engine final : EngineBase {
       if (nslots)
         CK(cudaMemcpyAsync(ck_fp.p + size_t(seg) * ns3, fprev.p, size_t(nslots) * sizeof(Vec4<A>),
                            cudaMemcpyDeviceToDevice, st));
-      if (len == K) {
+      if (len == K && graphs) {
         if (!g_fwd) {
           const int par0 = parity;
           g_fwd = capture([&] {
@@ -2938,8 +2954,6 @@ struct Engine final : EngineBase {
     cleanup.ss = {sb, sb2};
     cleanup.es = {e_fork, e_join, e_rec[0], e_rec[1], e_bwd[0], e_bwd[1]};
     const IbmArgs a0 = ibm_args(B, c);
-    const unsigned gs = unsigned(std::max<int64_t>(1, ceil_div(B.ns, ADJ_BLOCK)));
-    const unsigned gm = unsigned(std::max<int64_t>(1, ceil_div(B.nm, ADJ_BLOCK)));
     const unsigned gc = unsigned(ceil_div(n, ADJ_BLOCK));
     // recomputation of len steps from the restored checkpoint into b
     auto recompute = [&](SegBuf& b, int64_t len) {
@@ -3008,14 +3022,7 @@ struct Engine final : EngineBase {
         ab.xbar = xbar.p;
         ab.grad = grad.p;
         ab.tbar_step = b.tb.p + i;
-        for (int k = nsweep - 1; k >= 0; --k) {
-          adj_ibm_marker_kernel<<<gm, ADJ_BLOCK, 0, sb>>>(ab, k);
-          adj_ibm_slot_kernel<<<gs, ADJ_BLOCK, 0, sb>>>(ab, k);
-        }
-        adj_ibm_mob_slot_kernel<<<gs, ADJ_BLOCK, 0, sb>>>(ab);
-        adj_ibm_mob_marker_kernel<<<gm, ADJ_BLOCK, 0, sb>>>(ab);
-        adj_ibm_fbar_kernel<Q, A><<<gs, ADJ_BLOCK, 0, sb>>>(ab, lam_out, plane);
-        CK(cudaGetLastError());
+        launch_cluster(adj_ibm_kernel<Q, A>, 1, ADJ_IBM_THREADS, sb, ab, nsweep, lam_out, plane);
       }
     };
     auto capture_on = [&](cudaStream_t s0, auto&& body) {
@@ -3049,7 +3056,7 @@ struct Engine final : EngineBase {
       parity = 0;
       field_present = true;
       fprev_stale = false;
-      if (len == K) {
+      if (len == K && graphs) {
         if (!g_rec[bi]) {
           g_rec[bi] = capture_on(st, [&] { recompute(b, K); });
           cleanup.gs.push_back(g_rec[bi]);
@@ -3058,6 +3065,7 @@ struct Engine final : EngineBase {
         parity = 0;
       } else {
         recompute(b, len);
+        parity = 0;
       }
       CK(cudaEventRecord(e_rec[bi], st));
       used[bi] = true;
@@ -3072,7 +3080,7 @@ struct Engine final : EngineBase {
         CK(cudaMemcpyAsync(mu0.p, mu1.p, 3 * ns3 * sizeof(double), cudaMemcpyDeviceToDevice, sb));
         lam_in_is_0 = true;
       }
-      if (len == K) {
+      if (len == K && graphs) {
         if (!g_bwd[bi]) {
           g_bwd[bi] = capture_on(sb, [&] { backward(b, K); });
           cleanup.gs.push_back(g_bwd[bi]);

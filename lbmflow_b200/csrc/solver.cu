@@ -439,34 +439,7 @@ int lbmb_scalar_cv(lbmb_solver* h, int32_t k, double* cv) {
   return guarded([&] {
     NEED(h);
     if (!cv) throw Error(LBMB_ERR_INVALID, "null output");
-    const int64_t n = h->e->cells();
-    std::vector<double> c(static_cast<size_t>(n));
-    h->e->get_scalar(k, c.data());
-    const auto& solid = h->e->solid();
-    // qoi::scalar_cv (qoi.rs:507-532): population std / |mean| over fluid cells.
-    int64_t cnt = 0;
-    double sum = 0.0;
-    for (int64_t i = 0; i < n; ++i)
-      if (!solid[i]) {
-        ++cnt;
-        sum += c[i];
-      }
-    if (cnt == 0) {
-      *cv = std::nan("");
-      return;
-    }
-    const double mean = sum / double(cnt);
-    if (mean == 0.0) {
-      *cv = std::nan("");
-      return;
-    }
-    double var = 0.0;
-    for (int64_t i = 0; i < n; ++i)
-      if (!solid[i]) {
-        const double d = c[i] - mean;
-        var += d * d;
-      }
-    *cv = std::sqrt(var / double(cnt)) / std::fabs(mean);
+    *cv = h->e->scalar_cv(k);
   });
 }
 
