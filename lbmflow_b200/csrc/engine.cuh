@@ -325,9 +325,24 @@ struct Engine final : EngineBase {
     rows_aligned = (nx % TmaWin<S>::PAD == 0) && ((int64_t(nx) * ny) % TmaWin<S>::PAD == 0);
     // default sweep: the lean kernel where it applies (TRT/BGK, fp32/16-bit
     // storage, no uniform force), else cp.async (4/8-byte storage), the
-    // window kernel (16-bit storage) or direct loads (uniform force)
+    // window kernel (16-bit storage) or direct loads (uniform force); on a
+    // large grid with even nx the pair kernel instead of these. Runner step
+    // on B200, smaller grids first, default before / pair, us: D3Q27 fp32 48 x
+    // 48 x 60 24.8 / 25.9, 72 x 72 x 90 29.1 / 29.2, 96 x 96 x 120 62.1 /
+    // 61.7, 128 x 128 x 160 137 / 122; D3Q27 fp16 48 24.9 / 25.8, 96 67 / 51;
+    // D3Q19 fp16 96 35.1 / 34.5, 128 71 / 57; D3Q19 fp32 112 61 / 64, 128 87 /
+    // 79, 160 160 / 137.
     if (sizeof(S) < 4) kernel_mode = window_ok() ? LBMB_SWEEP_WINDOW : LBMB_SWEEP_DIRECT;
     if (lean_ok(coll)) kernel_mode = LBMB_SWEEP_LEAN;
+    const bool wide_trt = sizeof(S) == 4 && coll == COLL_TRT;
+    if (std::is_same<A, float>::value && nx % 2 == 0 && !has_uniform_force() && (coll == COLL_TRT || Q == 27) &&
+        n >= (int64_t(1) << (wide_trt ? 21 : 20)) && int64_t(Q + 1) * plane < (int64_t(1) << 31)) {
+      chosen_over = kernel_mode;
+      kernel_mode = LBMB_SWEEP_PAIR;
+      pair_minb[0] = PAIR_STAGED + 3;
+      pair_minb[1] = sizeof(S) == 4 ? 3 : 4;
+      prepare_pair_variant();
+    }
     red_blocks = int(std::min<int64_t>(ceil_div(n, RED_BLOCK), 1184));
     red_part.alloc(size_t(red_blocks) * 5);
     red_out.alloc(8);
@@ -588,6 +603,7 @@ struct Engine final : EngineBase {
     if (kind == LBMB_SWEEP_LEAN && !lean_ok(coll))
       throw Error(LBMB_ERR_UNSUPPORTED, "the lean sweep needs TRT/BGK, fp32/fp16/bf16 storage and no uniform body force");
     kernel_mode = kind;
+    chosen_over = -1;
     invalidate_graphs();
   }
   int sweep_kernel() const override { return kernel_mode; }
@@ -595,7 +611,25 @@ struct Engine final : EngineBase {
   // blocks per SM (4 = 128 registers with a 3-tile ring, 5 = 96 with 3,
   // 6 = 80 with 2); the persistent grid fills every resident slot.
   int async_minb[2] = {4, 4};
+  // The kind in whose place a large grid starts on the pair kernel (-1: the
+  // kind was set, or there is no such choice). A variant set on a solver whose
+  // kind was never set names that kind's budgets, as on any other grid.
+  int chosen_over = -1;
+
   void set_sweep_variant(int even, int odd) override {
+    if (chosen_over >= 0) {
+      const int pair_kind = kernel_mode, base = chosen_over;
+      chosen_over = -1;
+      kernel_mode = base;
+      try {
+        set_sweep_variant(even, odd);
+      } catch (...) {
+        kernel_mode = pair_kind;
+        chosen_over = base;
+        throw;
+      }
+      return;
+    }
     if (kernel_mode == LBMB_SWEEP_ASYNC) {
       auto ok = [](int v) { return v >= 4 && v <= 6; };
       if (!ok(even) || !ok(odd))
@@ -1156,6 +1190,7 @@ struct Engine final : EngineBase {
       }
     }
     kernel_mode = cands[best].kind;
+    chosen_over = -1;
     if (kernel_mode == LBMB_SWEEP_LEAN) {
       lean_minb[0] = cands[best].ev;
       lean_minb[1] = cands[best].od;
@@ -1441,7 +1476,10 @@ struct Engine final : EngineBase {
     // captured launch as it is
     const bool same = omega_on && omega_kind_ok(kernel_mode);
     omega_on = true;
-    if (!omega_kind_ok(kernel_mode)) kernel_mode = window_ok() ? LBMB_SWEEP_WINDOW : LBMB_SWEEP_DIRECT;
+    if (!omega_kind_ok(kernel_mode)) {
+      kernel_mode = window_ok() ? LBMB_SWEEP_WINDOW : LBMB_SWEEP_DIRECT;
+      chosen_over = -1;
+    }
     if (!same) invalidate_graphs();
   }
 
