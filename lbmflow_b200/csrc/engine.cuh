@@ -339,8 +339,10 @@ struct Engine final : EngineBase {
         n >= (int64_t(1) << (wide_trt ? 21 : 20)) && int64_t(Q + 1) * plane < (int64_t(1) << 31)) {
       chosen_over = kernel_mode;
       kernel_mode = LBMB_SWEEP_PAIR;
-      pair_minb[0] = PAIR_STAGED + 3;
-      pair_minb[1] = sizeof(S) == 4 ? 3 : 4;
+      // budgets the autotuner picks there (fp32 D3Q27 runner step: 4/4 112,
+      // staged 3 / 3 119 us; fp16 D3Q19: staged 3 / 4)
+      pair_minb[0] = coll == COLL_CM ? 4 : PAIR_STAGED + 3;
+      pair_minb[1] = 4;
       prepare_pair_variant();
     }
     red_blocks = int(std::min<int64_t>(ceil_div(n, RED_BLOCK), 1184));

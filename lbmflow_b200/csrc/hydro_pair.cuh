@@ -215,6 +215,17 @@ __device__ __forceinline__ void cm_bwd2(float2& k0, float2& k1, float2& k2, floa
   k2 = fp;
 }
 
+// The same with the moments of order 1 and 2 already halved (the transform is
+// linear, so the halves are taken once at its input): hu = u/2, hu2 = u^2/2,
+// u2 = 2u.
+__device__ __forceinline__ void cm_bwd2h(float2& k0, float2& k1, float2& k2, float2 hu, float2 hu2, float2 u2) {
+  const float2 m1 = fma2(hu, k0, k1);
+  const float2 m2 = fma2(hu2, k0, fma2(u2, k1, k2));
+  k1 = fma2(bc2(-2.f), m2, k0);
+  k0 = sub2(m2, m1);
+  k2 = add2(m2, m1);
+}
+
 // D3Q27 central-moment collision (kernels.rs:406-533, no force) of two
 // cells in float2 lanes, in the regularized form of collide_cm_x2
 // (hydro_async.cuh): f' = feq + T^-1 K', where K' holds only the five
@@ -284,9 +295,11 @@ __device__ __forceinline__ float2 cm_pair_reg(float2 (&f)[Q], const HydroParams<
   const float2 osc = fma2(os, mul2(usq, bc2(-0.16f)), os);
   const float2 keep = sub2(bc2(1.f), make_float2(fminf(osc.x, 2.f), fminf(osc.y, 2.f)));
   const float2 bulk = mul2(add2(add2(pxx, pyy), pzz), bc2(1.f / 3.f));
-  const float2 k200 = mul2(keep, sub2(pxx, bulk)), k020 = mul2(keep, sub2(pyy, bulk));
-  const float2 k002 = mul2(keep, sub2(pzz, bulk));
-  const float2 k110 = mul2(keep, pxy), k101 = mul2(keep, pxz), k011 = mul2(keep, pyz);
+  // moments of order 1 and 2 along y and z halved for cm_bwd2h
+  const float2 kh = mul2(keep, bc2(0.5f));
+  const float2 k200 = mul2(keep, sub2(pxx, bulk)), k020 = mul2(kh, sub2(pyy, bulk));
+  const float2 k002 = mul2(kh, sub2(pzz, bulk));
+  const float2 k110 = mul2(kh, pxy), k101 = mul2(kh, pxz), k011 = mul2(mul2(kh, bc2(0.5f)), pyz);
   // x pass: G[a][b][c], a = c_x + 1, on the six order-2 lines (b, c)
   const float2 ux2 = mul2(ux, ux);
   const float2 s0m = mul2(bc2(0.5f), sub2(ux2, ux)), s0p = mul2(bc2(0.5f), add2(ux2, ux));
@@ -315,18 +328,19 @@ __device__ __forceinline__ float2 cm_pair_reg(float2 (&f)[Q], const HydroParams<
   // y pass over b for each (a, c): c = 0 full, c = 1 without order 2,
   // c = 2 order 0 only
   const float2 uy2 = mul2(uy, uy);
-  const float2 t0m = mul2(bc2(0.5f), sub2(uy2, uy)), t0p = mul2(bc2(0.5f), add2(uy2, uy));
+  const float2 huy = mul2(bc2(0.5f), uy), huy2 = mul2(bc2(0.5f), uy2), uyd = add2(uy, uy);
+  const float2 t0m = sub2(huy2, huy), t0p = add2(huy2, huy);
   const float2 t00 = sub2(bc2(1.f), uy2);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    cm_bwd2(G[a][0][0], G[a][1][0], G[a][2][0], uy);
+    cm_bwd2h(G[a][0][0], G[a][1][0], G[a][2][0], huy, huy2, uyd);
     {
       const float2 k0 = G[a][0][1], k1 = G[a][1][1];
-      const float2 m1 = fma2(uy, k0, k1);
-      const float2 m2 = mul2(uy, fma2(uy, k0, mul2(bc2(2.f), k1)));
-      G[a][0][1] = mul2(bc2(0.5f), sub2(m2, m1));
-      G[a][1][1] = sub2(k0, m2);
-      G[a][2][1] = mul2(bc2(0.5f), add2(m2, m1));
+      const float2 m1 = fma2(huy, k0, k1);
+      const float2 m2 = fma2(huy2, k0, mul2(uyd, k1));
+      G[a][0][1] = sub2(m2, m1);
+      G[a][1][1] = fma2(bc2(-2.f), m2, k0);
+      G[a][2][1] = add2(m2, m1);
     }
     {
       const float2 k0 = G[a][0][2];
@@ -336,21 +350,40 @@ __device__ __forceinline__ float2 cm_pair_reg(float2 (&f)[Q], const HydroParams<
     }
   }
   // z pass over c for each (a, b)
+  const float2 huz = mul2(bc2(0.5f), uz), huz2 = mul2(huz, uz), uzd = add2(uz, uz);
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) cm_bwd2(G[a][b][0], G[a][b][1], G[a][b][2], uz);
-  // f' = feq + G: w (drho + rho (3 cu + 4.5 cu^2 - 1.5 u^2))
+    for (int b = 0; b < 3; ++b) cm_bwd2h(G[a][b][0], G[a][b][1], G[a][b][2], huz, huz2, uzd);
+  // f' = feq + G, opposite directions together: w (drho + rho (4.5 cu^2 -
+  // 1.5 u^2)) +- 3 w rho cu
   const float2 nusq = mul2(bc2(-1.5f), usq);
+  f[0] = fma2(bc2(float(L::w(0))), fma2(rho, nusq, drho), G[1][1][1]);
+  float2 wr = bc2(0.f), wd = bc2(0.f), w3 = bc2(0.f), n3 = bc2(0.f);
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    float2 cu = L::cx(q) ? (L::cx(q) > 0 ? ux : mul2(ux, bc2(-1.f))) : bc2(0.f);
-    if (L::cy(q)) cu = L::cy(q) > 0 ? add2(cu, uy) : sub2(cu, uy);
-    if (L::cz(q)) cu = L::cz(q) > 0 ? add2(cu, uz) : sub2(cu, uz);
-    const float2 inner = fma2(cu, fma2(bc2(4.5f), cu, bc2(3.f)), nusq);
-    const float2 v = fma2(bc2(float(L::w(q))), fma2(rho, inner, drho), G[L::cx(q) + 1][L::cy(q) + 1][L::cz(q) + 1]);
-    f[q].x = rest0 ? f[q].x : v.x;
-    f[q].y = rest1 ? f[q].y : v.y;
+  for (int k = 0; k < NP; ++k) {
+    const int a = 2 * k + 1, b = a + 1;
+    if (k == 0 || wclass<Q>(a) != wclass<Q>(a - 2)) {
+      const float w = float(L::w(a));
+      wr = mul2(bc2(w), rho);
+      wd = mul2(bc2(w), drho);
+      w3 = mul2(bc2(3.f), wr);
+      n3 = mul2(bc2(-3.f), wr);
+    }
+    float2 cu = L::cx(a) ? ux : (L::cy(a) ? uy : uz);
+    if (L::cx(a) && L::cy(a)) cu = L::cy(a) > 0 ? add2(cu, uy) : sub2(cu, uy);
+    if ((L::cx(a) || L::cy(a)) && L::cz(a)) cu = L::cz(a) > 0 ? add2(cu, uz) : sub2(cu, uz);
+    const float2 P = fma2(wr, fma2(bc2(4.5f), mul2(cu, cu), nusq), wd);
+    f[a] = fma2(w3, cu, add2(P, G[L::cx(a) + 1][L::cy(a) + 1][L::cz(a) + 1]));
+    f[b] = fma2(n3, cu, add2(P, G[L::cx(b) + 1][L::cy(b) + 1][L::cz(b) + 1]));
+  }
+  // a lane at exact rest keeps its populations, which are w (rho - 1)
+  if (rest0 || rest1) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (rest0) f[q].x = float(L::w(q) * (double(rho.x) - 1.0));
+      if (rest1) f[q].y = float(L::w(q) * (double(rho.y) - 1.0));
+    }
   }
   return rho;
 }
@@ -400,12 +433,20 @@ __device__ __forceinline__ float2 ld2_odd(const S* p) {
 //     own slot (bounce-back); the tile list marks the tiles holding such
 //     cells (TILE_BND), and the warp loads their solid-neighbour masks one
 //     tile ahead, so the selection needs no extra round trip;
-//   stores: a link whose downstream cell is solid writes the cell's own
-//     slot (odd step), and an inactive cell of the pair (solid, or IBM-forced
+//   stores of the even step: both elements at once for a pair of active
+//     cells, the one active element of a half-solid (or half-forced) pair;
+//   stores of the odd step: a link whose downstream cell is solid writes the
+//     cell's own slot, and an inactive cell of the pair (solid, or IBM-forced
 //     and updated by hydro_cells_kernel) writes its own word of the scratch
 //     plane Q, which nothing reads.
-// Cells on a periodic face, under the free-slip top or next to a moving
-// wall take the generic path.
+// Cells next to a moving wall and, on the odd step, on a periodic face or
+// under the free-slip top take the generic path.
+// Measured on B200 (runner step of the 128 x 128 x 160 tank, D3Q27 fp32):
+// 122.5 us with the order-1 and order-2 moments scaled inside every line of
+// the backward transform, a select per population for cells at rest and
+// per-element stores on even-step wall tiles, 112.5 us in this form (128
+// registers instead of 168 suffice); a branch per direction around the wall
+// accesses of the odd step: 138 us.
 constexpr int PAIR_TILE = 64;
 constexpr uint32_t TILE_BND = 0x80000000u;  // tile-list bit: a fluid cell of the tile has a solid neighbour
 
@@ -553,7 +594,8 @@ __device__ __forceinline__ void pair_finish(const HydroParams<float>& p, const P
   const uint32_t fl0 = fl2 & 0xffu, fl1 = fl2 >> 8;
   const bool act0 = !(fl0 & (F_SOLID | F_FORCED)), act1 = !(fl1 & (F_SOLID | F_FORCED));
   if (!(act0 || act1)) return;
-  if ((fl0 | fl1) & (F_WRAP | F_SLIP | F_MOVING)) {
+  // the even step touches own slots only: no wrap or reflection to handle
+  if ((fl0 | fl1) & (ODD ? (F_WRAP | F_SLIP | F_MOVING) : F_MOVING)) {
     const int nx = A.nx, nxy = A.nxy;
     const int z = int(c / uint32_t(nxy));
     const int r = int(c - uint32_t(z) * uint32_t(nxy));
@@ -582,15 +624,25 @@ __device__ __forceinline__ void pair_finish(const HydroParams<float>& p, const P
     }
     return;
   }
+  if constexpr (!ODD) {
+    // the access rules above
+    const bool both = act0 && act1;
+    if (both) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) IO::st2(cb + A.P(opp(q)), f[q]);
+    } else {
+      S* const c1 = cb + (act0 ? 0 : 1);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) IO::st1(c1 + A.P(opp(q)), act0 ? f[q].x : f[q].y);
+    }
+    return;
+  }
   const int32_t scratch = A.P(Q);
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const int o = opp(q);
-    int32_t d0 = A.P(o), d1 = A.P(o);
-    if (ODD) {
-      d0 = ((mk0 >> q) & 1u) ? A.P(o) : A.T(q);
-      d1 = ((mk1 >> q) & 1u) ? A.P(o) : A.T(q);
-    }
+    const int32_t d0 = ((mk0 >> q) & 1u) ? A.P(o) : A.T(q);
+    const int32_t d1 = ((mk1 >> q) & 1u) ? A.P(o) : A.T(q);
     IO::st1(cb + (act0 ? d0 : scratch), f[q].x);
     IO::st1(cb + (act1 ? d1 : scratch) + 1, f[q].y);
   }
