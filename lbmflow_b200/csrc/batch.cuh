@@ -85,7 +85,6 @@ static __global__ void __launch_bounds__(BATCH_IBM_THREADS, 4) batch_ibm_kernel(
   IbmRun<S> r = {};
   r.fb = static_cast<const S*>(b.hp.f);
   r.pl = int64_t(b.hp.plane);
-  r.nbr = b.hp.nbr;
   r.nx = b.nx;
   r.ny = b.ny;
   r.nz = b.nz;

@@ -110,7 +110,7 @@ struct BodyState {
   int radius = 0;  // radius the device stencils were built for (0: none)
   DevBuf<double> d_pos, d_weight, st_w, st_cks, wsum, cs_w, imp, mob, rmf, part_spread, part_diag;
   DevBuf<int32_t> st_off, st_slot, bslot, cs_off, cs_marker;
-  DevBuf<int2> brec;
+  DevBuf<int4> brec;
   int64_t ns = 0;
   bool empty_stencil = false;
 };
@@ -256,6 +256,7 @@ struct Engine final : EngineBase {
   int red_blocks = 0;
   // host mirrors
   std::vector<uint8_t> solid_h, flags_h;
+  std::vector<uint32_t> nbr_h;  // solid-neighbour masks
   std::vector<double> init_rho_h, init_u_h;
   bool init_is_rest = true;  // they hold rho = 1, u = 0 everywhere
   // device copy of init_u_h (the velocity the scalar equilibrium uses on
@@ -423,6 +424,7 @@ struct Engine final : EngineBase {
     nbr.upload(nb, st);
     wall_u.upload(w, st);
     CK(cudaStreamSynchronize(st));
+    nbr_h = std::move(nb);
     build_tiles();
   }
 
@@ -1890,8 +1892,11 @@ struct Engine final : EngineBase {
     B.st_w.upload(st_w, st);
     B.st_cks.upload(st_cks, st);
     B.wsum.upload(wsum, st);
-    std::vector<int2> brec(bslot.size());
-    for (size_t i = 0; i < bslot.size(); ++i) brec[i] = make_int2(bslot[i], int(slot_cell_h[size_t(bslot[i])]));
+    std::vector<int4> brec(bslot.size());
+    for (size_t i = 0; i < bslot.size(); ++i) {
+      const int64_t c = slot_cell_h[size_t(bslot[i])];
+      brec[i] = make_int4(bslot[i], int(c), int(nbr_h[size_t(c)]), 0);
+    }
     B.bslot.upload(bslot, st);
     B.brec.upload(brec, st);
     B.cs_off.upload(cs_off, st);
@@ -1971,7 +1976,6 @@ struct Engine final : EngineBase {
     IbmRun<S> r = {};
     r.fb = fp;
     r.pl = plane;
-    r.nbr = nbr.p;
     r.nx = nx;
     r.ny = ny;
     r.nz = nz;

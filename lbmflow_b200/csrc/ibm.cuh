@@ -40,8 +40,6 @@ namespace lbmb {
 constexpr int IBM_CLUSTER = 8;
 // Entries per partial sum of the global diagnostics.
 constexpr int IBM_CHUNK = 32;
-// Threads of the first block that reduce the partials.
-constexpr int IBM_REDUCE = 256;
 
 // All threads of the cluster; writes before it are visible after it.
 __device__ __forceinline__ void cluster_sync() {
@@ -69,7 +67,7 @@ struct IbmArgs {
   // slots touched by this body
   int64_t ns;
   const int32_t* bslot;    // body slot -> global slot
-  const int2* brec;        // body slot -> {global slot, cell}
+  const int4* brec;        // body slot -> {global slot, cell, solid-neighbour mask, 0}
   const int32_t* cs_off;   // ns + 1, contributions in marker order
   const int32_t* cs_marker;
   const double* cs_w;
@@ -159,7 +157,6 @@ struct IbmRun {
   using A = typename Codec<S>::A;
   const S* fb;
   int64_t pl;
-  const uint32_t* nbr;
   int nx, ny, nz, parity;
   Vec4<A>* fcur;       // force field by global slot
   int64_t nslots;
@@ -186,14 +183,12 @@ template <int Q, class S>
 __device__ __forceinline__ void ibm_prep_slot(const IbmArgs& a, const IbmRun<S>& r, int64_t i) {
   using A = typename Codec<S>::A;
   using L = Lat<Q>;
-  const int2 rec = a.brec[i];
+  const int4 rec = a.brec[i];
   const int32_t g = rec.x;
   const int64_t cell = rec.y;
-  const uint32_t mask = r.nbr[cell];  // zero away from solids
-  const int64_t nxy = int64_t(r.nx) * r.ny;
-  const int z = int(cell / nxy);
-  const int y = int((cell - int64_t(z) * nxy) / r.nx);
-  const int x = int(cell - int64_t(z) * nxy - int64_t(y) * r.nx);
+  const uint32_t mask = uint32_t(rec.z);  // zero away from solids
+  const int nxy = r.nx * r.ny;
+  const int z = rec.y / nxy, yx = rec.y - z * nxy, y = yx / r.nx, x = yx - y * r.nx;
   A f[Q];
   load_post_stream<Q, S>(r.fb, r.pl, cell, x, y, z, r.nx, r.ny, r.nz, mask, r.parity, f);
   A dr = A(0);
@@ -227,12 +222,28 @@ __device__ __forceinline__ void ibm_prep_slot(const IbmArgs& a, const IbmRun<S>&
   a.urec[g] = make_double4(u3[0], u3[1], u3[2], inv_rho);
 }
 
+// Row of a marker's stencil points, or of a slot's contributions: its range
+// and the first NB indices. These never change between calls, and a thread
+// loads its first row of each kind at the start of the kernel, so that every
+// phase begins with its gather instead of two dependent index loads.
+template <int NB>
+struct IbmIndex {
+  int32_t k0, k1, at[NB];
+  __device__ __forceinline__ void load(const int32_t* off, const int32_t* index, int64_t row) {
+    k0 = off[row];
+    k1 = off[row + 1];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) at[j] = k1 > k0 ? index[k0 + j < k1 ? k0 + j : k1 - 1] : 0;
+  }
+};
+
 // Interpolated velocity of a marker from its stencil points [k0, k1) in
 // order, NB gathers in flight (points past the end repeat the last one with
 // weight 0), and, with MOB, its mobility (solver.rs:3131-3140).
 template <int NB, bool MOB>
-__device__ __forceinline__ void ibm_marker_velocity(const IbmArgs& a, int32_t k0, int32_t k1, double (&um)[3],
+__device__ __forceinline__ void ibm_marker_velocity(const IbmArgs& a, const IbmIndex<NB>& ix, double (&um)[3],
                                                     double& mobility) {
+  const int32_t k0 = ix.k0, k1 = ix.k1;
   um[0] = um[1] = um[2] = 0.0;
   mobility = 0.0;
   for (int32_t k = k0; k < k1; k += NB) {
@@ -242,7 +253,7 @@ __device__ __forceinline__ void ibm_marker_velocity(const IbmArgs& a, int32_t k0
     for (int j = 0; j < NB; ++j) {
       const bool in = k + j < k1;
       const int32_t kk = in ? k + j : k1 - 1;
-      v[j] = a.urec[a.st_slot[kk]];
+      v[j] = a.urec[k == k0 ? ix.at[j] : a.st_slot[kk]];
       w[j] = in ? a.st_w[kk] : 0.0;
       if (MOB) n[j] = a.st_cks[kk];
     }
@@ -273,10 +284,9 @@ __device__ __forceinline__ void ibm_impulse(const IbmArgs& a, const IbmRun<S>& r
 // Spread the impulses into slot i, in marker order (solver.rs:3174-3209);
 // ff: the slot's share of the fluid force.
 template <int NB, class S>
-__device__ __forceinline__ void ibm_spread_slot(const IbmArgs& a, const IbmRun<S>& r, int64_t i, int sweep,
-                                                double (&ff)[3]) {
-  const int32_t g = a.brec[i].x;
-  const int32_t k0 = a.cs_off[i], k1 = a.cs_off[i + 1];
+__device__ __forceinline__ void ibm_spread_slot(const IbmArgs& a, const IbmRun<S>& r, int sweep,
+                                                const IbmIndex<NB>& ix, int32_t g, double (&ff)[3]) {
+  const int32_t k0 = ix.k0, k1 = ix.k1;
   double sp[3] = {0.0, 0.0, 0.0}, d[3] = {0.0, 0.0, 0.0};
   const double inv_rho = a.urec[g].w;
   if (sweep > 0)
@@ -293,7 +303,7 @@ __device__ __forceinline__ void ibm_spread_slot(const IbmArgs& a, const IbmRun<S
     for (int j = 0; j < NB; ++j) {
       const bool in = k + j < k1;
       const int32_t kk = in ? k + j : k1 - 1;
-      const double* im = a.imp + 3 * int64_t(a.cs_marker[kk]);
+      const double* im = a.imp + 3 * int64_t(k == k0 ? ix.at[j] : a.cs_marker[kk]);
       w[j] = in ? a.cs_w[kk] : 0.0;
       v[j][0] = im[0];
       v[j][1] = im[1];
@@ -332,11 +342,20 @@ __device__ __forceinline__ double warp_max(double v) {
 template <int Q, class S, int NB>
 __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, int rank, int ncta) {
   using A = typename Codec<S>::A;
-  __shared__ double sh[11 * (IBM_REDUCE / 32)];
   __shared__ double tot[11];
   const int lane = int(threadIdx.x) & 31, warp = int(threadIdx.x) >> 5;
   const int64_t nthr = int64_t(ncta) * blockDim.x;
   const int64_t tid = (int64_t(warp) * ncta + rank) * 32 + lane;  // few entries spread over the blocks
+  IbmIndex<NB> mine, slots;  // of this thread's first marker and first slot
+  if (tid < a.nm) mine.load(a.st_off, a.st_slot, tid);
+  if (tid < a.ns) slots.load(a.cs_off, a.cs_marker, tid);
+  const int32_t my_slot = tid < a.ns ? a.brec[tid].x : 0;
+  auto marker_row = [&](int64_t m) {
+    if (m == tid) return mine;
+    IbmIndex<NB> x;
+    x.load(a.st_off, a.st_slot, m);
+    return x;
+  };
   const int64_t nc_m = (a.nm + IBM_CHUNK - 1) / IBM_CHUNK, nc_s = (a.ns + IBM_CHUNK - 1) / IBM_CHUNK;
   for (int64_t i = tid; i < a.ns; i += nthr) ibm_prep_slot<Q, S>(a, r, i);
   if (r.clear)
@@ -345,7 +364,7 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
   for (int64_t m = tid; m < a.nm; m += nthr) {
     double t[3], x[3], um[3], mob;
     ibm_target(a, m, t, x);
-    ibm_marker_velocity<NB, true>(a, a.st_off[m], a.st_off[m + 1], um, mob);
+    ibm_marker_velocity<NB, true>(a, marker_row(m), um, mob);
     const double inv = mob != 0.0 ? a.relax / mob : 0.0;
     a.mob[m] = inv;
     if (r.sv_mob) r.sv_mob[m] = mob;
@@ -362,7 +381,14 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
     double* const px = pd + 8 * nc_m;
     for (int64_t i0 = tid - lane; i0 < a.ns; i0 += nthr) {
       double ff[3] = {0.0, 0.0, 0.0};
-      if (i0 + lane < a.ns) ibm_spread_slot<NB>(a, r, i0 + lane, s, ff);
+      const int64_t i = i0 + lane;
+      if (i == tid && i < a.ns) {
+        ibm_spread_slot<NB>(a, r, s, slots, my_slot, ff);
+      } else if (i < a.ns) {
+        IbmIndex<NB> ix;
+        ix.load(a.cs_off, a.cs_marker, i);
+        ibm_spread_slot<NB>(a, r, s, ix, a.brec[i].x, ff);
+      }
       for (int c = 0; c < 3; ++c) {
         const double v = warp_sum(ff[c]);
         if (lane == 0) ps[3 * (i0 / IBM_CHUNK) + c] = v;
@@ -379,9 +405,9 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
         const double* f = a.rmf + 3 * m;
         const double f0 = f[0], f1 = f[1], f2 = f[2], wt = a.weight[m], inv = a.mob[m];
         ibm_target(a, m, t, x);
-        const int32_t k0 = a.st_off[m], k1 = a.st_off[m + 1];
-        ibm_marker_velocity<NB, false>(a, k0, k1, um, none);
-        if (k1 > k0) {
+        const IbmIndex<NB> ix = marker_row(m);
+        ibm_marker_velocity<NB, false>(a, ix, um, none);
+        if (ix.k1 > ix.k0) {
           const double sl[3] = {t[0] - um[0], t[1] - um[1], t[2] - um[2]};
           const double s2 = sl[0] * sl[0] + sl[1] * sl[1] + sl[2] * sl[2];
           const double mag = sqrt(s2);
@@ -411,43 +437,42 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
     for (int64_t c = lane; c < nc_m; c += 32) amax = fmax(amax, px[c]);
     amax = __shfl_sync(0xffffffffu, warp_max(amax), 0);
     if (rank == 0) {
-      // the first block sums the partials: IBM_REDUCE threads, chunks
-      // t, t + IBM_REDUCE, ... in order, then a fixed tree
-      double acc[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // 8 slip sums, 3 spread sums
-      if (threadIdx.x < IBM_REDUCE) {
-        for (int64_t c = threadIdx.x; c < nc_m; c += IBM_REDUCE)
-          for (int k = 0; k < 8; ++k) acc[k] += pd[8 * c + k];
-        for (int64_t c = threadIdx.x; c < nc_s; c += IBM_REDUCE)
-          for (int k = 0; k < 3; ++k) acc[8 + k] += ps[3 * c + k];
-        for (int k = 0; k < 11; ++k) {
-          const double y = warp_sum(acc[k]);
-          if (lane == 0) sh[k * (IBM_REDUCE / 32) + warp] = y;
-        }
+      // the first block sums the partials, one warp per sum: lane t takes
+      // chunks t, t + 32, ... in order, then a tree (8 slip sums, then the 3
+      // spread sums)
+      for (int k = warp; k < 11; k += int(blockDim.x) >> 5) {
+        double y = 0.0;
+        if (k < 8)
+          for (int64_t c = lane; c < nc_m; c += 32) y += pd[8 * c + k];
+        else
+          for (int64_t c = lane; c < nc_s; c += 32) y += ps[3 * c + k - 8];
+        y = warp_sum(y);
+        if (lane == 0) tot[k] = y;
       }
       __syncthreads();
-      if (threadIdx.x < 11) {
-        double y = 0.0;
-        for (int w = 0; w < IBM_REDUCE / 32; ++w) y += sh[int(threadIdx.x) * (IBM_REDUCE / 32) + w];
-        run += y;
-        if (threadIdx.x < 2) tot[threadIdx.x] = y;
-      }
-      __syncthreads();  // sh is written again by the next sweep
+      if (threadIdx.x < 11) run += tot[threadIdx.x];
       slip_max = amax;
       ssq = tot[0];
       wsum = tot[1];
+      __syncthreads();  // tot is written again by the next sweep
     }
     done = s + 1;
     if (!r.sv_imp && amax / a.scale <= a.tol) break;  // the adjoint records a fixed number of sweeps
   }
-  // force field += spread in the storage arithmetic (solver.rs:3256-3279);
-  // each slot's spread was written by this thread
-  for (int64_t i = tid; i < a.ns; i += nthr) {
-    const int32_t g = a.brec[i].x;
-    Vec4<A> v = r.fcur[g];
-    v.x = v.x + A(a.spread[3 * g + 0]);
-    v.y = v.y + A(a.spread[3 * g + 1]);
-    v.z = v.z + A(a.spread[3 * g + 2]);
-    r.fcur[g] = v;
+  // force field += spread in the storage arithmetic (solver.rs:3256-3279),
+  // by the blocks that have no diagnostics to write
+  if (rank > 0 || ncta == 1) {
+    const int first = ncta > 1 ? 1 : 0;
+    const int64_t t0 = (int64_t(warp) * (ncta - first) + rank - first) * 32 + lane;
+    const int64_t step = int64_t(ncta - first) * blockDim.x;
+    for (int64_t i = t0; i < a.ns; i += step) {
+      const int32_t g = a.brec[i].x;
+      Vec4<A> v = r.fcur[g];
+      v.x = v.x + A(a.spread[3 * g + 0]);
+      v.y = v.y + A(a.spread[3 * g + 1]);
+      v.z = v.z + A(a.spread[3 * g + 2]);
+      r.fcur[g] = v;
+    }
   }
   if (rank == 0 && warp == 0) {
     // lane k holds sum k (see above); the torque on the body is minus the
