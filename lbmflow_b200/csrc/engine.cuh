@@ -86,7 +86,7 @@ struct DevBuf {
 // them took longer than the kernels (stress summary of a 128 x 128 x 160
 // grid: 2.3 of 3.2 ms). Every use is on the main stream.
 struct Scratch {
-  DevBuf<char> slot[4];
+  DevBuf<char> slot[8];
   template <class T>
   T* get(int k, size_t count) {
     const size_t b = std::max<size_t>(count, 1) * sizeof(T);
@@ -2464,34 +2464,35 @@ struct Engine final : EngineBase {
                      int64_t* active) override {
     auto& sc = scalar(k);
     OxygenSourceArgs a = a0;
-    DevBuf<double> dc, cs, ar, vo, de, part;
-    DevBuf<int> err;
-    DevBuf<unsigned long long> cnt;
-    if (a0.cstar) cs.upload(a0.cstar, size_t(n), st);
-    if (a0.area) ar.upload(a0.area, size_t(n), st);
-    if (a0.vol) vo.upload(a0.vol, size_t(n), st);
-    if (a0.density) de.upload(a0.density, size_t(n), st);
-    a.cstar = a0.cstar ? cs.p : nullptr;
-    a.area = a0.area ? ar.p : nullptr;
-    a.vol = a0.vol ? vo.p : nullptr;
-    a.density = a0.density ? de.p : nullptr;
-    dc.alloc(size_t(n));
+    auto up = [&](int slot, const double* h) -> const double* {
+      if (!h) return nullptr;
+      double* d = scratch.get<double>(slot, size_t(n));
+      CK(cudaMemcpyAsync(d, h, size_t(n) * sizeof(double), cudaMemcpyHostToDevice, st));
+      return d;
+    };
+    a.cstar = up(1, a0.cstar);
+    a.area = up(2, a0.area);
+    a.vol = up(3, a0.vol);
+    a.density = up(4, a0.density);
+    double* const dc = scratch.get<double>(0, size_t(n));
     const unsigned g = unsigned(ceil_div(n, 128));
-    gather_scalar(sc, dc.p, 0, n);
+    gather_scalar(sc, dc, 0, n);
     const int64_t nb = ceil_div(n, OXY_BLOCK);
-    part.alloc(size_t(2 * nb));
-    err.alloc(1);
-    cnt.alloc(2);
-    CK(cudaMemsetAsync(err.p, 0, sizeof(int), st));
-    CK(cudaMemsetAsync(cnt.p, 0, 2 * sizeof(unsigned long long), st));
-    oxygen_source_kernel<<<unsigned(nb), OXY_BLOCK, 0, st>>>(dc.p, a, err.p, part.p, cnt.p, n);
+    double* const part = scratch.get<double>(5, size_t(2 * nb));
+    struct Flags {
+      unsigned long long cnt[2];
+      int err;
+    };
+    Flags* const fl = scratch.get<Flags>(6, 1);
+    CK(cudaMemsetAsync(fl, 0, sizeof(Flags), st));
+    oxygen_source_kernel<<<unsigned(nb), OXY_BLOCK, 0, st>>>(dc, a, &fl->err, part, fl->cnt, n);
     CK(cudaGetLastError());
     int e = 0;
     unsigned long long hc[2] = {0, 0};
     std::vector<double> hp(static_cast<size_t>(2 * nb));
-    CK(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hc, cnt.p, sizeof(hc), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hp.data(), part.p, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&e, &fl->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hc, fl->cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hp.data(), part, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (e & 1) invalid("cell volume must be finite and positive");
     if (e & 2) invalid("oxygen transfer source inputs must be finite (C_L, C*, area density >= 0)");
@@ -2511,11 +2512,12 @@ struct Engine final : EngineBase {
     }
     // set_scalar_concentration: equilibrium of the new C at the current u
     ScalarParams<A> p = scalar_params(sc);
-    if (sc.q == 7) scalar_set_kernel<7, Q, S><<<g, 128, 0, st>>>(p, dc.p, init_u_dev(), n);
-    else scalar_set_kernel<Q, Q, S><<<g, 128, 0, st>>>(p, dc.p, init_u_dev(), n);
+    if (sc.q == 7) scalar_set_kernel<7, Q, S><<<g, 128, 0, st>>>(p, dc, init_u_dev(), n);
+    else scalar_set_kernel<Q, Q, S><<<g, 128, 0, st>>>(p, dc, init_u_dev(), n);
     CK(cudaGetLastError());
     sc.parity = 0;
     CK(cudaStreamSynchronize(st));
+    scratch.trim();
   }
 
   // Device CV of a scalar into *out (two deterministic passes).
