@@ -364,9 +364,10 @@ int lbmb_scalar_cv(lbmb_solver* h, int32_t k, double* cv);
  * run there (status "diverged"): the call returns LBMB_ERR_DIVERGED, the
  * outputs hold the executed steps (NaN, iterations 0, after them) and
  * lbmb_run_impeller_status reports the executed step count. Between checks
- * the loop replays a CUDA graph of 16 steps, captured on the first call and
- * kept by the handle (with its series buffers) while the body, the IBM
- * configuration, the sweep kernel and the scalar set are unchanged; the
+ * the loop replays CUDA graphs of 16, 8, 4 and 2 steps, captured when a call
+ * first uses them and kept by the handle (with its series buffers) while the
+ * body, the IBM configuration, the sweep kernel and the scalar set are
+ * unchanged; the
  * device time of lbmb_last_timing covers the steps only. */
 int lbmb_run_impeller(lbmb_solver* h, int32_t body, const lbmb_ibm_config* cfg, int64_t steps,
                       int32_t scalar, int64_t probe_every, double* torque_lu, double* fluid_force,
@@ -452,6 +453,10 @@ int lbmb_reduce_populations_noalloc(const void* f, int32_t storage, int32_t q, i
  *                      shared memory by 16-byte cp.async windows several
  *                      tiles ahead (TRT/BGK or central moment, fp32/fp16/
  *                      bf16 storage, no uniform body force).
+ * A solver starts on LBMB_SWEEP_LEAN where it applies, else LBMB_SWEEP_ASYNC
+ * (4/8-byte storage) or LBMB_SWEEP_WINDOW, and on LBMB_SWEEP_PAIR in place of
+ * lean and window for grids that it can run of at least 2^20 cells (16-bit
+ * storage) or 2^21 cells (fp32).
  * A kind that cannot run the solver's configuration returns
  * LBMB_ERR_UNSUPPORTED and leaves the current kind in place. */
 typedef enum {
@@ -465,15 +470,18 @@ typedef enum {
 } lbmb_sweep_kind;
 int lbmb_set_sweep_kernel(lbmb_solver* h, int32_t kind);
 int lbmb_get_sweep_kernel(lbmb_solver* h, int32_t* kind);
-/* Launch variant of the current sweep kernel (no reference counterpart).
+/* Launch variant of the current sweep kernel (no reference counterpart); of a
+ * solver that started on the pair kernel and whose kind was never set or
+ * tuned, of the kind it would have started on below that size (the solver
+ * moves to that kind).
  * Lean kernel: register budget per parity, as resident 128-thread blocks per
  * SM the kernel is compiled for: 10 (48 registers), 9 (56), 8 (64), 7 (72)
  * or 6 (80); more
  * registers avoid spills, fewer keep more warps resident. cp.async kernel
  * (fp32 storage): the same per parity with 4 (128 registers, 3-tile ring,
  * the default), 5 (96, 3 tiles) or 6 (80, 2 tiles); its persistent grid
- * fills every resident slot, less 32 block slots in the sweep of a runner
- * step, where the IBM kernels run concurrently on a side stream. Window
+ * fills every resident slot, less those of 8 SMs in the sweep of a runner
+ * step, where the direct forcing runs beside it. Window
  * kernel: resident 256-thread blocks per SM per parity, 2 (128 registers),
  * 3 (80) or 4 (64), with a tile ring of 3 where shared memory allows, else
  * 2; default 2 for the central moment, 3 for TRT/BGK. Pair kernel (TRT/BGK,
@@ -482,8 +490,8 @@ int lbmb_get_sweep_kernel(lbmb_solver* h, int32_t* kind);
  * budgets with the populations of the next tile staged in shared memory by
  * cp.async while the warp computes the current one (two stages of Q x 32
  * 8-byte slots per warp; the grid holds as many blocks as shared memory
- * allows, at most the budget's). The persistent pair grid leaves 32 block
- * slots free in a runner step as the cp.async kernel does. */
+ * allows, at most the budget's). The persistent pair grid leaves 8 SMs free
+ * in a runner step as the cp.async kernel does. */
 int lbmb_set_sweep_variant(lbmb_solver* h, int32_t even_blocks_per_sm, int32_t odd_blocks_per_sm);
 
 /* Sweep autotuner (no reference counterpart): times every sweep kernel kind
@@ -510,8 +518,8 @@ int lbmb_autotune_sweep(lbmb_solver* h, int32_t steps_per_trial, lbmb_autotune_r
  * ncases solvers of one lattice and storage type (TRT/BGK, fp32/fp16/bf16,
  * no uniform force, no scalar distributions, one device, same step parity)
  * are advanced in lockstep: per step one launch per kernel family covers
- * every case (IBM prep / interp / spread / diag / commit, forced cells, the
- * full-grid sweep, the cached-field refresh), captured in CUDA graphs. Each
+ * every case (direct forcing, forced cells, the full-grid sweep, the
+ * cached-field refresh), captured in CUDA graphs. Each
  * case runs the runner step of its own body (bodies[k], NULL = body 0, set
  * with lbmb_ibm_set_body) with cfg; per-case results equal running the case
  * alone with the lean sweep kernel. The solvers must outlive the batch and

@@ -303,7 +303,7 @@ struct Engine final : EngineBase {
     CK(cudaEventCreate(&ev1));
     solid_h.assign(size_t(n), 0);
     if (solid)
-      for (int64_t i = 0; i < n; ++i) solid_h[i] = solid[i] ? 1 : 0;
+      for (int64_t i = 0; i < n; ++i) n_solid += solid_h[i] = solid[i] ? 1 : 0;
     if (wu) wall_u_in.assign(wu, wu + 3 * n);
     build_flags(wu);
     // Guard margin: shifted TMA windows of the odd step reach up to
@@ -327,21 +327,22 @@ struct Engine final : EngineBase {
     // default sweep: the lean kernel where it applies (TRT/BGK, fp32/16-bit
     // storage, no uniform force), else cp.async (4/8-byte storage), the
     // window kernel (16-bit storage) or direct loads (uniform force); on a
-    // large grid with even nx the pair kernel instead of these. Runner step
-    // on B200, smaller grids first, default before / pair, us: D3Q27 fp32 48 x
-    // 48 x 60 24.8 / 25.9, 72 x 72 x 90 29.1 / 29.2, 96 x 96 x 120 62.1 /
-    // 61.7, 128 x 128 x 160 137 / 122; D3Q27 fp16 48 24.9 / 25.8, 96 67 / 51;
-    // D3Q19 fp16 96 35.1 / 34.5, 128 71 / 57; D3Q19 fp32 112 61 / 64, 128 87 /
-    // 79, 160 160 / 137.
+    // large grid with even nx the pair kernel in place of lean and window.
+    // Runner step on B200, default before / pair, us: D3Q27 fp16 48 x 48 x 60
+    // 24.9 / 25.8, 96 x 96 x 120 67 / 45; D3Q19 fp16 96 35.1 / 34.5, 128 71 /
+    // 57, 256 506 / 398; D3Q19 fp32 112 61 / 64, 128 87 / 79, 160 160 / 134.
+    // The fp32 central moment keeps cp.async, although the pair kernel takes
+    // 112 us there against 137 (128): it is closer to the 64-bit result
+    // (1.7e-3 -> 4e-5 of the near-wall velocities of a tank just started), but
+    // a default must not move results by that much.
     if (sizeof(S) < 4) kernel_mode = window_ok() ? LBMB_SWEEP_WINDOW : LBMB_SWEEP_DIRECT;
     if (lean_ok(coll)) kernel_mode = LBMB_SWEEP_LEAN;
-    const bool wide_trt = sizeof(S) == 4 && coll == COLL_TRT;
-    if (std::is_same<A, float>::value && nx % 2 == 0 && !has_uniform_force() && (coll == COLL_TRT || Q == 27) &&
-        n >= (int64_t(1) << (wide_trt ? 21 : 20)) && int64_t(Q + 1) * plane < (int64_t(1) << 31)) {
+    if (std::is_same<A, float>::value && nx % 2 == 0 && !has_uniform_force() &&
+        (sizeof(S) == 4 ? coll == COLL_TRT : coll == COLL_TRT || Q == 27) &&
+        n >= (int64_t(1) << (sizeof(S) == 4 ? 21 : 20)) && int64_t(Q + 1) * plane < (int64_t(1) << 31)) {
       chosen_over = kernel_mode;
       kernel_mode = LBMB_SWEEP_PAIR;
-      // budgets the autotuner picks there (fp32 D3Q27 runner step: 4/4 112,
-      // staged 3 / 3 119 us; fp16 D3Q19: staged 3 / 4)
+      // budgets the autotuner picks there
       pair_minb[0] = coll == COLL_CM ? 4 : PAIR_STAGED + 3;
       pair_minb[1] = 4;
       prepare_pair_variant();
@@ -2807,17 +2808,17 @@ struct Engine final : EngineBase {
     fprev_stale = false;
   }
 
+  // Sweeps launched while one of these is alive follow the direct forcing.
+  struct BesideIbm {
+    bool& flag;
+    explicit BesideIbm(Engine& e) : flag(e.after_ibm) { flag = true; }
+    ~BesideIbm() { flag = false; }
+  };
   // The full-grid sweep of a runner step, launched on the main stream right
   // behind the direct forcing.
   void sweep_beside_ibm() {
-    after_ibm = true;
-    try {
-      launch_hydro(parity, st, true, false);
-    } catch (...) {
-      after_ibm = false;
-      throw;
-    }
-    after_ibm = false;
+    BesideIbm beside(*this);
+    launch_hydro(parity, st, true, false);
   }
 
   void snapshot(S* out) {
@@ -3182,11 +3183,8 @@ struct Engine final : EngineBase {
     }
   }
 
-  int64_t solid_count() const {
-    int64_t s = 0;
-    for (auto v : solid_h) s += v ? 1 : 0;
-    return s;
-  }
+  int64_t n_solid = 0;  // the solid mask does not change
+  int64_t solid_count() const { return n_solid; }
 
   void fill_nan(double* p, int64_t k) {
     std::vector<double> h(size_t(k), std::nan(""));
@@ -3319,9 +3317,10 @@ struct Batch final : BatchBase {
     else batch_cells_kernel<Q, S, false><<<unsigned(nb_slots), BATCH_BLOCK, 0, st2>>>(cases.p, off_slots.p, ncase);
     batch_fprev_kernel<<<unsigned(nb_slots), BATCH_BLOCK, 0, st2>>>(cases.p, off_slots.p, ncase);
     CK(cudaGetLastError());
-    eng[0]->after_ibm = true;
-    hydro(parity);
-    eng[0]->after_ibm = false;
+    {
+      typename E::BesideIbm beside(*eng[0]);
+      hydro(parity);
+    }
     CK(cudaEventRecord(ev_join, st2));
     CK(cudaStreamWaitEvent(st, ev_join, 0));
     parity ^= 1;

@@ -65,7 +65,8 @@ def test_percentiles_are_the_sorted_ranks(n, scale):
 
 
 @pytest.mark.parametrize("dims,q,coll,storage,kind", [
-    ((128, 128, 64), 27, "cm", "f32", "pair"), ((128, 128, 64), 19, "trt", "f16", "pair"),
+    ((128, 128, 64), 27, "cm", "f16", "pair"), ((128, 128, 64), 19, "trt", "f16", "pair"),
+    ((128, 128, 128), 27, "cm", "f32", "async"),
     ((128, 128, 128), 19, "trt", "f32", "pair"), ((128, 128, 64), 19, "trt", "f32", "lean"),
     ((127, 128, 129), 19, "trt", "f32", "lean"), ((126, 128, 64), 27, "cm", "f32", "async"),
     ((128, 128, 64), 27, "cm", "f64", "async")])
@@ -92,6 +93,9 @@ def test_default_sweep_and_its_variants(dims, q, coll, storage, kind):
     if coll == "trt":
         h.set_sweep_variant(8, 7)
         assert h.sweep_kernel == "lean"
+    elif storage == "f16":
+        h.set_sweep_variant(3, 3)
+        assert h.sweep_kernel == "window"
     else:
         h.set_sweep_variant(4, 4)
         assert h.sweep_kernel == "async"
