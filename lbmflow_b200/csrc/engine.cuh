@@ -691,7 +691,7 @@ struct Engine final : EngineBase {
   void launch_lean_mb(const HydroParams<A>& p, cudaStream_t s) {
     if constexpr (std::is_same<A, float>::value) {
       launch_sweep(hydro_lean_kernel<Q, S, ODD, MINB>, dim3(unsigned(ceil_div(n, LEAN_BLOCK))), LEAN_BLOCK, 0, s, p,
-                   uint32_t(n));
+                   uint32_t(n), chained ? 1 : 0);
     }
   }
 
@@ -957,6 +957,11 @@ struct Engine final : EngineBase {
       CK(cudaEventRecord(ev_join, st2));
       CK(cudaStreamWaitEvent(st, ev_join, 0));
     } else {
+      chained = true;
+      struct Off {
+        bool& f;
+        ~Off() { f = false; }
+      } off{chained};
       launch_hydro(parity);
     }
     parity ^= 1;
@@ -2031,6 +2036,7 @@ struct Engine final : EngineBase {
   // launched before it on the same stream when after_ibm is set: it starts
   // once the cluster's blocks run (it shares no data with them).
   bool after_ibm = false;
+  bool chained = false;  // a plain step behind another one (lean kernel)
   template <class... KArgs, class... Args>
   void launch_sweep(void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t lc = {};
@@ -2042,7 +2048,7 @@ struct Engine final : EngineBase {
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at;
-    lc.numAttrs = after_ibm ? 1 : 0;
+    lc.numAttrs = after_ibm || (chained && kernel_mode == LBMB_SWEEP_LEAN) ? 1 : 0;
     CK(cudaLaunchKernelEx(&lc, kernel, static_cast<KArgs>(args)...));
   }
 
