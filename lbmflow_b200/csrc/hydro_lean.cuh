@@ -175,7 +175,8 @@ __device__ __forceinline__ void lean_cell(const HydroParams<float>& p, uint32_t 
 // chained: launched as the programmatic dependent of the step before, whose
 // completion it waits for here, with its blocks already scheduled. On a small
 // grid the launch gap is much of a step: 24^3 cavity 3.2 -> 2.9 us per step on
-// B200 (64 steps with their calls 216 -> 175 us), 64^3 8.0 -> 7.5 us.
+// B200 (a 64-step pass with its moments' readback 272 -> 233 us), 64^3 8.0 ->
+// 7.5 us.
 template <int Q, class S, bool ODD, int MINB>
 __global__ void __launch_bounds__(LEAN_BLOCK, MINB) hydro_lean_kernel(HydroParams<float> p, uint32_t n, int chained) {
   if (chained) {
