@@ -454,9 +454,8 @@ int lbmb_reduce_populations_noalloc(const void* f, int32_t storage, int32_t q, i
  *                      tiles ahead (TRT/BGK or central moment, fp32/fp16/
  *                      bf16 storage, no uniform body force).
  * A solver starts on LBMB_SWEEP_LEAN where it applies, else LBMB_SWEEP_ASYNC
- * (4/8-byte storage) or LBMB_SWEEP_WINDOW, and on LBMB_SWEEP_PAIR in place of
- * lean and window for grids that it can run of at least 2^20 cells (16-bit
- * storage) or 2^21 cells (fp32).
+ * (4/8-byte storage) or LBMB_SWEEP_WINDOW (16-bit storage); with a uniform
+ * body force 16-bit storage starts on LBMB_SWEEP_DIRECT.
  * A kind that cannot run the solver's configuration returns
  * LBMB_ERR_UNSUPPORTED and leaves the current kind in place. */
 typedef enum {
@@ -470,10 +469,7 @@ typedef enum {
 } lbmb_sweep_kind;
 int lbmb_set_sweep_kernel(lbmb_solver* h, int32_t kind);
 int lbmb_get_sweep_kernel(lbmb_solver* h, int32_t* kind);
-/* Launch variant of the current sweep kernel (no reference counterpart); of a
- * solver that started on the pair kernel and whose kind was never set or
- * tuned, of the kind it would have started on below that size (the solver
- * moves to that kind).
+/* Launch variant of the current sweep kernel (no reference counterpart).
  * Lean kernel: register budget per parity, as resident 128-thread blocks per
  * SM the kernel is compiled for: 10 (48 registers), 9 (56), 8 (64), 7 (72)
  * or 6 (80); more

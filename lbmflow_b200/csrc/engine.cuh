@@ -326,27 +326,16 @@ struct Engine final : EngineBase {
     rows_aligned = (nx % TmaWin<S>::PAD == 0) && ((int64_t(nx) * ny) % TmaWin<S>::PAD == 0);
     // default sweep: the lean kernel where it applies (TRT/BGK, fp32/16-bit
     // storage, no uniform force), else cp.async (4/8-byte storage), the
-    // window kernel (16-bit storage) or direct loads (uniform force); on a
-    // large grid with even nx the pair kernel in place of lean and window.
-    // Runner step on B200, default before / pair, us: D3Q27 fp16 48 x 48 x 60
-    // 24.9 / 25.8, 96 x 96 x 120 67 / 45; D3Q19 fp16 96 35.1 / 34.5, 128 71 /
-    // 57, 256 506 / 398; D3Q19 fp32 112 61 / 64, 128 87 / 79, 160 160 / 134.
-    // The fp32 central moment keeps cp.async, although the pair kernel takes
-    // 112 us there against 137 (128): it is closer to the 64-bit result
-    // (1.7e-3 -> 4e-5 of the near-wall velocities of a tank just started), but
-    // a default must not move results by that much.
+    // window kernel (16-bit storage) or direct loads (uniform force). The pair
+    // kernel, which is the faster one on large grids (runner step on B200,
+    // default / pair: D3Q19 fp16 256 506 / 398 us, fp32 128 87 / 79 us, D3Q27
+    // fp16 96 67 / 45 us, fp32 128 137 / 112 us), rounds in another order, so
+    // it runs where the caller or the autotuner chooses it: the size of a
+    // grid alone must not move results, which 16-bit storage amplifies most
+    // (fp16 tank of 72 cells after 60 steps, lean against pair: forces 5e-3
+    // apart; fp32 3e-5).
     if (sizeof(S) < 4) kernel_mode = window_ok() ? LBMB_SWEEP_WINDOW : LBMB_SWEEP_DIRECT;
     if (lean_ok(coll)) kernel_mode = LBMB_SWEEP_LEAN;
-    if (std::is_same<A, float>::value && nx % 2 == 0 && !has_uniform_force() &&
-        (sizeof(S) == 4 ? coll == COLL_TRT : coll == COLL_TRT || Q == 27) &&
-        n >= (int64_t(1) << (sizeof(S) == 4 ? 21 : 20)) && int64_t(Q + 1) * plane < (int64_t(1) << 31)) {
-      chosen_over = kernel_mode;
-      kernel_mode = LBMB_SWEEP_PAIR;
-      // budgets the autotuner picks there
-      pair_minb[0] = coll == COLL_CM ? 4 : PAIR_STAGED + 3;
-      pair_minb[1] = 4;
-      prepare_pair_variant();
-    }
     red_blocks = int(std::min<int64_t>(ceil_div(n, RED_BLOCK), 1184));
     red_part.alloc(size_t(red_blocks) * 5);
     red_out.alloc(8);
@@ -608,7 +597,6 @@ struct Engine final : EngineBase {
     if (kind == LBMB_SWEEP_LEAN && !lean_ok(coll))
       throw Error(LBMB_ERR_UNSUPPORTED, "the lean sweep needs TRT/BGK, fp32/fp16/bf16 storage and no uniform body force");
     kernel_mode = kind;
-    chosen_over = -1;
     invalidate_graphs();
   }
   int sweep_kernel() const override { return kernel_mode; }
@@ -616,25 +604,8 @@ struct Engine final : EngineBase {
   // blocks per SM (4 = 128 registers with a 3-tile ring, 5 = 96 with 3,
   // 6 = 80 with 2); the persistent grid fills every resident slot.
   int async_minb[2] = {4, 4};
-  // The kind in whose place a large grid starts on the pair kernel (-1: the
-  // kind was set, or there is no such choice). A variant set on a solver whose
-  // kind was never set names that kind's budgets, as on any other grid.
-  int chosen_over = -1;
 
   void set_sweep_variant(int even, int odd) override {
-    if (chosen_over >= 0) {
-      const int pair_kind = kernel_mode, base = chosen_over;
-      chosen_over = -1;
-      kernel_mode = base;
-      try {
-        set_sweep_variant(even, odd);
-      } catch (...) {
-        kernel_mode = pair_kind;
-        chosen_over = base;
-        throw;
-      }
-      return;
-    }
     if (kernel_mode == LBMB_SWEEP_ASYNC) {
       auto ok = [](int v) { return v >= 4 && v <= 6; };
       if (!ok(even) || !ok(odd))
@@ -1200,7 +1171,6 @@ struct Engine final : EngineBase {
       }
     }
     kernel_mode = cands[best].kind;
-    chosen_over = -1;
     if (kernel_mode == LBMB_SWEEP_LEAN) {
       lean_minb[0] = cands[best].ev;
       lean_minb[1] = cands[best].od;
@@ -1486,10 +1456,7 @@ struct Engine final : EngineBase {
     // captured launch as it is
     const bool same = omega_on && omega_kind_ok(kernel_mode);
     omega_on = true;
-    if (!omega_kind_ok(kernel_mode)) {
-      kernel_mode = window_ok() ? LBMB_SWEEP_WINDOW : LBMB_SWEEP_DIRECT;
-      chosen_over = -1;
-    }
+    if (!omega_kind_ok(kernel_mode)) kernel_mode = window_ok() ? LBMB_SWEEP_WINDOW : LBMB_SWEEP_DIRECT;
     if (!same) invalidate_graphs();
   }
 
