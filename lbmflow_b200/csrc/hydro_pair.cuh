@@ -439,8 +439,8 @@ __device__ __forceinline__ float2 ld2_odd(const S* p) {
 //     cell's own slot, and an inactive cell of the pair (solid, or IBM-forced
 //     and updated by hydro_cells_kernel) writes its own word of the scratch
 //     plane Q, which nothing reads.
-// Cells next to a moving wall and, on the odd step, on a periodic face or
-// under the free-slip top take the generic path.
+// Cells on a periodic face, under the free-slip top or next to a moving
+// wall take the generic path.
 // Measured on B200 (runner step of the 128 x 128 x 160 tank, D3Q27 fp32):
 // 122.5 us with the order-1 and order-2 moments scaled inside every line of
 // the backward transform, a select per population for cells at rest and
@@ -594,8 +594,10 @@ __device__ __forceinline__ void pair_finish(const HydroParams<float>& p, const P
   const uint32_t fl0 = fl2 & 0xffu, fl1 = fl2 >> 8;
   const bool act0 = !(fl0 & (F_SOLID | F_FORCED)), act1 = !(fl1 & (F_SOLID | F_FORCED));
   if (!(act0 || act1)) return;
-  // the even step touches own slots only: no wrap or reflection to handle
-  if ((fl0 | fl1) & (ODD ? (F_WRAP | F_SLIP | F_MOVING) : F_MOVING)) {
+  // on the even step too, where wrap and slip cells would need no special
+  // access: the generic collision rounds in another order than the packed
+  // one, and 16-bit storage amplifies that
+  if ((fl0 | fl1) & (F_WRAP | F_SLIP | F_MOVING)) {
     const int nx = A.nx, nxy = A.nxy;
     const int z = int(c / uint32_t(nxy));
     const int r = int(c - uint32_t(z) * uint32_t(nxy));

@@ -99,6 +99,39 @@ def test_pair_kernel_low_precision_matches_direct(prec, kind, q, coll):
     assert l2 < {"f16": 5e-3, "bf16": 5e-2}[prec], l2
 
 
+@pytest.mark.parametrize("variant", [(4, 4), (13, 13)])
+@pytest.mark.parametrize("q,coll", [(19, "trt"), (27, "trt"), (27, "cm")])
+@pytest.mark.parametrize("prec", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("form", ["slip", "wrap"])
+def test_pair_kernel_wrap_and_slip_cells_round_like_direct(form, prec, q, coll, variant):
+    # every pair holds a cell under the free-slip top, or on a periodic face:
+    # the pair kernel takes its generic path for all of them, with the direct
+    # kernel's arithmetic, on both parities
+    from cases import seeded_state
+    dims = (16, 12, 3) if form == "slip" else (4, 40, 3)
+    solid = np.zeros(dims[::-1], np.uint8)
+    solid[0] = solid[-1] = 1  # one fluid layer: a wall above and below every cell
+    solid[:, 0] = solid[:, -1] = 1
+    if form == "slip":
+        solid[:, :, 0] = solid[:, :, -1] = 1
+    solid[1, 5, 2] = 1  # a half-solid pair
+    solid = solid.ravel()
+    kw = dict(lattice=q, collision=coll, storage=prec, nu=0.03, solid=solid, smagorinsky_cs=0.1)
+    kw.update({"free_slip_top": True} if form == "slip" else {"periodic": (True, False, False)})
+    a, b = lb.Solver(dims, **kw), lb.Solver(dims, **kw)
+    a.set_sweep_kernel("direct")
+    b.set_sweep_kernel("pair")
+    b.set_sweep_variant(*variant)
+    f = seeded_state(q, a.n, 11)
+    f[:, solid != 0] = 0.0
+    for g in (a, b):
+        g.stage_in(f)
+    for _ in range(4):
+        a.run(1)
+        b.run(1)
+        assert np.array_equal(a.stage_out()[:, solid == 0], b.stage_out()[:, solid == 0])
+
+
 @pytest.mark.parametrize("kind", ["pair", "tile", "lean", "direct", "bulk", "async", "window"])
 def test_runner_loop_each_kernel_matches_oracle(kind):
     from oracle import oracle as o
