@@ -216,8 +216,8 @@ __device__ __forceinline__ void cm_bwd2(float2& k0, float2& k1, float2& k2, floa
 }
 
 // The same with the moments of order 1 and 2 already halved (the transform is
-// linear, so the halves are taken once at its input): hu = u/2, hu2 = u^2/2,
-// u2 = 2u.
+// linear, so the halves, which are exact, are taken once at its input, and
+// the rounding is that of cm_bwd2): hu = u/2, hu2 = u^2/2, u2 = 2u.
 __device__ __forceinline__ void cm_bwd2h(float2& k0, float2& k1, float2& k2, float2 hu, float2 hu2, float2 u2) {
   const float2 m1 = fma2(hu, k0, k1);
   const float2 m2 = fma2(hu2, k0, fma2(u2, k1, k2));
@@ -287,9 +287,11 @@ __device__ __forceinline__ float2 cm_pair_reg(float2 (&f)[Q], const HydroParams<
     const float2 q2 = fma2(pxx, pxx, fma2(pyy, pyy, mul2(pzz, pzz)));
     const float2 o2 = fma2(pxy, pxy, fma2(pxz, pxz, mul2(pyz, pyz)));
     const float2 n2 = fma2(bc2(2.f), o2, q2);
+    // the contraction is spelled out: left to the compiler it differs between
+    // register budgets
     const float t0 = p.tau0;
-    const float te0 = 0.5f * (t0 + sqrt_fast(t0 * t0 + p.les_c * sqrt_fast(n2.x) * inv.x));
-    const float te1 = 0.5f * (t0 + sqrt_fast(t0 * t0 + p.les_c * sqrt_fast(n2.y) * inv.y));
+    const float te0 = 0.5f * (t0 + sqrt_fast(__fmaf_rn(t0, t0, __fmul_rn(__fmul_rn(p.les_c, sqrt_fast(n2.x)), inv.x))));
+    const float te1 = 0.5f * (t0 + sqrt_fast(__fmaf_rn(t0, t0, __fmul_rn(__fmul_rn(p.les_c, sqrt_fast(n2.y)), inv.y))));
     os = make_float2(rcp_fast(te0), rcp_fast(te1));
   }
   const float2 osc = fma2(os, mul2(usq, bc2(-0.16f)), os);
@@ -337,7 +339,7 @@ __device__ __forceinline__ float2 cm_pair_reg(float2 (&f)[Q], const HydroParams<
     {
       const float2 k0 = G[a][0][1], k1 = G[a][1][1];
       const float2 m1 = fma2(huy, k0, k1);
-      const float2 m2 = fma2(huy2, k0, mul2(uyd, k1));
+      const float2 m2 = mul2(huy, fma2(uy, k0, mul2(bc2(4.f), k1)));  // k1 is a half
       G[a][0][1] = sub2(m2, m1);
       G[a][1][1] = fma2(bc2(-2.f), m2, k0);
       G[a][2][1] = add2(m2, m1);
@@ -355,27 +357,22 @@ __device__ __forceinline__ float2 cm_pair_reg(float2 (&f)[Q], const HydroParams<
   for (int a = 0; a < 3; ++a)
 #pragma unroll
     for (int b = 0; b < 3; ++b) cm_bwd2h(G[a][b][0], G[a][b][1], G[a][b][2], huz, huz2, uzd);
-  // f' = feq + G, opposite directions together: w (drho + rho (4.5 cu^2 -
-  // 1.5 u^2)) +- 3 w rho cu
+  // f' = feq + G: w (drho + rho (3 cu + 4.5 cu^2 - 1.5 u^2)), opposite
+  // directions from the same cu (4.5 cu - 3 times cu for the second: the
+  // same roundings with the sign moved)
   const float2 nusq = mul2(bc2(-1.5f), usq);
   f[0] = fma2(bc2(float(L::w(0))), fma2(rho, nusq, drho), G[1][1][1]);
-  float2 wr = bc2(0.f), wd = bc2(0.f), w3 = bc2(0.f), n3 = bc2(0.f);
 #pragma unroll
   for (int k = 0; k < NP; ++k) {
     const int a = 2 * k + 1, b = a + 1;
-    if (k == 0 || wclass<Q>(a) != wclass<Q>(a - 2)) {
-      const float w = float(L::w(a));
-      wr = mul2(bc2(w), rho);
-      wd = mul2(bc2(w), drho);
-      w3 = mul2(bc2(3.f), wr);
-      n3 = mul2(bc2(-3.f), wr);
-    }
+    const float2 w = bc2(float(L::w(a)));
     float2 cu = L::cx(a) ? ux : (L::cy(a) ? uy : uz);
     if (L::cx(a) && L::cy(a)) cu = L::cy(a) > 0 ? add2(cu, uy) : sub2(cu, uy);
     if ((L::cx(a) || L::cy(a)) && L::cz(a)) cu = L::cz(a) > 0 ? add2(cu, uz) : sub2(cu, uz);
-    const float2 P = fma2(wr, fma2(bc2(4.5f), mul2(cu, cu), nusq), wd);
-    f[a] = fma2(w3, cu, add2(P, G[L::cx(a) + 1][L::cy(a) + 1][L::cz(a) + 1]));
-    f[b] = fma2(n3, cu, add2(P, G[L::cx(b) + 1][L::cy(b) + 1][L::cz(b) + 1]));
+    const float2 ia = fma2(cu, fma2(bc2(4.5f), cu, bc2(3.f)), nusq);
+    const float2 ib = fma2(cu, fma2(bc2(4.5f), cu, bc2(-3.f)), nusq);
+    f[a] = fma2(w, fma2(rho, ia, drho), G[L::cx(a) + 1][L::cy(a) + 1][L::cz(a) + 1]);
+    f[b] = fma2(w, fma2(rho, ib, drho), G[L::cx(b) + 1][L::cy(b) + 1][L::cz(b) + 1]);
   }
   // a lane at exact rest keeps its populations, which are w (rho - 1)
   if (rest0 || rest1) {
