@@ -367,8 +367,9 @@ int lbmb_scalar_cv(lbmb_solver* h, int32_t k, double* cv);
  * the loop replays CUDA graphs of 16, 8, 4 and 2 steps, captured when a call
  * first uses them and kept by the handle (with its series buffers) while the
  * body, the IBM configuration, the sweep kernel and the scalar set are
- * unchanged; the
- * device time of lbmb_last_timing covers the steps only. */
+ * unchanged; the device time of lbmb_last_timing covers the steps only. The
+ * sweep runs beside the direct forcing of its step, except with a uniform
+ * body force, which forces every cell: then it follows it. */
 int lbmb_run_impeller(lbmb_solver* h, int32_t body, const lbmb_ibm_config* cfg, int64_t steps,
                       int32_t scalar, int64_t probe_every, double* torque_lu, double* fluid_force,
                       double* cv, int32_t* ibm_iterations);

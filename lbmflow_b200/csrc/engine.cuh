@@ -2610,26 +2610,35 @@ struct Engine final : EngineBase {
     if (k >= 0) fill_nan(run_cv.p, steps);
     int64_t launches = 0;
     auto one_step = [&](int64_t step_index) {
-      // The direct forcing (with the clear) starts first; the full-grid
-      // sweep follows on the main stream once its blocks are resident, and
-      // the forced cells wait for it on the high-priority side stream. The
-      // two touch disjoint population slots (each cell's AA read/write set
-      // is its own).
+      // The direct forcing (with the clear) starts first; without a uniform
+      // force the full-grid sweep, which leaves out the forced cells, follows
+      // on the main stream once its blocks are resident, and the forced cells
+      // wait for it on the high-priority side stream. The two touch disjoint
+      // population slots (each cell's AA read/write set is its own).
       // Solver::clear_body_force_field: the IBM field is non-uniform, so the
       // cached moments keep it (F_prev) while the new field starts at zero.
       enqueue_ibm(B, c, run_torque.p, run_ff.p, run_it.p, run_counter.p, false, true);
-      CK(cudaEventRecord(ev_fork, st));
-      CK(cudaStreamWaitEvent(st2, ev_fork, 0));
       field_present = true;
       fprev_stale = true;
-      launch_hydro(parity, st2, false, true);
-      sweep_beside_ibm();
-      // cached-moment field refresh on the side stream behind the forced
-      // cells, hidden by the full-grid sweep
-      if (nslots) CK(cudaMemcpyAsync(fprev.p, fcur.p, size_t(nslots) * sizeof(Vec4<A>), cudaMemcpyDeviceToDevice, st2));
+      if (has_uniform_force()) {
+        // The sweep forces every cell: it reads the field and rewrites the
+        // populations that the forcing works on, so the three follow each
+        // other.
+        launch_hydro(parity);
+        if (nslots) CK(cudaMemcpyAsync(fprev.p, fcur.p, size_t(nslots) * sizeof(Vec4<A>), cudaMemcpyDeviceToDevice, st));
+      } else {
+        CK(cudaEventRecord(ev_fork, st));
+        CK(cudaStreamWaitEvent(st2, ev_fork, 0));
+        launch_hydro(parity, st2, false, true);
+        sweep_beside_ibm();
+        // cached-moment field refresh on the side stream behind the forced
+        // cells, hidden by the full-grid sweep
+        if (nslots)
+          CK(cudaMemcpyAsync(fprev.p, fcur.p, size_t(nslots) * sizeof(Vec4<A>), cudaMemcpyDeviceToDevice, st2));
+        CK(cudaEventRecord(ev_join, st2));
+        CK(cudaStreamWaitEvent(st, ev_join, 0));
+      }
       fprev_stale = false;
-      CK(cudaEventRecord(ev_join, st2));
-      CK(cudaStreamWaitEvent(st, ev_join, 0));
       parity ^= 1;
       for (auto& sc : scalars) scalar_step(*sc);
       ++launches;

@@ -131,6 +131,35 @@ def test_runner_matches_host_driven_loop():
     assert np.array_equal(a.stage_out(), b.stage_out())
 
 
+@pytest.mark.parametrize("q,coll,prec", [(19, "trt", "f64"), (27, "cm", "f64"), (19, "trt", "f32"), (27, "cm", "f32"),
+                                         (19, "trt", "f16")])
+def test_runner_loop_with_a_uniform_force(q, coll, prec):
+    # the sweep then forces every cell and needs the spread field of its step:
+    # the loop equals the calls one by one, and the oracle
+    from oracle import oracle as o
+    dims, solid, body = small_tank(n=24)
+    kw = dict(collision=coll, nu=0.02, omega_shear=1.0 / (3.0 * 0.02 + 0.5), solid=solid, force=(2e-6, -1e-6, 3e-6))
+    a, b = lb.Solver(dims, lattice=q, storage=prec, **kw), lb.Solver(dims, lattice=q, storage=prec, **kw)
+    r = a.run_impeller(body, 37)
+    tq = []
+    for _ in range(37):
+        b.clear_body_force_field()
+        tq.append(-b.apply_rotating_ibm(body).torque[2])
+        b.run(1)
+    assert np.array_equal(r["torque_lu"], np.array(tq))
+    assert np.array_equal(a.stage_out(), b.stage_out())
+    assert np.array_equal(a.force_field(), b.force_field())
+    if prec == "f16":
+        return
+    c = o.OracleSolver(dims, q=q, real_bits=64 if prec == "f64" else 32, **kw)
+    rc = c.run_tank(body.positions, body.weights, body.center, body.omega, 37)
+    tol = 1e-9 if prec == "f64" else 2e-4
+    assert np.abs(r["torque_lu"] - rc["torque_lu"]).max() <= tol * np.abs(rc["torque_lu"]).max()
+    fl = solid == 0
+    ug, uc = np.stack(a.read_moments()[1:])[:, fl], np.stack(c.moments()[1:])[:, fl]
+    assert np.abs(ug - uc).max() <= (1e-9 if prec == "f64" else 1e-5) * np.abs(uc).max()
+
+
 def _slab_cylinder(omega_z):
     # 3D analogue of the reference 2D rotating-cylinder KATs
     # (crates/lbm-core/tests/rotating_ibm.rs:71-140): a circle of 96 markers
