@@ -108,7 +108,7 @@ struct BodyState {
   double center[3] = {0, 0, 0}, omega[3] = {0, 0, 0};
   double scale = 1.0;
   int radius = 0;  // radius the device stencils were built for (0: none)
-  DevBuf<double> d_pos, d_weight, st_w, st_cks, wsum, cs_w, imp, mob, rmf, part_spread, part_diag;
+  DevBuf<double> d_pos, d_weight, st_w, st_cks, wsum, cs_w, imp, mob, inv_mob, rmf, part_spread, part_diag;
   DevBuf<int32_t> st_off, st_slot, bslot, cs_off, cs_marker;
   DevBuf<int4> brec;
   int64_t ns = 0;
@@ -1775,6 +1775,7 @@ struct Engine final : EngineBase {
     bs->d_weight.upload(bs->weight, st);
     bs->imp.alloc(size_t(3 * nm));
     bs->mob.alloc(size_t(nm));
+    bs->inv_mob.alloc(size_t(nm));
     bs->rmf.alloc(size_t(3 * nm));
     bs->part_diag.alloc(size_t(2 * 9 * ceil_div(nm, IBM_CHUNK)));
     CK(cudaStreamSynchronize(st));
@@ -1904,6 +1905,7 @@ struct Engine final : EngineBase {
     a.spread = s_spread.p;
     a.imp = B.imp.p;
     a.mob = B.mob.p;
+    a.inv_mob = B.inv_mob.p;
     a.rmf = B.rmf.p;
     a.part_spread = B.part_spread.p;
     a.part_diag = B.part_diag.p;

@@ -30,6 +30,7 @@
 #pragma once
 #include "common.cuh"
 #include "lattice.cuh"
+#include "quotient.hpp"
 
 namespace lbmb {
 
@@ -79,7 +80,8 @@ struct IbmArgs {
   double* spread;    // x3
   // per marker state
   double* imp;       // x3
-  double* mob;       // relaxation / mobility (0: none)
+  double* mob;
+  double* inv_mob;   // reciprocal(mob)
   double* rmf;       // x3 represented marker force of this sweep
   // partials
   double* part_spread;  // 2 x ceil(ns / IBM_CHUNK) x 3 (two sweeps in flight)
@@ -247,34 +249,43 @@ __device__ __forceinline__ void ibm_marker_velocity(const IbmArgs& a, const IbmI
   um[0] = um[1] = um[2] = 0.0;
   mobility = 0.0;
   for (int32_t k = k0; k < k1; k += NB) {
-    double w[NB], n[NB];
+    double w[NB], n[NB], rho[NB];
     double4 v[NB];
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
       const bool in = k + j < k1;
       const int32_t kk = in ? k + j : k1 - 1;
-      v[j] = a.urec[k == k0 ? ix.at[j] : a.st_slot[kk]];
+      const int32_t s = k == k0 ? ix.at[j] : a.st_slot[kk];
+      v[j] = a.urec[s];
       w[j] = in ? a.st_w[kk] : 0.0;
-      if (MOB) n[j] = a.st_cks[kk];
+      if (MOB) {
+        n[j] = a.st_cks[kk];
+        rho[j] = a.rho[s];
+      }
     }
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
       um[0] += w[j] * v[j].x;
       um[1] += w[j] * v[j].y;
       um[2] += w[j] * v[j].z;
-      if (MOB) mobility += w[j] * n[j] * v[j].w;
+      if (MOB) mobility += quotient(w[j] * n[j], fmax(rho[j], 1.0e-30), v[j].w);
     }
   }
 }
 
-// Impulse of a marker from the interpolated velocity (solver.rs:3118-3173);
-// inv_mob = relaxation / mobility (0: no impulse).
+// Impulse of a marker from the interpolated velocity (solver.rs:3118-3173),
+// none without mobility. The quotients here and in the mobility round as the
+// reference's divisions: plain products with the reciprocals differ in the
+// last place, and now and then a force in 32 bits with them, which a long
+// 16-bit run amplifies. Divisions proper call a subroutine, whose register
+// limits make the phases spill: 48 x 48 x 60 and 96 x 96 x 120 tank 22.8 and
+// 39.4 us per step, 21.5 and 37.2 us in this form.
 template <class S>
 __device__ __forceinline__ void ibm_impulse(const IbmArgs& a, const IbmRun<S>& r, int64_t m, const double (&t)[3],
-                                            const double (&um)[3], double inv_mob, int sweep) {
+                                            const double (&um)[3], double mob, double inv_mob, int sweep) {
   const double ws = a.wsum[m];
   for (int c = 0; c < 3; ++c) {
-    const double imp = (t[c] - um[c]) * inv_mob;
+    const double imp = mob != 0.0 ? quotient(a.relax * (t[c] - um[c]), mob, inv_mob) : 0.0;
     a.imp[3 * m + c] = imp;
     a.rmf[3 * m + c] = imp * ws;
     if (r.sv_imp) r.sv_imp[(int64_t(sweep) * a.nm + m) * 3 + c] = imp;
@@ -365,10 +376,11 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
     double t[3], x[3], um[3], mob;
     ibm_target(a, m, t, x);
     ibm_marker_velocity<NB, true>(a, marker_row(m), um, mob);
-    const double inv = mob != 0.0 ? a.relax / mob : 0.0;
-    a.mob[m] = inv;
+    const double inv = reciprocal(mob);
+    a.mob[m] = mob;
+    a.inv_mob[m] = inv;
     if (r.sv_mob) r.sv_mob[m] = mob;
-    ibm_impulse(a, r, m, t, um, inv, 0);
+    ibm_impulse(a, r, m, t, um, mob, inv, 0);
   }
   cluster_sync();
   // block 0: running sums of the call (thread k of the first warp holds sum k:
@@ -403,7 +415,8 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
       if (m < a.nm) {
         double t[3], x[3], um[3], none;
         const double* f = a.rmf + 3 * m;
-        const double f0 = f[0], f1 = f[1], f2 = f[2], wt = a.weight[m], inv = a.mob[m];
+        const double f0 = f[0], f1 = f[1], f2 = f[2], wt = a.weight[m];
+        const double mob = a.mob[m], inv = a.inv_mob[m];
         ibm_target(a, m, t, x);
         const IbmIndex<NB> ix = marker_row(m);
         ibm_marker_velocity<NB, false>(a, ix, um, none);
@@ -421,7 +434,7 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
         v[5] = x[1] * f2 - x[2] * f1;
         v[6] = x[2] * f0 - x[0] * f2;
         v[7] = x[0] * f1 - x[1] * f0;
-        if (s + 1 < r.sweeps) ibm_impulse(a, r, m, t, um, inv, s + 1);
+        if (s + 1 < r.sweeps) ibm_impulse(a, r, m, t, um, mob, inv, s + 1);
       }
       smax = warp_max(smax);
       if (lane == 0) px[m0 / IBM_CHUNK] = smax;

@@ -39,6 +39,36 @@ def test_marker_counts_match_oracle(nm, radius, tol):
         assert np.abs(fg - fc).max() <= 1e-12 * np.abs(fc).max()
 
 
+# CRC-32 of the force field after two calls from integer-made inputs, as a
+# chain of kernels with plain divisions gave it.
+FIELD_CRC = {(300, 1): 0xa94664c8, (300, 2): 0x0d310867, (5000, 1): 0xcbb8dd4d, (5000, 2): 0xfc32f19a}
+
+
+@pytest.mark.parametrize("nm,radius", list(FIELD_CRC))
+def test_force_field_keeps_its_rounding(nm, radius):
+    import zlib
+    solid = np.zeros((22, 20, 18), np.uint8)
+    solid[0] = solid[-1] = 1
+    solid[:, 0] = solid[:, -1] = 1
+    solid[:, :, 0] = solid[:, :, -1] = 1
+    solid = solid.ravel()
+
+    def lcg(k, m):  # m numbers in [0, 1)
+        i = np.arange(m, dtype=np.uint64) + np.uint64(k)
+        return ((i * np.uint64(2654435761) >> np.uint64(13)) % np.uint64(262144)).astype(np.float64) / 262144.0
+
+    g = lb.Solver((18, 20, 22), lattice=19, storage="f64", nu=0.03, solid=solid)
+    f = 2e-3 * (lcg(5, 19 * g.n).reshape(19, g.n) - 0.5)
+    f[:, solid != 0] = 0.0
+    g.stage_in(f)
+    pos = 0.7 + lcg(77, 3 * nm).reshape(nm, 3) * np.array([15.6, 17.6, 19.6])
+    body = lb.RotatingBody([8.5, 9.5, 10.5], [0.001, 0.0, 0.003], pos, 0.25 + 0.5 * lcg(9, nm))
+    for relax in (1.0, 0.9):
+        g.apply_rotating_ibm(body, lb.DirectForcingConfig(4, 0.0, radius, relax))
+    out = np.ascontiguousarray(g.force_field() + 0.0)
+    assert np.isfinite(out).all() and zlib.crc32(out.tobytes()) == FIELD_CRC[nm, radius], hex(zlib.crc32(out.tobytes()))
+
+
 @pytest.mark.parametrize("storage", ["f32", "f16"])
 def test_runner_loop_repeats_bitwise(storage):
     # the phases of one call are ordered by cluster barriers only: a missing

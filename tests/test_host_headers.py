@@ -1,0 +1,59 @@
+"""Host-side headers of the library, compiled and run as plain C++."""
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lbmflow_b200", "csrc")
+
+
+def run_cpp(tmp_path, body):
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text(body)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    return subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout
+
+
+@pytest.mark.parametrize("spread", [1, 40, 400])
+def test_quotient_is_the_division(tmp_path, spread):
+    # 4 million operand pairs with exponents within +-spread: every quotient
+    # is the correctly rounded one; so are the special operands' results
+    out = run_cpp(tmp_path, r"""
+#include <cstdint>
+#include <cstdio>
+#include <cstring>
+#include <initializer_list>
+#include <limits>
+#include "quotient.hpp"
+static uint64_t s = 88172645463325252ull;
+static uint64_t next() { s ^= s << 13; s ^= s >> 7; s ^= s << 17; return s; }
+static double draw(int spread) {
+  uint64_t m = next() & 0xfffffffffffffull;
+  if (next() % 8 == 0) m |= 0xffffffffff000ull;  // mantissas close to a power of two
+  if (next() % 8 == 0) m &= 0xfffull;
+  const uint64_t e = uint64_t(1023 + int(next() % uint64_t(2 * spread + 1)) - spread);
+  const uint64_t b = (next() & 0x8000000000000000ull) | (e << 52) | m;
+  double d;
+  std::memcpy(&d, &b, 8);
+  return d;
+}
+static bool same(double a, double b) { return (a != a && b != b) || a == b; }
+int main() {
+  long bad = 0;
+  for (int i = 0; i < 4000000; ++i) {
+    const double a = draw(SPREAD), b = draw(SPREAD);
+    bad += !same(lbmb::quotient(a, b, lbmb::reciprocal(b)), a / b);
+  }
+  const double inf = std::numeric_limits<double>::infinity(), nan = std::numeric_limits<double>::quiet_NaN();
+  const double v[] = {0.0, 1.0, -3.0, 1e300, -1e300, 1e-300, inf, -inf, nan};
+  for (double a : v)
+    for (double b : {1.0, 3.0, 1e-30, 1e300, inf, nan}) {
+      const double q = lbmb::quotient(a, b, lbmb::reciprocal(b)), t = a / b;
+      // (tiny quotients: last place only)
+      bad += !(same(q, t) || std::fabs(q - t) <= std::numeric_limits<double>::denorm_min());
+    }
+  bad += !same(lbmb::quotient(0.0, 1e-310, lbmb::reciprocal(1e-310)), 0.0);
+  std::printf("%ld\n", bad);
+}
+""".replace("SPREAD", str(spread)))
+    assert int(out) == 0
