@@ -22,6 +22,7 @@
 #include "../../include/lbmb.h"
 #include "checkpoint.hpp"
 #include "readback.hpp"
+#include "run_graphs.hpp"
 #include "aux.cuh"
 #include "hydro.cuh"
 #include "hydro_tma.cuh"
@@ -98,6 +99,40 @@ struct Scratch {
     for (DevBuf<char>& b : slot)
       if (b.n > (size_t(256) << 20)) b.release();
   }
+};
+
+// What `enqueue` puts on stream s, as an instantiated graph. An exception on
+// the way ends the capture, so that the stream works on.
+template <class Enqueue>
+cudaGraphExec_t capture_graph(cudaStream_t s, const Enqueue& enqueue) {
+  struct Graph {
+    cudaGraph_t g = nullptr;
+    ~Graph() {
+      if (g) cudaGraphDestroy(g);
+    }
+  } gr;
+  CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+  try {
+    enqueue();
+  } catch (...) {
+    cudaStreamEndCapture(s, &gr.g);
+    cudaGetLastError();  // the exception tells
+    throw;
+  }
+  CK(cudaStreamEndCapture(s, &gr.g));
+  cudaGraphExec_t exec = nullptr;
+  CK(cudaGraphInstantiate(&exec, gr.g, 0));
+  return exec;
+}
+// The step parity while steps are captured.
+struct KeepParity {
+  int& parity;
+  const int was;
+  explicit KeepParity(int& p) : parity(p), was(p) {}
+  ~KeepParity() { parity = was; }
+};
+struct FreeGraph {
+  void operator()(cudaGraphExec_t g) const { cudaGraphExecDestroy(g); }
 };
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
@@ -347,8 +382,7 @@ struct Engine final : EngineBase {
   ~Engine() override {
     if (step_graph) cudaGraphExecDestroy(step_graph);
     for (auto& e : fused_cache) cudaGraphExecDestroy(e.exec);
-    for (auto& g : run_graphs)
-      if (g) cudaGraphExecDestroy(g);
+    run_graphs.drop();
     if (st) cudaStreamSynchronize(st);
     bodies.clear();
     scalars.clear();
@@ -424,7 +458,7 @@ struct Engine final : EngineBase {
       step_graph = nullptr;
     }
     drop_fused_graphs();
-    drop_run_graphs();
+    run_graphs.drop();
   }
 
   // Grow the force-slot arrays, keeping content.
@@ -994,14 +1028,11 @@ struct Engine final : EngineBase {
         continue;
       }
       if (!step_graph) {
-        cudaGraph_t g;
-        CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < G; ++i) enqueue_step();
-        CK(cudaStreamEndCapture(st, &g));
-        CK(cudaGraphInstantiate(&step_graph, g, 0));
-        CK(cudaGraphDestroy(g));
+        const KeepParity keep(parity);
+        step_graph = capture_graph(st, [&] {
+          for (int i = 0; i < G; ++i) enqueue_step();
+        });
         step_graph_len = G;
-        parity = 0;  // G is even
       }
       CK(cudaGraphLaunch(step_graph, st));
       done += G;
@@ -2117,12 +2148,7 @@ struct Engine final : EngineBase {
           CK(cudaGraphExecDestroy(fused_cache.front().exec));
           fused_cache.erase(fused_cache.begin());
         }
-        cudaGraph_t g;
-        CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        enqueue_runner_step(B, cfg_ibm, true);
-        CK(cudaStreamEndCapture(st, &g));
-        CK(cudaGraphInstantiate(&exec, g, 0));
-        CK(cudaGraphDestroy(g));
+        exec = capture_graph(st, [&] { enqueue_runner_step(B, cfg_ibm, true); });
         fused_cache.push_back({k, exec});
       }
       CK(cudaEventRecord(ev0, st));
@@ -2530,9 +2556,9 @@ struct Engine final : EngineBase {
   DevBuf<int32_t> run_it;
   DevBuf<int64_t> run_counter;
   int64_t run_cap = 0;
-  // The instantiated runner graph (RUN_G steps from parity 0) and what it
-  // was captured with: the IBM launch arguments, the body, the probed scalar
-  // and the parity of every scalar at the graph's first step. Sweep kernel,
+  // The instantiated runner graphs (RUN_G steps and fewer, from parity 0) and
+  // what they were captured with: the IBM launch arguments, the body and the
+  // parity of every scalar at the graph's first step. Sweep kernel,
   // geometry, slots and scalar set changes destroy it (invalidate_graphs).
   static constexpr int64_t RUN_G = 16;
   struct RunKey {
@@ -2542,12 +2568,10 @@ struct Engine final : EngineBase {
     const void* sc_h[8];
     int32_t sc_par[8];
   };
-  RunKey run_key;
   // graphs of 16, 8, 4 and 2 steps (index 0..3) for the same key, so that a
   // span that is not a multiple of 16 replays graphs down to one step
   static constexpr int RUN_NG = 4;
-  cudaGraphExec_t run_graphs[RUN_NG] = {nullptr, nullptr, nullptr, nullptr};
-  bool run_graph = false;
+  GraphSet<RunKey, cudaGraphExec_t, FreeGraph, RUN_NG> run_graphs;
   // Outcome of the last run_impeller call (runner.rs:1077-1129): steps
   // executed and whether the run stopped on a non-finite total mass.
   int64_t run_executed = 0;
@@ -2555,15 +2579,6 @@ struct Engine final : EngineBase {
   // The runner checks the f64 total mass after every DIVERGE_EVERY-th step
   // of a run and stops at the first non-finite value (runner.rs:1125-1128).
   static constexpr int64_t DIVERGE_EVERY = 1000;
-
-  void drop_run_graphs() {
-    for (auto& g : run_graphs)
-      if (g) {
-        CK(cudaGraphExecDestroy(g));
-        g = nullptr;
-      }
-    run_graph = false;
-  }
 
   // The spans of a run of `steps` steps from step parity par: visit(gi) for a
   // graph of RUN_G >> gi steps, visit(-1) for a single step; no span crosses
@@ -2597,7 +2612,7 @@ struct Engine final : EngineBase {
     run_cv.alloc(size_t(cap));
     run_counter.alloc(1);
     run_cap = cap;
-    drop_run_graphs();
+    run_graphs.drop();
   }
 
   void run_impeller(int b, const lbmb_ibm_config& c, int64_t steps, int k, int64_t probe_every, double* torque,
@@ -2668,41 +2683,44 @@ struct Engine final : EngineBase {
         key.sc_h[i] = scalars[i]->h.p;
         key.sc_par[i] = scalars[i]->parity ^ parity;
       }
-      if (run_graph && std::memcmp(&key, &run_key, sizeof(key)) != 0) drop_run_graphs();
-      // the graph sizes that this call's spans use and that are not there yet
-      bool need[RUN_NG] = {false, false, false, false}, any = false;
+      // the graph sizes that this call's spans use
+      bool need[RUN_NG] = {false, false, false, false};
       for_spans(steps, parity, true, [&](int gi) {
-        if (gi >= 0 && !run_graphs[gi]) need[gi] = any = true;
+        if (gi >= 0) need[gi] = true;
       });
-      if (any) {
-        // capture from parity 0 with the scalar parities the graph will
-        // start from, then put the host state back
-        const int par0 = parity;
-        std::vector<int> spar(scalars.size());
-        for (size_t i = 0; i < scalars.size(); ++i) spar[i] = scalars[i]->parity;
-        const bool fpres = field_present, fstale = fprev_stale;
-        for (int gi = 0; gi < RUN_NG; ++gi) {
-          if (!need[gi]) continue;
-          for (size_t i = 0; i < scalars.size(); ++i) scalars[i]->parity = key.sc_par[i];
-          parity = 0;
-          cudaGraph_t g;
-          CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-          for (int64_t i = 0; i < (RUN_G >> gi); ++i) one_step(0);
-          CK(cudaStreamEndCapture(st, &g));
-          CK(cudaGraphInstantiate(&run_graphs[gi], g, 0));
-          CK(cudaGraphDestroy(g));
-          // upload now, so that the first replay inside a timed span does
-          // not carry it
-          CK(cudaGraphUpload(run_graphs[gi], st));
+      // captured from parity 0 with the scalar parities the graph will start
+      // from; the host state is put back, also when a capture fails
+      struct HostState {
+        Engine& e;
+        const int par = e.parity;
+        const bool present = e.field_present, stale = e.fprev_stale;
+        std::vector<int> spar;
+        explicit HostState(Engine& e_) : e(e_) {
+          for (auto& sc : e.scalars) spar.push_back(sc->parity);
         }
-        run_graph = true;
-        parity = par0;
-        for (size_t i = 0; i < scalars.size(); ++i) scalars[i]->parity = spar[i];
-        field_present = fpres;
-        fprev_stale = fstale;
-        launches = 0;
-        run_key = key;
-      }
+        ~HostState() {
+          e.parity = par;
+          for (size_t i = 0; i < spar.size(); ++i) e.scalars[i]->parity = spar[i];
+          e.field_present = present;
+          e.fprev_stale = stale;
+        }
+      } state(*this);
+      run_graphs.prepare(key, need, [&](int gi) {
+        for (size_t i = 0; i < scalars.size(); ++i) scalars[i]->parity = key.sc_par[i];
+        parity = 0;
+        const cudaGraphExec_t g = capture_graph(st, [&] {
+          for (int64_t i = 0; i < (RUN_G >> gi); ++i) one_step(0);
+        });
+        // upload now, so that the first replay inside a timed span does not
+        // carry it
+        const cudaError_t up = cudaGraphUpload(g, st);
+        if (up != cudaSuccess) {
+          cudaGraphExecDestroy(g);
+          CK(up);
+        }
+        return g;
+      });
+      launches = 0;
     }
     CK(cudaEventRecord(ev0, st));
     int64_t done = 0;
@@ -2853,16 +2871,6 @@ struct Engine final : EngineBase {
     }
     // Graph of one full segment (K steps; K even, so every segment starts
     // at the same parity and the graph replays unchanged).
-    auto capture = [&](auto&& body) {
-      cudaGraph_t gr;
-      cudaGraphExec_t ex = nullptr;
-      CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      body();
-      CK(cudaStreamEndCapture(st, &gr));
-      CK(cudaGraphInstantiate(&ex, gr, 0));
-      CK(cudaGraphDestroy(gr));
-      return ex;
-    };
     cudaGraphExec_t g_fwd = nullptr;
     CK(cudaEventRecord(ev0, st));
     for (int64_t seg = 0; seg < nseg; ++seg) {
@@ -2874,7 +2882,7 @@ struct Engine final : EngineBase {
       if (len == K && graphs) {
         if (!g_fwd) {
           const int par0 = parity;
-          g_fwd = capture([&] {
+          g_fwd = capture_graph(st, [&] {
             for (int64_t i = 0; i < K; ++i) enqueue_runner_step(B, c, d_torque.p, d_counter.p);
           });
           parity = par0;
@@ -3056,16 +3064,6 @@ struct Engine final : EngineBase {
         launch_cluster(adj_ibm_kernel<Q, A>, 1, ADJ_IBM_THREADS, sb, ab, nsweep, lam_out, plane);
       }
     };
-    auto capture_on = [&](cudaStream_t s0, auto&& body) {
-      cudaGraph_t gr;
-      cudaGraphExec_t ex = nullptr;
-      CK(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
-      body();
-      CK(cudaStreamEndCapture(s0, &gr));
-      CK(cudaGraphInstantiate(&ex, gr, 0));
-      CK(cudaGraphDestroy(gr));
-      return ex;
-    };
     cudaGraphExec_t g_rec[2] = {nullptr, nullptr}, g_bwd[2] = {nullptr, nullptr};
     std::vector<double> tbh(static_cast<size_t>(nseg * K), 0.0);
     for (int64_t t = ac.window_begin; t < N; ++t) tbh[size_t(t)] = Tbar;
@@ -3089,7 +3087,7 @@ struct Engine final : EngineBase {
       fprev_stale = false;
       if (len == K && graphs) {
         if (!g_rec[bi]) {
-          g_rec[bi] = capture_on(st, [&] { recompute(b, K); });
+          g_rec[bi] = capture_graph(st, [&] { recompute(b, K); });
           cleanup.gs.push_back(g_rec[bi]);
         }
         CK(cudaGraphLaunch(g_rec[bi], st));
@@ -3113,7 +3111,7 @@ struct Engine final : EngineBase {
       }
       if (len == K && graphs) {
         if (!g_bwd[bi]) {
-          g_bwd[bi] = capture_on(sb, [&] { backward(b, K); });
+          g_bwd[bi] = capture_graph(sb, [&] { backward(b, K); });
           cleanup.gs.push_back(g_bwd[bi]);
         }
         CK(cudaGraphLaunch(g_bwd[bi], sb));
@@ -3330,14 +3328,10 @@ struct Batch final : BatchBase {
     cudaGraphExec_t exec = nullptr;
     while (steps - done >= G) {
       if (!exec) {
-        cudaGraph_t g;
-        const int par0 = parity;
-        CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        for (int64_t i = 0; i < G; ++i) one_step();
-        CK(cudaStreamEndCapture(st, &g));
-        CK(cudaGraphInstantiate(&exec, g, 0));
-        CK(cudaGraphDestroy(g));
-        parity = par0;
+        const KeepParity keep(parity);
+        exec = capture_graph(st, [&] {
+          for (int64_t i = 0; i < G; ++i) one_step();
+        });
       }
       CK(cudaGraphLaunch(exec, st));
       done += G;

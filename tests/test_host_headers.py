@@ -57,3 +57,54 @@ int main() {
 }
 """.replace("SPREAD", str(spread)))
     assert int(out) == 0
+
+
+def test_graph_set_keeps_one_key_and_survives_a_failed_capture(tmp_path):
+    out = run_cpp(tmp_path, r"""
+#include <cstdio>
+#include <stdexcept>
+#include "run_graphs.hpp"
+struct Key { int body, cfg; };
+static int live = 0;
+struct Free { void operator()(int*) const { --live; } };
+static int pool[64], used = 0;
+static int fail_at = -1;
+static int* make(int i) {
+  if (i == fail_at) throw std::runtime_error("no memory");
+  ++live;
+  pool[used] = used;
+  return &pool[used++];
+}
+int main() {
+  {
+    lbmb::GraphSet<Key, int*, Free, 4> g;
+    const bool two[4] = {true, false, true, false}, all[4] = {true, true, true, true}, none[4] = {};
+    g.prepare(Key{1, 1}, two, make);
+    std::printf("%d %d\n", live, g[0] && !g[1] && g[2] && !g[3]);
+    int* const first = g[0];
+    g.prepare(Key{1, 1}, all, make);  // the missing ones are added
+    std::printf("%d %d\n", live, g[0] == first);
+    g.prepare(Key{2, 1}, two, make);  // another key: none of the first is left
+    std::printf("%d %d\n", live, g[0] != first && !g[1]);
+    fail_at = 2;  // a later length fails after an earlier one was made
+    bool thrown = false;
+    try {
+      g.prepare(Key{3, 1}, two, make);
+    } catch (const std::runtime_error&) {
+      thrown = true;
+    }
+    std::printf("%d %d\n", live, thrown && !g[0] && !g[2]);
+    fail_at = -1;
+    g.prepare(Key{2, 1}, two, make);  // a call with another key starts afresh
+    std::printf("%d %d\n", live, g[0] && g[2]);
+    g.prepare(Key{2, 1}, none, make);
+    std::printf("%d %d\n", live, g[0] && g[2]);
+    g.drop();
+    std::printf("%d %d\n", live, !g[0]);
+    g.prepare(Key{2, 1}, two, make);  // the same key after a drop
+    std::printf("%d %d\n", live, g[0] && g[2]);
+  }
+  std::printf("%d 1\n", live);
+}
+""")
+    assert out.split() == "2 1 4 1 2 1 0 1 2 1 2 1 0 1 2 1 0 1".split()
