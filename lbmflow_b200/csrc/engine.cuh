@@ -85,19 +85,28 @@ struct DevBuf {
 // Device work arrays of the QOI calls, kept between calls by slot (grown
 // when a call needs more) and freed with the solver: allocating and freeing
 // them took longer than the kernels (stress summary of a 128 x 128 x 160
-// grid: 2.3 of 3.2 ms). Every use is on the main stream.
+// grid: 2.3 of 3.2 ms). Every use is on the main stream. A solver keeps KEEP
+// bytes at most: above that (grids of about 6 million cells and more) all go
+// when the call that holds a Use ends, also by an exception.
 struct Scratch {
+  static constexpr size_t KEEP = size_t(256) << 20;
+  struct Use {
+    Scratch& s;
+    explicit Use(Scratch& s_) : s(s_) {}
+    Use(const Use&) = delete;
+    ~Use() {
+      size_t held = 0;
+      for (const DevBuf<char>& b : s.slot) held += b.n;
+      if (held > KEEP)
+        for (DevBuf<char>& b : s.slot) b.release();
+    }
+  };
   DevBuf<char> slot[8];
   template <class T>
   T* get(int k, size_t count) {
     const size_t b = std::max<size_t>(count, 1) * sizeof(T);
     if (slot[k].n < b) slot[k].alloc(b);
     return reinterpret_cast<T*>(slot[k].p);
-  }
-  // after a call: arrays of a very large grid are not kept
-  void trim() {
-    for (DevBuf<char>& b : slot)
-      if (b.n > (size_t(256) << 20)) b.release();
   }
 };
 
@@ -1508,6 +1517,7 @@ struct Engine final : EngineBase {
   }
 
   void velocity_gradient(double* g9) override {
+    const Scratch::Use use(scratch);
     double* const u3 = scratch.get<double>(0, size_t(3) * n);
     velocity_moments(u3);
     const StrainArgs<S> a = strain_args();
@@ -1533,6 +1543,7 @@ struct Engine final : EngineBase {
       if (A(tau_eff_max) < tau0) invalid("tau_eff_max must be at least the laminar tau for this solver");
       nu_t_max = (A(tau_eff_max) - tau0) / A(3.0);
     }
+    const Scratch::Use use(scratch);
     double* const u3 = scratch.get<double>(0, size_t(3) * n);
     unsigned long long* const cnt = scratch.get<unsigned long long>(2, 2);
     CK(cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), st));
@@ -1581,6 +1592,7 @@ struct Engine final : EngineBase {
 
   void stress_field(double dx, double dt, double mu, double* s6, double* gamma, double* viscous) override {
     check_si(dx, dt, mu);
+    const Scratch::Use use(scratch);
     double* const u3 = scratch.get<double>(0, size_t(3) * n);
     velocity_moments(u3);
     std::vector<ReadField> fields;
@@ -1606,6 +1618,7 @@ struct Engine final : EngineBase {
     check_si(dx, dt, mu);
     // the values of the ranks, selected on the device (stress.cuh): only the
     // bins that hold them are sorted
+    const Scratch::Use use(scratch);
     double* const u3 = scratch.get<double>(0, size_t(3) * n);
     double* const key = scratch.get<double>(1, size_t(n));
     struct Work {
@@ -1676,7 +1689,6 @@ struct Engine final : EngineBase {
     };
     fill(pg, 1.0, hg, above[0]);
     fill(pt, mu, ht, above[1]);
-    scratch.trim();
   }
 
   void wall_shear(double dx, double dt, double rho, double mu, lbmb_wall_shear* out, int64_t capacity,
@@ -2466,6 +2478,7 @@ struct Engine final : EngineBase {
                      int64_t* active) override {
     auto& sc = scalar(k);
     OxygenSourceArgs a = a0;
+    const Scratch::Use use(scratch);
     auto up = [&](int slot, const double* h) -> const double* {
       if (!h) return nullptr;
       double* d = scratch.get<double>(slot, size_t(n));
@@ -2519,7 +2532,6 @@ struct Engine final : EngineBase {
     CK(cudaGetLastError());
     sc.parity = 0;
     CK(cudaStreamSynchronize(st));
-    scratch.trim();
   }
 
   // Device CV of a scalar into *out (two deterministic passes).

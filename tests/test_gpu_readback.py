@@ -99,3 +99,22 @@ def test_renewed_relaxation_field_replays_like_single_steps():
                 g.run_impeller(body, k)
         out.append(g.stage_out())
     assert np.array_equal(out[0], out[1])
+
+
+def test_work_arrays_of_a_very_large_grid_are_given_back():
+    # 24 bytes a cell is 288 MB here, above what a solver keeps between calls
+    import torch
+    dims = (240, 240, 208)
+    g = lb.Solver(dims, lattice=19, storage="f16", nu=0.02, solid=box(dims))
+    g.set_omega_field(np.full(g.n, 1.8))
+    g.read_moments()
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    before = free()
+    for call in (g.wale_update, lambda: g.stress_field(0.01, 0.001, 0.7), g.velocity_gradient,
+                 lambda: g.stress_summary(0.01, 0.001, 0.7)):
+        call()
+        assert free() >= before - (64 << 20)
