@@ -54,8 +54,9 @@ class StagePool {
       }
     }
     void* b = nullptr;
-    return cudaHostAlloc(&b, SLOTS * SLOT_BYTES, cudaHostAllocPortable) == cudaSuccess ? static_cast<char*>(b)
-                                                                                       : nullptr;
+    if (cudaHostAlloc(&b, SLOTS * SLOT_BYTES, cudaHostAllocPortable) == cudaSuccess) return static_cast<char*>(b);
+    cudaGetLastError();  // else the next launch check reports this failure
+    return nullptr;
   }
   void give(char* b) {
     {

@@ -7,10 +7,11 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lbmflow_b200", "csrc")
 
 
-def run_cpp(tmp_path, body):
+def run_cpp(tmp_path, body, *flags):
     src, exe = tmp_path / "t.cpp", tmp_path / "t"
     src.write_text(body)
-    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", *flags, "-I", CSRC, str(src), "-o", str(exe)],
+                   check=True)
     return subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout
 
 
@@ -108,3 +109,94 @@ int main() {
 }
 """)
     assert out.split() == "2 1 4 1 2 1 0 1 2 1 2 1 0 1 2 1 0 1".split()
+
+
+FAKE_CUDA = r"""
+#pragma once
+#include <atomic>
+#include <cstddef>
+#include <cstdlib>
+using cudaError_t = int;
+using cudaStream_t = void*;
+using cudaEvent_t = void*;
+enum { cudaSuccess = 0, cudaErrorMemoryAllocation = 2, cudaErrorUnknown = 999 };
+enum { cudaHostAllocPortable = 1, cudaEventDisableTiming = 2 };
+inline std::atomic<int> fake_last{0}, fake_blocks{0}, fake_events{0};
+inline bool fake_no_memory = false;
+inline cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+  if (fake_no_memory) return fake_last = cudaErrorMemoryAllocation;
+  ++fake_blocks;
+  *p = std::malloc(n);
+  return cudaSuccess;
+}
+inline cudaError_t cudaFreeHost(void* p) { --fake_blocks; std::free(p); return cudaSuccess; }
+inline cudaError_t cudaGetLastError() { return fake_last.exchange(0); }
+inline cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { ++fake_events; *e = nullptr; return cudaSuccess; }
+inline cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+inline cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+inline cudaError_t cudaEventDestroy(cudaEvent_t) { --fake_events; return cudaSuccess; }
+"""
+
+
+def test_readback_chunks_threads_and_failures(tmp_path):
+    # a fake of the few CUDA calls: every cell of every field once, in chunks
+    # of any worker; blocks and events given back, also by a failing chunk;
+    # without pinned memory an error and nothing left for the next check
+    (tmp_path / "cuda_runtime.h").write_text(FAKE_CUDA)
+    out = run_cpp(tmp_path, r"""
+#include <cstdio>
+#include <stdexcept>
+#include "readback.hpp"
+using lbmb::ReadField;
+static void check(cudaError_t e) { if (e != cudaSuccess) throw std::runtime_error("cuda"); }
+int main() {
+  auto pool = lbmb::StagePool::get();
+  long bad = 0;
+  const int64_t slot = int64_t(lbmb::StagePool::SLOT_BYTES);
+  for (int64_t n : {int64_t(1), int64_t(127), slot / 64 - 1, slot / 64, slot / 64 + 1, 5 * (slot / 64) + 77}) {
+    std::vector<double> a(size_t(6 * n), -1.0), b(size_t(n), -1.0), c(size_t(n), -1.0);
+    lbmb::read_fields(0, nullptr, *pool, n, {ReadField{a.data(), 6}, ReadField{b.data(), 1}, ReadField{c.data(), 1}},
+                      [&](const std::vector<double*>& d, int64_t c0, int64_t c1) {
+                        for (int64_t i = c0; i < c1; ++i) {
+                          for (int k = 0; k < 6; ++k) d[0][6 * (i - c0) + k] = double(10 * i + k);
+                          d[1][i - c0] = double(i);
+                          d[2][i - c0] = double(-i);
+                        }
+                      },
+                      check);
+    for (int64_t i = 0; i < n; ++i) {
+      for (int k = 0; k < 6; ++k) bad += a[size_t(6 * i + k)] != double(10 * i + k);
+      bad += b[size_t(i)] != double(i) || c[size_t(i)] != double(-i);
+    }
+  }
+  std::printf("%ld\n", bad);
+  // a chunk that fails: the error arrives, the block goes back to the pool
+  std::vector<double> v(static_cast<size_t>(slot));
+  bool thrown = false;
+  try {
+    lbmb::read_fields(0, nullptr, *pool, slot, {ReadField{v.data(), 1}},
+                      [&](const std::vector<double*>&, int64_t c0, int64_t) {
+                        if (c0 > slot / 2) throw std::runtime_error("launch");
+                      },
+                      check);
+  } catch (const std::runtime_error&) {
+    thrown = true;
+  }
+  std::printf("%d %d %d\n", thrown, fake_blocks.load(), fake_events.load());
+  char* const held = pool->take();  // the pool's block is in use, no other to be had
+  fake_no_memory = true;
+  thrown = false;
+  try {
+    lbmb::read_fields(0, nullptr, *pool, 8, {ReadField{v.data(), 1}},
+                      [](const std::vector<double*>&, int64_t, int64_t) {}, check);
+  } catch (const std::runtime_error&) {
+    thrown = true;
+  }
+  std::printf("%d %d\n", thrown, cudaGetLastError());
+  pool->give(held);
+  pool.reset();
+  std::printf("%d\n", fake_blocks.load());
+}
+""", "-pthread", "-I", str(tmp_path))
+    assert out.split() == "0 1 1 0 1 0 0".split()
