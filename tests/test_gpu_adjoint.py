@@ -96,6 +96,32 @@ def test_adjoint_f32_tracks_f64(case):
     assert np.linalg.norm(g32 - g64) <= 1e-3 * np.linalg.norm(g64)
 
 
+@pytest.mark.parametrize("warm", [0, 3])
+@pytest.mark.parametrize("storage", ["f64", "f32"])
+def test_adjoint_segments_as_graphs_equal_eager_ones(storage, warm):
+    # 101 steps in segments of 16 (six replayed as graphs and an odd
+    # remainder), of 26 (launched one by one) and in one: the same steps, so
+    # the same sums up to the order of the atomic additions into f64
+    # accumulators (at most 1e7 terms of one sign mix: 1e-12)
+    c, geo = tank()
+    got = []
+    for every in (16, 26, 102):
+        g = lb.Solver(c.dims, lattice=19, collision="trt", storage=storage, nu=c.nu, solid=geo["solid"])
+        body = lb.RotatingBody(geo["center"], [0.0, 0.0, c.omega], geo["marker_pos"], geo["marker_w"])
+        if warm:
+            g.run_impeller(body, warm, CFG)
+        r = g.adjoint_torque(body, 101, 37, every, CFG)
+        got.append((r, g.stage_out()))
+        g.close()
+    (a, fa), rest = got[0], got[1:]
+    for b, fb in rest:
+        assert np.array_equal(a["torque"], b["torque"]) and a["J"] == b["J"]
+        assert np.array_equal(fa, fb)
+        for k in ("dJ_dnu", "dJ_domega_z"):
+            assert abs(a[k] - b[k]) <= 1e-12 * abs(a[k]), k
+        assert np.abs(a["dJ_dpos"] - b["dJ_dpos"]).max() <= 1e-12 * np.abs(a["dJ_dpos"]).max()
+
+
 def test_adjoint_rejects_unsupported():
     c, geo = tank()
     g = lb.Solver(c.dims, lattice=27, collision="cm", storage="f32", nu=c.nu, solid=geo["solid"])
