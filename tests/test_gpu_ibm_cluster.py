@@ -69,16 +69,30 @@ def test_force_field_keeps_its_rounding(nm, radius):
     assert np.isfinite(out).all() and zlib.crc32(out.tobytes()) == FIELD_CRC[nm, radius], hex(zlib.crc32(out.tobytes()))
 
 
-@pytest.mark.parametrize("storage", ["f32", "f16"])
-def test_runner_loop_repeats_bitwise(storage):
-    # the phases of one call are ordered by cluster barriers only: a missing
-    # one shows as a difference between two runs
+@pytest.mark.parametrize("T,q,coll,storage,kind", [
+    (32, 19, "trt", "f32", None), (32, 19, "trt", "f16", None), (32, 27, "cm", "f64", None),
+    # above 4,096 slots (the form of 1,024 threads), beside each persistent sweep
+    (112, 19, "trt", "f32", "pair"), (112, 19, "trt", "f16", "pair"), (112, 19, "trt", "f32", "lean"),
+    (112, 27, "cm", "f32", "async"), (112, 27, "cm", "bf16", "window"), (112, 27, "cm", "f16", "pair")])
+def test_runner_loop_repeats_bitwise(T, q, coll, storage, kind):
+    # the phases of one call are ordered by cluster barriers only, and the
+    # sweep runs beside it: a missing barrier or a shared slot shows as a
+    # difference between two runs
     from lbmflow_b200 import sweep
+    case = sweep.TankCase(T, 0.05, 600.0)
+    geo = sweep.tank_geometry(T)
+    body = lb.RotatingBody(geo["center"], [0.0, 0.0, case.omega], geo["marker_pos"], geo["marker_w"])
     ref = None
     for _ in range(4):
-        g, body = sweep.build_case(sweep.TankCase(32, 0.05, 600.0), storage=storage)
+        g = lb.Solver(case.dims, lattice=q, collision=coll, storage=storage, nu=case.nu, solid=geo["solid"],
+                      smagorinsky_cs=0.1)
+        if kind:
+            g.set_sweep_kernel(kind)
         r = g.run_impeller(body, 40)
         got = (r["torque_lu"], r["ibm_iterations"], g.stage_out())
+        if T > 100:
+            assert np.count_nonzero(np.any(g.force_field().reshape(-1, 3) != 0.0, axis=1)) > 4096
+        g.close()
         if ref is not None:
             assert all(np.array_equal(a, b) for a, b in zip(ref, got))
         ref = got
