@@ -99,6 +99,55 @@ def test_pair_kernel_low_precision_matches_direct(prec, kind, q, coll):
     assert l2 < {"f16": 5e-3, "bf16": 5e-2}[prec], l2
 
 
+@pytest.mark.parametrize("kind,variant,q,coll", [
+    ("pair", (4, 4), 19, "trt"), ("pair", (13, 13), 19, "trt"), ("pair", (15, 5), 27, "trt"), ("pair", (4, 3), 27, "cm"),
+    ("pair", (13, 14), 27, "cm"), ("tile", None, 19, "trt"), ("tile", None, 27, "cm"), ("lean", None, 19, "trt"),
+    ("lean", None, 27, "trt"), ("window", None, 19, "trt"), ("window", None, 27, "cm")])
+@pytest.mark.parametrize("prec", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("odd", [False, True])
+def test_one_step_within_the_storage_rounding_of_direct(odd, prec, kind, variant, q, coll):
+    # one step of each parity from the same state. Both kernels compute in
+    # fp32 with the density rounded at 1 (a few times 2^-24) and round to the
+    # storage once, so a population may differ by one unit of it at most; a
+    # wrong link or a lost element is a thousand times that
+    from cases import seeded_state
+    dims = (20, 14, 10)
+    solid = np.zeros(dims[::-1], np.uint8)
+    solid[0] = solid[-1] = 1
+    solid[:, 0] = solid[:, -1] = 1
+    solid[3, 4, 7] = solid[5, 8, 12] = solid[6, 8, 2:6] = 1  # odd and even ends of half-solid pairs
+    fl3 = solid == 0
+    wall = np.zeros(dims[::-1] + (3,))
+    wall[:, 0, :, 0] = 0.01  # a moving wall
+    kw = dict(lattice=q, collision=coll, storage=prec, nu=0.02, solid=solid.ravel(), smagorinsky_cs=0.1,
+              wall_u=wall.reshape(-1, 3), periodic=(True, False, False), free_slip_top=True)
+    f = seeded_state(q, solid.size, 5, scale=2e-3)
+    f[:, ~fl3.ravel()] = 0.0
+    out = []
+    for k in ("direct", kind):
+        g = lb.Solver(dims, **kw)
+        g.set_sweep_kernel("direct")
+        g.stage_in(f)
+        if odd:
+            g.run(1)
+        g.set_sweep_kernel(k)
+        if k != "direct" and variant:
+            g.set_sweep_variant(*variant)
+        g.run(1)
+        out.append(g.stage_out())
+    bits = {"f32": 24, "f16": 11, "bf16": 8}[prec]
+    size = np.maximum(np.abs(out[0]), np.abs(out[1]))
+    unit = 2.0 ** (np.floor(np.log2(np.maximum(size, 2.0 ** -14 if prec == "f16" else 1e-30))) + 1 - bits)
+    excess = np.abs(out[0] - out[1]) - unit - 8 * 2.0 ** -24
+    assert np.abs(out[0]).max() > 5e-3
+    z3, y3, x3 = np.meshgrid(np.arange(10), np.arange(14), np.arange(20), indexing="ij")
+    half = fl3 & (solid[:, :, np.arange(20) ^ 1] != 0)
+    groups = {"half-solid pair": half, "slip": fl3 & (z3 == 8), "wrap": fl3 & ((x3 == 0) | (x3 == 19)),
+              "moving wall": fl3 & (y3 == 1), "any": fl3}
+    for name, m in groups.items():
+        assert m.any() and excess[:, m.ravel()].max() <= 0.0, name
+
+
 # CRC-32 of the fluid populations after six steps from integer-made inputs, as
 # the pair kernel gave them with its back transform written out line by line:
 # a form of the collision that rounds elsewhere moves 16-bit runs.
