@@ -278,11 +278,8 @@ __global__ void wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typena
       sdsd = sdsd + sd[i][j] * sd[i][j];
     }
   const A cwd = A(0.325) * A(1);
-  // the powers 5/2, 5/4 and 3/2 as products and square roots (each within
-  // two roundings; three pow calls took most of the kernel's instructions)
-  const A rt = sqrt(sdsd);
-  const A denom = ss * ss * sqrt(ss) + sdsd * sqrt(rt);
-  A nut = denom > A(0) ? (cwd * cwd) * (sdsd * rt) / denom : A(0);
+  const A denom = pow(ss, A(2.5)) + pow(sdsd, A(1.25));
+  A nut = denom > A(0) ? (cwd * cwd) * pow(sdsd, A(1.5)) / denom : A(0);
   if (nut == nut) {  // the reference's max ignores NaN
     const double nd = double(nut);
     atomicMax(maxbits, (unsigned long long)__double_as_longlong(nd));

@@ -133,3 +133,31 @@ def test_field_refusals_and_removal():
         s.wale_update()
     with pytest.raises(lb.SpecError):
         g.wale_update(0.4)
+
+
+# CRC-32 of nu_t from integer-made inputs, with the reference's powers: other
+# forms of them round elsewhere, and a 16-bit run that renews the field
+# amplifies that (fp16 tank of 72 cells: nu_t 3e-3 apart after 80 steps).
+NU_T_CRC = {(19, "trt", "f32"): 0x3d13b3d9, (19, "trt", "f16"): 0x8f739c1d, (27, "cm", "f32"): 0xab4c7e45,
+            (27, "cm", "f64"): 0x9caea76d}
+
+
+@pytest.mark.parametrize("q,coll,storage", list(NU_T_CRC))
+def test_nu_t_keeps_its_rounding(q, coll, storage):
+    import zlib
+    solid = np.zeros((14, 12, 18), np.uint8)
+    solid[0] = solid[-1] = 1
+    solid[:, 0] = solid[:, -1] = 1
+    solid[:, :, 0] = solid[:, :, -1] = 1
+    solid = solid.ravel()
+    g = lb.Solver((18, 12, 14), lattice=q, collision=coll, storage=storage, nu=0.01, solid=solid)
+    i = np.arange(q * g.n, dtype=np.uint64)
+    f = ((i * np.uint64(2654435761) >> np.uint64(15)) % np.uint64(65536)).astype(np.float64) / 65536.0 - 0.5
+    f = (4e-3 * f).reshape(q, g.n)
+    f[:, solid != 0] = 0.0
+    g.stage_in(f)
+    for _ in range(3):
+        nu_t, _ = g.wale_update()
+        g.run(2)
+    out = np.ascontiguousarray(nu_t + 0.0)
+    assert out.max() > 1e-4 and zlib.crc32(out.tobytes()) == NU_T_CRC[q, coll, storage], hex(zlib.crc32(out.tobytes()))
