@@ -215,17 +215,6 @@ __device__ __forceinline__ void cm_bwd2(float2& k0, float2& k1, float2& k2, floa
   k2 = fp;
 }
 
-// The same with the moments of order 1 and 2 already halved (the transform is
-// linear, so the halves, which are exact, are taken once at its input, and
-// the rounding is that of cm_bwd2): hu = u/2, hu2 = u^2/2, u2 = 2u.
-__device__ __forceinline__ void cm_bwd2h(float2& k0, float2& k1, float2& k2, float2 hu, float2 hu2, float2 u2) {
-  const float2 m1 = fma2(hu, k0, k1);
-  const float2 m2 = fma2(hu2, k0, fma2(u2, k1, k2));
-  k1 = fma2(bc2(-2.f), m2, k0);
-  k0 = sub2(m2, m1);
-  k2 = add2(m2, m1);
-}
-
 // D3Q27 central-moment collision (kernels.rs:406-533, no force) of two
 // cells in float2 lanes, in the regularized form of collide_cm_x2
 // (hydro_async.cuh): f' = feq + T^-1 K', where K' holds only the five
@@ -297,11 +286,9 @@ __device__ __forceinline__ float2 cm_pair_reg(float2 (&f)[Q], const HydroParams<
   const float2 osc = fma2(os, mul2(usq, bc2(-0.16f)), os);
   const float2 keep = sub2(bc2(1.f), make_float2(fminf(osc.x, 2.f), fminf(osc.y, 2.f)));
   const float2 bulk = mul2(add2(add2(pxx, pyy), pzz), bc2(1.f / 3.f));
-  // moments of order 1 and 2 along y and z halved for cm_bwd2h
-  const float2 kh = mul2(keep, bc2(0.5f));
-  const float2 k200 = mul2(keep, sub2(pxx, bulk)), k020 = mul2(kh, sub2(pyy, bulk));
-  const float2 k002 = mul2(kh, sub2(pzz, bulk));
-  const float2 k110 = mul2(kh, pxy), k101 = mul2(kh, pxz), k011 = mul2(mul2(kh, bc2(0.5f)), pyz);
+  const float2 k200 = mul2(keep, sub2(pxx, bulk)), k020 = mul2(keep, sub2(pyy, bulk));
+  const float2 k002 = mul2(keep, sub2(pzz, bulk));
+  const float2 k110 = mul2(keep, pxy), k101 = mul2(keep, pxz), k011 = mul2(keep, pyz);
   // x pass: G[a][b][c], a = c_x + 1, on the six order-2 lines (b, c)
   const float2 ux2 = mul2(ux, ux);
   const float2 s0m = mul2(bc2(0.5f), sub2(ux2, ux)), s0p = mul2(bc2(0.5f), add2(ux2, ux));
@@ -330,19 +317,18 @@ __device__ __forceinline__ float2 cm_pair_reg(float2 (&f)[Q], const HydroParams<
   // y pass over b for each (a, c): c = 0 full, c = 1 without order 2,
   // c = 2 order 0 only
   const float2 uy2 = mul2(uy, uy);
-  const float2 huy = mul2(bc2(0.5f), uy), huy2 = mul2(bc2(0.5f), uy2), uyd = add2(uy, uy);
-  const float2 t0m = sub2(huy2, huy), t0p = add2(huy2, huy);
+  const float2 t0m = mul2(bc2(0.5f), sub2(uy2, uy)), t0p = mul2(bc2(0.5f), add2(uy2, uy));
   const float2 t00 = sub2(bc2(1.f), uy2);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    cm_bwd2h(G[a][0][0], G[a][1][0], G[a][2][0], huy, huy2, uyd);
+    cm_bwd2(G[a][0][0], G[a][1][0], G[a][2][0], uy);
     {
       const float2 k0 = G[a][0][1], k1 = G[a][1][1];
-      const float2 m1 = fma2(huy, k0, k1);
-      const float2 m2 = mul2(huy, fma2(uy, k0, mul2(bc2(4.f), k1)));  // k1 is a half
-      G[a][0][1] = sub2(m2, m1);
-      G[a][1][1] = fma2(bc2(-2.f), m2, k0);
-      G[a][2][1] = add2(m2, m1);
+      const float2 m1 = fma2(uy, k0, k1);
+      const float2 m2 = mul2(uy, fma2(uy, k0, mul2(bc2(2.f), k1)));
+      G[a][0][1] = mul2(bc2(0.5f), sub2(m2, m1));
+      G[a][1][1] = sub2(k0, m2);
+      G[a][2][1] = mul2(bc2(0.5f), add2(m2, m1));
     }
     {
       const float2 k0 = G[a][0][2];
@@ -352,11 +338,10 @@ __device__ __forceinline__ float2 cm_pair_reg(float2 (&f)[Q], const HydroParams<
     }
   }
   // z pass over c for each (a, b)
-  const float2 huz = mul2(bc2(0.5f), uz), huz2 = mul2(huz, uz), uzd = add2(uz, uz);
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) cm_bwd2h(G[a][b][0], G[a][b][1], G[a][b][2], huz, huz2, uzd);
+    for (int b = 0; b < 3; ++b) cm_bwd2(G[a][b][0], G[a][b][1], G[a][b][2], uz);
   // f' = feq + G: w (drho + rho (3 cu + 4.5 cu^2 - 1.5 u^2)), opposite
   // directions from the same cu (4.5 cu - 3 times cu for the second: the
   // same roundings with the sign moved)
@@ -438,12 +423,14 @@ __device__ __forceinline__ float2 ld2_odd(const S* p) {
 //     plane Q, which nothing reads.
 // Cells on a periodic face, under the free-slip top or next to a moving
 // wall take the generic path.
-// Measured on B200 (runner step of the 128 x 128 x 160 tank, D3Q27 fp32):
-// 122.5 us with the order-1 and order-2 moments scaled inside every line of
-// the backward transform, a select per population for cells at rest and
-// per-element stores on even-step wall tiles, 112.5 us in this form (128
-// registers instead of 168 suffice); a branch per direction around the wall
-// accesses of the odd step: 138 us.
+// Measured on B200 (runner step of the 128 x 128 x 160 tank, D3Q27 fp32, best
+// budgets): 119 us with c.u formed and a select made per population and
+// per-element stores on even-step wall tiles, 114.5 us in this form (128
+// registers instead of 168 suffice on the odd step). The back transform's
+// moments halved at its input instead of in every line: 113.4 us, but
+// subnormal numbers, which the front of a flow started from rest passes
+// through, then lose a bit. A branch per direction around the wall accesses of
+// the odd step: 138 us.
 constexpr int PAIR_TILE = 64;
 constexpr uint32_t TILE_BND = 0x80000000u;  // tile-list bit: a fluid cell of the tile has a solid neighbour
 

@@ -151,13 +151,16 @@ def test_one_step_within_the_storage_rounding_of_direct(odd, prec, kind, variant
 # CRC-32 of the fluid populations after six steps from integer-made inputs, as
 # the pair kernel gave them with its back transform written out line by line:
 # a form of the collision that rounds elsewhere moves 16-bit runs.
-CM_PAIR_CRC = {("f32", 0.0): 0xe1ad584d, ("f32", 0.1): 0x665243bf, ("f16", 0.0): 0x0344f91a,
-               ("f16", 0.1): 0x4315d52e, ("bf16", 0.0): 0xf92ea331, ("bf16", 0.1): 0x4681b840}
+CM_PAIR_CRC = {("f32", 0.0, 1.0): 0xe1ad584d, ("f32", 0.1, 1.0): 0x665243bf, ("f16", 0.0, 1.0): 0x0344f91a,
+               ("f16", 0.1, 1.0): 0x4315d52e, ("bf16", 0.0, 1.0): 0xf92ea331, ("bf16", 0.1, 1.0): 0x4681b840,
+               # subnormal numbers, as at the front of a flow started from rest
+               ("f32", 0.0, 2.0 ** -120): 0xc8c4fdc8, ("f32", 0.1, 2.0 ** -116): 0xaffd55fb,
+               ("bf16", 0.1, 2.0 ** -119): 0x7cad5cf7}
 
 
 @pytest.mark.parametrize("variant", [(4, 4), (3, 13)])
-@pytest.mark.parametrize("prec,cs", list(CM_PAIR_CRC))
-def test_pair_central_moment_keeps_its_rounding(prec, cs, variant):
+@pytest.mark.parametrize("prec,cs,scale", list(CM_PAIR_CRC))
+def test_pair_central_moment_keeps_its_rounding(prec, cs, scale, variant):
     import zlib
     dims = (20, 12, 10)
     solid = np.zeros(dims[::-1], np.uint8)
@@ -171,13 +174,14 @@ def test_pair_central_moment_keeps_its_rounding(prec, cs, variant):
     g.set_sweep_variant(*variant)
     i = np.arange(27 * g.n, dtype=np.uint64)
     f = ((i * np.uint64(2654435761) >> np.uint64(16)) % np.uint64(65536)).astype(np.float64) / 65536.0 - 0.5
-    f = (4e-3 * f).reshape(27, g.n)
+    f = (4e-3 * scale * f).reshape(27, g.n)
     f[:, solid != 0] = 0.0
     f[:, np.arange(g.n) // (dims[0] * dims[1]) > 6] = 0.0  # cells at exact rest too
     g.stage_in(f)
     g.run(6)
     out = np.ascontiguousarray(g.stage_out()[:, solid == 0] + 0.0)
-    assert np.abs(out).max() < 0.1 and zlib.crc32(out.tobytes()) == CM_PAIR_CRC[prec, cs], hex(zlib.crc32(out.tobytes()))
+    crc = zlib.crc32(out.tobytes())
+    assert 1e-3 * scale < np.abs(out).max() < 0.1 * scale and crc == CM_PAIR_CRC[prec, cs, scale], hex(crc)
 
 
 @pytest.mark.parametrize("variant", [(4, 4), (13, 13)])
