@@ -43,16 +43,16 @@ sys.path.insert(0, ROOT)
 PEAKS_FILE = os.path.join(ROOT, "MEASURED_PEAKS.json")
 
 # DRAM traffic per launch (dram__bytes_read.sum + dram__bytes_write.sum, mean of
-# one even and one odd launch) from an ncu full-set capture of the sweep kernel
-# the autotuner picks for the form, on the tank of the given diameter.
+# one even and one odd launch) from an ncu capture of the sweep kernel the
+# autotuner picks for the form, on the tank of the given diameter.
 NCU_TRAFFIC = {("hydro_async_kernel", 27, "cm", "f32", 128): 448.2e6,
-               ("hydro_pair_kernel", 27, "cm", "f32", 128): 466.0e6,
-               ("hydro_pair_kernel", 19, "trt", "f32", 256): 2720.2e6,
-               ("hydro_pair_kernel", 19, "trt", "f16", 256): 1406.1e6,
-               ("hydro_pair_kernel", 19, "trt", "bf16", 256): 1403.9e6,
-               ("hydro_pair_kernel", 27, "cm", "f32", 256): 3916.6e6,
-               ("hydro_pair_kernel", 27, "cm", "f16", 256): 2006.1e6,
-               ("hydro_pair_kernel", 27, "cm", "bf16", 256): 2016.5e6}
+               ("hydro_pair_kernel", 27, "cm", "f32", 128): 458.0e6,
+               ("hydro_pair_kernel", 19, "trt", "f32", 256): 2732e6,
+               ("hydro_pair_kernel", 19, "trt", "f16", 256): 1401.9e6,
+               ("hydro_pair_kernel", 19, "trt", "bf16", 256): 1401.9e6,
+               ("hydro_pair_kernel", 27, "cm", "f32", 256): 3880e6,
+               ("hydro_pair_kernel", 27, "cm", "f16", 256): 1998e6,
+               ("hydro_pair_kernel", 27, "cm", "bf16", 256): 1999e6}
 KERNEL_NAME = {"lean": "hydro_lean_kernel", "pair": "hydro_pair_kernel", "tile": "hydro_tile_kernel",
                "window": "hydro_window_kernel", "async": "hydro_async_kernel", "direct": "hydro_aa_kernel",
                "bulk": "hydro_tma_kernel"}

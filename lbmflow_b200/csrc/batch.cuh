@@ -72,11 +72,13 @@ static __global__ void __launch_bounds__(BATCH_BLOCK) batch_cells_kernel(const B
 
 // The direct forcing of every case, cluster k working on case k; the runner
 // clears the force field before it, so the field at call time is zero.
-// Small blocks (64 registers a thread), so that the clusters of many cases run at once: the sweep starts when the last
+// Small blocks (64 registers a thread, which spill 296 bytes and load 436), so
+// that the clusters of many cases run at once: the sweep starts when the last
 // of them has.
 constexpr int BATCH_IBM_THREADS = 256;
 template <int Q, class S>
-static __global__ void __launch_bounds__(BATCH_IBM_THREADS, 4) batch_ibm_kernel(const BatchCase* cs, int parity, int sweeps) {
+static __global__ void __launch_bounds__(BATCH_IBM_THREADS, 4)
+    batch_ibm_kernel(const BatchCase* cs, int parity, int sweeps) {
   release_dependents();
   int rank, ncta;
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));

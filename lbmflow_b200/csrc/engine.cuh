@@ -899,7 +899,6 @@ struct Engine final : EngineBase {
         launch_tile<ODD, COLL>(p, s);
       } else if (kernel_mode == LBMB_SWEEP_LEAN && lean_ok(COLL) && !p.uniform_force) {
         launch_lean<ODD>(p, s);
-
       } else if (!p.uniform_force && kernel_mode == 1) {
         if (rows_aligned) launch_tma<COLL, ODD, true>(p, s);
         else launch_tma<COLL, ODD, false>(p, s);
@@ -2019,8 +2018,12 @@ struct Engine final : EngineBase {
       r.sv_slots = int64_t(sv->ns3);
     }
     cudaStream_t sx = s_ ? s_ : st;
-    // one round of up to 8 x 512 entries with 8 gathers in flight, else 8 x
-    // 1024 threads with 4 (T = 128 tank: 6,186 slots)
+    // One round of up to 8 x 512 entries with 8 gathers in flight, else 8 x
+    // 1024 threads with 4. D3Q19 fp32 tanks, us per runner step in the first /
+    // second form: 1,118 slots 22.4 / 28.7, 3,836 37.0 / 42.9, 4,158 48.4 /
+    // 51.2, 5,042 65.9 / 64.1, 6,292 89.5 / 86.7, 7,753 116.5 / 117.7. The
+    // second has 64 registers a thread and spills (180 bytes stored, 220
+    // loaded); the first 128, with 56 and 24.
     if (std::max(B.ns, B.nm) <= int64_t(IBM_CLUSTER) * 512)
       launch_cluster(ibm_chain_kernel<Q, S, 512, 8>, 1, 512, sx, a, r);
     else
@@ -2861,7 +2864,12 @@ struct Engine final : EngineBase {
     const int64_t nseg = ceil_div(N, K);
     // Whole segments replay as graphs where they repeat often enough: each
     // buffer's graph is used every other segment, and capturing and
-    // instantiating one costs about two eager passes of its launches.
+    // instantiating one costs about two eager passes of its launches. Calls in
+    // segments of 20 steps, launched one by one / as graphs, ms on B200 (calls
+    // of one kind differ by up to a fifth): tank of 48, 2 segments 13.8 / 20.4,
+    // 4 19.9 / 24.5, 6 25.8 / 33.0; 64, 2 17.1 / 22.0, 4 25.7 / 28.0, 8 44.7 /
+    // 40.7, 12 54.3 / 53.3; 96, 2 26.4 / 31.3, 4 40.4 / 43.2, 8 77.3 / 65.7, 12
+    // 91.5 / 88.3.
     const bool graphs = nseg >= 6;
     const size_t fsz = size_t(Q) * size_t(plane);
     const size_t ns3 = size_t(std::max<int64_t>(nslots, 1));

@@ -237,9 +237,10 @@ __device__ __forceinline__ void vel_grad_cell(const StrainArgs<S>& a, const doub
 
 // Velocity gradient of every cell (g9, n x 9 row-major) and / or WALE
 // (les.rs:120-211, Cw 0.325, Delta 1): nu_t and the omega+ field for the
-// next collision, cells [c0, c1) (g9 and nu_t start at cell c0); clip bound nu_t_max when clip != 0; counts[0] = clipped
-// cells, maxbits = bits of the largest nu_t before clipping (non-negative,
-// so integer order is value order).
+// next collision, cells [c0, c1) (g9 and nu_t start at cell c0); clip bound
+// nu_t_max when clip != 0; counts[0] = clipped cells, maxbits = bits of the
+// largest nu_t before clipping (non-negative, so integer order is value
+// order).
 template <int Q, class S>
 __global__ void wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typename Codec<S>::A>* wall_u, int per_x,
                             int per_y, int per_z, typename Codec<S>::A nu0, int clip,
