@@ -276,6 +276,7 @@ struct Engine final : EngineBase {
   // IBM
   std::vector<std::unique_ptr<BodyState>> bodies;
   DevBuf<IbmDiagDev> d_diag;
+  DevBuf<IbmWide> d_wide;
   DevBuf<int> d_err;  // device error flag (bounded waits)
   DevBuf<int> d_flag;  // scratch flag of clear_force_field
   int sm_count = 148;
@@ -362,6 +363,7 @@ struct Engine final : EngineBase {
     CK(cudaMemsetAsync(fslot.p, 0xff, size_t(n) * sizeof(int32_t), st));
     grow_slots(64);
     d_diag.alloc(1);
+    d_wide.alloc(1);
     d_err.alloc(1);
     CK(cudaMemsetAsync(d_err.p, 0, sizeof(int), st));
     d_flag.alloc(1);
@@ -1948,6 +1950,7 @@ struct Engine final : EngineBase {
     a.imp = B.imp.p;
     a.mob = B.mob.p;
     a.inv_mob = B.inv_mob.p;
+    a.wide = d_wide.p;
     a.rmf = B.rmf.p;
     a.part_spread = B.part_spread.p;
     a.part_diag = B.part_diag.p;
@@ -1984,10 +1987,16 @@ struct Engine final : EngineBase {
     size_t ns3, nm;
   };
 
-  // The direct forcing of one call: one cluster of IBM_CLUSTER blocks.
+  // Whether a body's forcing beside a sweep of `cells` cells runs as full-chip
+  // kernels instead of a cluster.
+  static bool wide_beside(const BodyState& B, int64_t cells) { return std::max(B.ns, B.nm) > ibm_wide_beside(cells); }
+  static bool wide_alone(const BodyState& B) { return std::max(B.ns, B.nm) > IBM_WIDE_ALONE; }
+
+  // The direct forcing of one call: one cluster of IBM_CLUSTER blocks, or the
+  // wide form's kernels.
   // clear: the current field is zeroed first (the call then sees no field).
   void enqueue_ibm(BodyState& B, const lbmb_ibm_config& c, double* s_torque, double* s_ff, int32_t* s_it,
-                   int64_t* counter, bool field_at_call, bool clear, cudaStream_t s_ = nullptr,
+                   int64_t* counter, bool field_at_call, bool clear, bool wide, cudaStream_t sx,
                    const IbmSave* sv = nullptr) {
     const IbmArgs a = ibm_args(B, c);
     IbmRun<S> r = {};
@@ -2017,7 +2026,18 @@ struct Engine final : EngineBase {
       r.sv_imp = sv->imp;
       r.sv_slots = int64_t(sv->ns3);
     }
-    cudaStream_t sx = s_ ? s_ : st;
+    if (wide) {
+      auto blocks = [](int64_t k) { return unsigned(std::max<int64_t>(1, ceil_div(k, IBM_WIDE_BLOCK))); };
+      const unsigned gs = blocks(B.ns), gm = blocks(B.nm);
+      launch_wide(ibm_wide_prep_kernel<Q, S>, blocks(std::max(B.ns, clear ? nslots : 0)), false, sx, a, r);
+      launch_wide(ibm_wide_impulse_kernel<S>, gm, true, sx, a, r);
+      for (int s = 0; s < r.sweeps; ++s) {
+        launch_wide(ibm_wide_spread_kernel<S>, gs, true, sx, a, r, s);
+        launch_wide(ibm_wide_slip_kernel<S>, gm, true, sx, a, r, s);
+      }
+      launch_wide(ibm_wide_commit_kernel<S>, gs, true, sx, a, r);
+      return;
+    }
     // One round of up to 8 x 512 entries with 8 gathers in flight, else 8 x
     // 1024 threads with 4. D3Q19 fp32 tanks, us per runner step in the first /
     // second form: 1,118 slots 22.4 / 28.7, 3,836 37.0 / 42.9, 4,158 48.4 /
@@ -2028,6 +2048,22 @@ struct Engine final : EngineBase {
       launch_cluster(ibm_chain_kernel<Q, S, 512, 8>, 1, 512, sx, a, r);
     else
       launch_cluster(ibm_chain_kernel<Q, S, 1024, 4>, 1, 1024, sx, a, r);
+  }
+
+  // A kernel of the wide form; dependent: the programmatic dependent of the
+  // one before.
+  template <class... KArgs, class... Args>
+  static void launch_wide(void (*kernel)(KArgs...), unsigned grid, bool dependent, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(IBM_WIDE_BLOCK);
+    lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = dependent ? 1 : 0;
+    CK(cudaLaunchKernelEx(&lc, kernel, static_cast<KArgs>(args)...));
   }
 
   // n clusters of IBM_CLUSTER blocks.
@@ -2079,7 +2115,7 @@ struct Engine final : EngineBase {
 
   void ibm_apply(int b, const lbmb_ibm_config& c, lbmb_ibm_diag* out) override {
     BodyState& B = body_for(b, c);
-    enqueue_ibm(B, c, nullptr, nullptr, nullptr, nullptr, field_present, false);
+    enqueue_ibm(B, c, nullptr, nullptr, nullptr, nullptr, field_present, false, wide_alone(B), st);
     field_present = true;
     fprev_stale = true;
     IbmDiagDev d;
@@ -2126,10 +2162,8 @@ struct Engine final : EngineBase {
   void enqueue_runner_step(BodyState& B, const lbmb_ibm_config& c, bool captured) {
     const bool full = nslots == n;
     if (captured && full) enqueue_clear_device();
-    enqueue_ibm(B, c, nullptr, nullptr, nullptr, nullptr, false, captured && !full);
-    CK(cudaEventRecord(ev_fork, st));
-    CK(cudaStreamWaitEvent(st2, ev_fork, 0));
-    sweep_beside_ibm();
+    fork_forcing(B, c, nullptr, nullptr, nullptr, nullptr, captured && !full);
+    sweep_beside_ibm(B);
     CK(cudaMemcpyAsync(h_diag, d_diag.p, sizeof(IbmDiagDev), cudaMemcpyDeviceToHost, st2));
     // inside a graph, an external record node: the host waits on it
     CK(cudaEventRecordWithFlags(ev_diag, st2, captured ? cudaEventRecordExternal : cudaEventRecordDefault));
@@ -2649,20 +2683,19 @@ struct Engine final : EngineBase {
       // population slots (each cell's AA read/write set is its own).
       // Solver::clear_body_force_field: the IBM field is non-uniform, so the
       // cached moments keep it (F_prev) while the new field starts at zero.
-      enqueue_ibm(B, c, run_torque.p, run_ff.p, run_it.p, run_counter.p, false, true);
       field_present = true;
       fprev_stale = true;
       if (has_uniform_force()) {
+        enqueue_ibm(B, c, run_torque.p, run_ff.p, run_it.p, run_counter.p, false, true, wide_alone(B), st);
         // The sweep forces every cell: it reads the field and rewrites the
         // populations that the forcing works on, so the three follow each
         // other.
         launch_hydro(parity);
         if (nslots) CK(cudaMemcpyAsync(fprev.p, fcur.p, size_t(nslots) * sizeof(Vec4<A>), cudaMemcpyDeviceToDevice, st));
       } else {
-        CK(cudaEventRecord(ev_fork, st));
-        CK(cudaStreamWaitEvent(st2, ev_fork, 0));
+        fork_forcing(B, c, run_torque.p, run_ff.p, run_it.p, run_counter.p, true);
         launch_hydro(parity, st2, false, true);
-        sweep_beside_ibm();
+        sweep_beside_ibm(B);
         // cached-moment field refresh on the side stream behind the forced
         // cells, hidden by the full-grid sweep
         if (nslots)
@@ -2812,12 +2845,10 @@ struct Engine final : EngineBase {
   // side stream, full-grid sweep on the main stream, field refresh), eager.
   void enqueue_runner_step(BodyState& B, const lbmb_ibm_config& c, double* s_torque, int64_t* counter,
                            const IbmSave* sv = nullptr) {
-    enqueue_ibm(B, c, s_torque, nullptr, nullptr, counter, false, true, st, sv);
-    CK(cudaEventRecord(ev_fork, st));
-    CK(cudaStreamWaitEvent(st2, ev_fork, 0));
+    fork_forcing(B, c, s_torque, nullptr, nullptr, counter, true, sv);
     field_present = true;
     launch_hydro(parity, st2, false, true);
-    sweep_beside_ibm();
+    sweep_beside_ibm(B);
     CK(cudaEventRecord(ev_join, st2));
     CK(cudaStreamWaitEvent(st, ev_join, 0));
     parity ^= 1;
@@ -2825,6 +2856,19 @@ struct Engine final : EngineBase {
     fprev_stale = false;
   }
 
+  // The direct forcing of a runner step and the fork: what follows on st2 has
+  // the new field, the sweep comes next on st. The cluster starts first, on
+  // st, and the sweep once its blocks run (sweep_beside_ibm); the wide form's
+  // kernels share the chip with the sweep from the start, on the
+  // high-priority stream.
+  void fork_forcing(BodyState& B, const lbmb_ibm_config& c, double* s_torque, double* s_ff, int32_t* s_it,
+                    int64_t* counter, bool clear, const IbmSave* sv = nullptr) {
+    const bool wide = wide_beside(B, n);
+    if (!wide) enqueue_ibm(B, c, s_torque, s_ff, s_it, counter, false, clear, false, st, sv);
+    CK(cudaEventRecord(ev_fork, st));
+    CK(cudaStreamWaitEvent(st2, ev_fork, 0));
+    if (wide) enqueue_ibm(B, c, s_torque, s_ff, s_it, counter, false, clear, true, st2, sv);
+  }
   // Sweeps launched while one of these is alive follow the direct forcing.
   struct BesideIbm {
     bool& flag;
@@ -2832,8 +2876,12 @@ struct Engine final : EngineBase {
     ~BesideIbm() { flag = false; }
   };
   // The full-grid sweep of a runner step, launched on the main stream right
-  // behind the direct forcing.
-  void sweep_beside_ibm() {
+  // behind the direct forcing (the wide form: beside it).
+  void sweep_beside_ibm(const BodyState& B) {
+    if (wide_beside(B, n)) {
+      launch_hydro(parity, st, true, false);
+      return;
+    }
     BesideIbm beside(*this);
     launch_hydro(parity, st, true, false);
   }

@@ -17,10 +17,11 @@
 // What bounds it: latency. The data (a few MB) sits in L2 and each phase is
 // two or three dependent gathers, so the time is the number of phases times
 // (gathers + barrier). Per runner step on B200, as 2 + 3 x sweeps dependent
-// kernels -> in this form: 46.3 -> 21.7 us (48 x 48 x 60 tank, 1,139 slots;
-// 20 us of it the call), 69.0 -> 36.4 us (96 x 96 x 120), 131.6 -> 86.7 us
-// (128 x 128 x 160, D3Q19); where the sweep hides it, 121.2 -> 123.1 us
-// (128 x 128 x 160, D3Q27) and 408 -> 399 us (256 x 256 x 320, fp16).
+// kernels -> in this form: 46.2 -> 22.0 us (48 x 48 x 60 tank, 1,139 slots; 20
+// us of it the call), 74.7 -> 36.9 us (96 x 96 x 120), 133 -> 88 us (128 x 128
+// x 160, D3Q19); 121 -> 117 us (128 x 128 x 160, D3Q27, pair sweep) and 415 ->
+// 399 us (256 x 256 x 320, fp16), where the sweep hides it. Bodies of many more
+// markers take the wide form at the end of this file.
 //
 // Summation order: per slot the contributions are gathered in ascending
 // marker order (the reference's loop order), so spread, du and the cell
@@ -55,6 +56,8 @@ struct IbmDiagDev {
   int pad;
 };
 
+struct IbmWide;
+
 struct IbmArgs {
   // markers
   int64_t nm;
@@ -87,6 +90,7 @@ struct IbmArgs {
   double* part_spread;  // 2 x ceil(ns / IBM_CHUNK) x 3 (two sweeps in flight)
   double* part_diag;    // 2 x ceil(nm / IBM_CHUNK) x 9 (8 sums, then the maxima)
   IbmDiagDev* diag;
+  IbmWide* wide;        // state of the wide form
   double center[3], omega[3];
   double scale, relax, tol;
 };
@@ -346,6 +350,105 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
+// First impulse of marker m, its mobility with it.
+template <int NB, class S>
+__device__ __forceinline__ void ibm_first_impulse(const IbmArgs& a, const IbmRun<S>& r, int64_t m,
+                                                  const IbmIndex<NB>& ix) {
+  double t[3], x[3], um[3], mob;
+  ibm_target(a, m, t, x);
+  ibm_marker_velocity<NB, true>(a, ix, um, mob);
+  const double inv = reciprocal(mob);
+  a.mob[m] = mob;
+  a.inv_mob[m] = inv;
+  if (r.sv_mob) r.sv_mob[m] = mob;
+  ibm_impulse(a, r, m, t, um, mob, inv, 0);
+}
+
+// Slip statistics of marker m after sweep s (solver.rs:3211-3253): v = ssq,
+// wsum, force, torque; and the next sweep's impulse.
+template <int NB, class S>
+__device__ __forceinline__ void ibm_slip_marker(const IbmArgs& a, const IbmRun<S>& r, int s, int64_t m,
+                                                const IbmIndex<NB>& ix, double (&v)[8], double& smax) {
+  double t[3], x[3], um[3], none;
+  const double* f = a.rmf + 3 * m;
+  const double f0 = f[0], f1 = f[1], f2 = f[2], wt = a.weight[m];
+  const double mob = a.mob[m], inv = a.inv_mob[m];
+  ibm_target(a, m, t, x);
+  ibm_marker_velocity<NB, false>(a, ix, um, none);
+  if (ix.k1 > ix.k0) {
+    const double sl[3] = {t[0] - um[0], t[1] - um[1], t[2] - um[2]};
+    const double s2 = sl[0] * sl[0] + sl[1] * sl[1] + sl[2] * sl[2];
+    const double mag = sqrt(s2);
+    smax = fmax(mag, 0.0);  // a diverged state (NaN) has no slip
+    v[0] = wt * mag * mag;
+    v[1] = wt;
+  }
+  v[2] = f0;
+  v[3] = f1;
+  v[4] = f2;
+  v[5] = x[1] * f2 - x[2] * f1;
+  v[6] = x[2] * f0 - x[0] * f2;
+  v[7] = x[0] * f1 - x[1] * f0;
+  if (s + 1 < r.sweeps) ibm_impulse(a, r, m, t, um, mob, inv, s + 1);
+}
+
+// Force field += spread of slot i in the storage arithmetic
+// (solver.rs:3256-3279).
+template <class S>
+__device__ __forceinline__ void ibm_commit_slot(const IbmArgs& a, const IbmRun<S>& r, int64_t i) {
+  using A = typename Codec<S>::A;
+  const int32_t g = a.brec[i].x;
+  Vec4<A> v = r.fcur[g];
+  v.x = v.x + A(a.spread[3 * g + 0]);
+  v.y = v.y + A(a.spread[3 * g + 1]);
+  v.z = v.z + A(a.spread[3 * g + 2]);
+  r.fcur[g] = v;
+}
+
+// Diagnostics and series of a call by one warp, lane k holding the call's sum
+// k (0..1 slip, 2..4 marker force, 5..7 marker torque, 8..10 fluid force); the
+// torque on the body is minus the marker torque. slip_max, ssq, wsum: of the
+// last sweep, done: its number.
+template <class S>
+__device__ __forceinline__ void ibm_write_diag(const IbmArgs& a, const IbmRun<S>& r, int lane, double run,
+                                               double slip_max, double ssq, double wsum, int done) {
+  IbmDiagDev* d = a.diag;
+  const double sgn = lane >= 5 && lane < 8 ? -run : run;
+  const double e = __shfl_sync(0xffffffffu, run, lane < 3 ? lane + 8 : 0) -
+                   __shfl_sync(0xffffffffu, run, lane < 3 ? lane + 2 : 0);
+  const double f = __shfl_sync(0xffffffffu, run, lane < 3 ? lane + 2 : 0);
+  const double e0 = __shfl_sync(0xffffffffu, e, 0), e1 = __shfl_sync(0xffffffffu, e, 1),
+               e2 = __shfl_sync(0xffffffffu, e, 2);
+  const double f0 = __shfl_sync(0xffffffffu, f, 0), f1 = __shfl_sync(0xffffffffu, f, 1),
+               f2 = __shfl_sync(0xffffffffu, f, 2);
+  const int64_t st = r.step_counter ? *r.step_counter : 0;
+  __syncwarp();
+  if (lane >= 2 && lane < 5) d->marker_force[lane - 2] = run;
+  if (lane >= 5 && lane < 8) d->torque[lane - 5] = sgn;
+  if (lane >= 8 && lane < 11) d->fluid_force[lane - 8] = run;
+  if (r.step_counter) {
+    if (lane == 7 && r.series_torque) r.series_torque[st] = -sgn;
+    if (lane >= 8 && lane < 11 && r.series_ff) r.series_ff[3 * st + lane - 8] = run;
+  }
+  if (lane == 0) {
+    d->slip_max = slip_max;
+    d->slip_max_rel = slip_max / a.scale;
+    d->iterations = done;
+    if (r.step_counter) {
+      if (r.series_iters) r.series_iters[st] = done;
+      *r.step_counter = st + 1;
+    }
+  }
+  if (lane == 1) {
+    const double rms = wsum > 0.0 ? sqrt(ssq / wsum) : 0.0;
+    d->slip_rms = rms;
+    d->slip_rms_rel = rms / a.scale;
+  }
+  if (lane == 11)
+    d->momentum_error_rel =
+        sqrt(e0 * e0 + e1 * e1 + e2 * e2) / fmax(sqrt(f0 * f0 + f1 * f1 + f2 * f2), 1.0e-12);
+}
+
 // One apply_rotating_ibm call of one body by one cluster; rank: block in the
 // cluster, ncta: its blocks; NB: gathers in flight per thread. Every barrier
 // is reached by every thread: the sweep loop's exit is decided from the same
@@ -372,19 +475,10 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
   if (r.clear)
     for (int64_t s = tid; s < r.nslots; s += nthr) r.fcur[s] = Vec4<A>{A(0), A(0), A(0), A(0)};
   cluster_sync();
-  for (int64_t m = tid; m < a.nm; m += nthr) {
-    double t[3], x[3], um[3], mob;
-    ibm_target(a, m, t, x);
-    ibm_marker_velocity<NB, true>(a, marker_row(m), um, mob);
-    const double inv = reciprocal(mob);
-    a.mob[m] = mob;
-    a.inv_mob[m] = inv;
-    if (r.sv_mob) r.sv_mob[m] = mob;
-    ibm_impulse(a, r, m, t, um, mob, inv, 0);
-  }
+  for (int64_t m = tid; m < a.nm; m += nthr) ibm_first_impulse<NB>(a, r, m, marker_row(m));
   cluster_sync();
-  // block 0: running sums of the call (thread k of the first warp holds sum k:
-  // 0..1 slip, 2..4 marker force, 5..7 marker torque, 8..10 fluid force)
+  // block 0: running sums of the call, thread k of the first warp holding sum
+  // k of ibm_write_diag
   double run = 0.0, slip_max = 0.0, ssq = 0.0, wsum = 0.0;
   int done = 0;
   for (int s = 0; s < r.sweeps; ++s) {
@@ -407,35 +501,10 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
       }
     }
     cluster_sync();
-    // slip statistics (solver.rs:3211-3253) and the next sweep's impulse
     for (int64_t m0 = tid - lane; m0 < a.nm; m0 += nthr) {
       const int64_t m = m0 + lane;
-      double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // ssq, wsum, mf[3], tq[3]
-      double smax = 0.0;
-      if (m < a.nm) {
-        double t[3], x[3], um[3], none;
-        const double* f = a.rmf + 3 * m;
-        const double f0 = f[0], f1 = f[1], f2 = f[2], wt = a.weight[m];
-        const double mob = a.mob[m], inv = a.inv_mob[m];
-        ibm_target(a, m, t, x);
-        const IbmIndex<NB> ix = marker_row(m);
-        ibm_marker_velocity<NB, false>(a, ix, um, none);
-        if (ix.k1 > ix.k0) {
-          const double sl[3] = {t[0] - um[0], t[1] - um[1], t[2] - um[2]};
-          const double s2 = sl[0] * sl[0] + sl[1] * sl[1] + sl[2] * sl[2];
-          const double mag = sqrt(s2);
-          smax = fmax(mag, 0.0);  // a diverged state (NaN) has no slip
-          v[0] = wt * mag * mag;
-          v[1] = wt;
-        }
-        v[2] = f0;
-        v[3] = f1;
-        v[4] = f2;
-        v[5] = x[1] * f2 - x[2] * f1;
-        v[6] = x[2] * f0 - x[0] * f2;
-        v[7] = x[0] * f1 - x[1] * f0;
-        if (s + 1 < r.sweeps) ibm_impulse(a, r, m, t, um, mob, inv, s + 1);
-      }
+      double v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, smax = 0.0;
+      if (m < a.nm) ibm_slip_marker<NB>(a, r, s, m, marker_row(m), v, smax);
       smax = warp_max(smax);
       if (lane == 0) px[m0 / IBM_CHUNK] = smax;
       double* const p = pd + 8 * (m0 / IBM_CHUNK);
@@ -450,17 +519,21 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
     for (int64_t c = lane; c < nc_m; c += 32) amax = fmax(amax, px[c]);
     amax = __shfl_sync(0xffffffffu, warp_max(amax), 0);
     if (rank == 0) {
-      // the first block sums the partials, one warp per sum: lane t takes
-      // chunks t, t + 32, ... in order, then a tree (8 slip sums, then the 3
-      // spread sums)
+      // the first block sums the partials, one warp per sum (8 slip sums, then
+      // the 3 spread sums): four sums over every 128th chunk per lane, a tree
+      // for each, and the four in order, as the wide form's block of 128 does
       for (int k = warp; k < 11; k += int(blockDim.x) >> 5) {
-        double y = 0.0;
-        if (k < 8)
-          for (int64_t c = lane; c < nc_m; c += 32) y += pd[8 * c + k];
-        else
-          for (int64_t c = lane; c < nc_s; c += 32) y += ps[3 * c + k - 8];
-        y = warp_sum(y);
-        if (lane == 0) tot[k] = y;
+        const double* const p = k < 8 ? pd + k : ps + k - 8;
+        const int64_t n = k < 8 ? nc_m : nc_s, w = k < 8 ? 8 : 3;
+        double y[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int64_t c = lane; c < n; c += 128)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (c + 32 * j < n) y[j] += p[w * (c + 32 * j)];
+        double v = 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v += warp_sum(y[j]);
+        if (lane == 0) tot[k] = v;
       }
       __syncthreads();
       if (threadIdx.x < 11) run += tot[threadIdx.x];
@@ -472,60 +545,14 @@ __device__ __forceinline__ void ibm_chain(const IbmArgs& a, const IbmRun<S>& r, 
     done = s + 1;
     if (!r.sv_imp && amax / a.scale <= a.tol) break;  // the adjoint records a fixed number of sweeps
   }
-  // force field += spread in the storage arithmetic (solver.rs:3256-3279),
-  // by the blocks that have no diagnostics to write
+  // the commit by the blocks that have no diagnostics to write
   if (rank > 0 || ncta == 1) {
     const int first = ncta > 1 ? 1 : 0;
     const int64_t t0 = (int64_t(warp) * (ncta - first) + rank - first) * 32 + lane;
     const int64_t step = int64_t(ncta - first) * blockDim.x;
-    for (int64_t i = t0; i < a.ns; i += step) {
-      const int32_t g = a.brec[i].x;
-      Vec4<A> v = r.fcur[g];
-      v.x = v.x + A(a.spread[3 * g + 0]);
-      v.y = v.y + A(a.spread[3 * g + 1]);
-      v.z = v.z + A(a.spread[3 * g + 2]);
-      r.fcur[g] = v;
-    }
+    for (int64_t i = t0; i < a.ns; i += step) ibm_commit_slot(a, r, i);
   }
-  if (rank == 0 && warp == 0) {
-    // lane k holds sum k (see above); the torque on the body is minus the
-    // marker torque
-    IbmDiagDev* d = a.diag;
-    const double sgn = lane >= 5 && lane < 8 ? -run : run;
-    const double e = __shfl_sync(0xffffffffu, run, lane < 3 ? lane + 8 : 0) -
-                     __shfl_sync(0xffffffffu, run, lane < 3 ? lane + 2 : 0);
-    const double f = __shfl_sync(0xffffffffu, run, lane < 3 ? lane + 2 : 0);
-    const double e0 = __shfl_sync(0xffffffffu, e, 0), e1 = __shfl_sync(0xffffffffu, e, 1),
-                 e2 = __shfl_sync(0xffffffffu, e, 2);
-    const double f0 = __shfl_sync(0xffffffffu, f, 0), f1 = __shfl_sync(0xffffffffu, f, 1),
-                 f2 = __shfl_sync(0xffffffffu, f, 2);
-    const int64_t st = r.step_counter ? *r.step_counter : 0;
-    __syncwarp();
-    if (lane >= 2 && lane < 5) d->marker_force[lane - 2] = run;
-    if (lane >= 5 && lane < 8) d->torque[lane - 5] = sgn;
-    if (lane >= 8 && lane < 11) d->fluid_force[lane - 8] = run;
-    if (r.step_counter) {
-      if (lane == 7 && r.series_torque) r.series_torque[st] = -sgn;
-      if (lane >= 8 && lane < 11 && r.series_ff) r.series_ff[3 * st + lane - 8] = run;
-    }
-    if (lane == 0) {
-      d->slip_max = slip_max;
-      d->slip_max_rel = slip_max / a.scale;
-      d->iterations = done;
-      if (r.step_counter) {
-        if (r.series_iters) r.series_iters[st] = done;
-        *r.step_counter = st + 1;
-      }
-    }
-    if (lane == 1) {
-      const double rms = wsum > 0.0 ? sqrt(ssq / wsum) : 0.0;
-      d->slip_rms = rms;
-      d->slip_rms_rel = rms / a.scale;
-    }
-    if (lane == 11)
-      d->momentum_error_rel =
-          sqrt(e0 * e0 + e1 * e1 + e2 * e2) / fmax(sqrt(f0 * f0 + f1 * f1 + f2 * f2), 1.0e-12);
-  }
+  if (rank == 0 && warp == 0) ibm_write_diag(a, r, lane, run, slip_max, ssq, wsum, done);
 }
 
 // The sweep of the unforced cells is launched as this kernel's programmatic
@@ -539,6 +566,154 @@ template <int Q, class S, int NT, int NB>
 __global__ void __launch_bounds__(NT, 1) ibm_chain_kernel(IbmArgs a, IbmRun<S> r) {
   release_dependents();
   ibm_chain<Q, S, NB>(a, r, int(blockIdx.x), int(gridDim.x));
+}
+
+// ---- wide form ------------------------------------------------------------
+// The same phases as one full-chip kernel each, for bodies of so many entries
+// (slots or markers) that eight SMs take longer than the launches do. One entry
+// per thread; the last block of a slip kernel sums the sweep's partials (in the
+// cluster's order: both forms give the same bits) and decides the early exit,
+// and every kernel of a later sweep then returns at once. Each kernel is the
+// programmatic dependent of the one before and waits for its writes.
+constexpr int IBM_WIDE_BLOCK = 128;
+// Entries above which a call runs in this form: on its own, one round of the
+// cluster's smaller blocks (call with its readback on B200, cluster / wide, one
+// sweep: 3,836 slots 47 / 51 us, 4,553 48 / 53, 6,292 74 / 58, 13,694 106 / 61,
+// 133,915 552 / 90; three sweeps: 3,836 74 / 74, 6,292 108 / 82).
+constexpr int64_t IBM_WIDE_ALONE = IBM_CLUSTER * 512;
+// Beside a sweep of n cells, which hides the cluster on its own SMs but shares
+// the chip with the wide form, more of them: D3Q19 fp32 boxes, us per step with
+// the cluster / wide form, one sweep and three: 64^3 4,553 slots 32 / 36 and 52
+// / 53, 7,752 42 / 38 and 70 / 60, 20,421 93 / 44 and 163 / 69; 128^3 11,825 77
+// / 103 and 99 / 123, 18,285 85 / 105 and 130 / 127, 30,382 121 / 109 and 200 /
+// 135; 200^3 39,789 247 / 276 and 285 / 296, 63,598 283 / 281 and 423 / 316.
+inline int64_t ibm_wide_beside(int64_t n) { return 6000 + n / 200; }
+
+struct IbmWide {
+  double run[11];  // sums of the call (see ibm_write_diag)
+  double slip_max, ssq, wsum;
+  int done, converged;
+  unsigned int ticket;
+  int pad;
+};
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The phases for block `blk` of a body's blocks (all of a block's threads).
+template <int Q, class S>
+__device__ __forceinline__ void wide_prep(const IbmArgs& a, const IbmRun<S>& r, int64_t blk) {
+  using A = typename Codec<S>::A;
+  const int64_t i = blk * IBM_WIDE_BLOCK + threadIdx.x;
+  if (i == 0) *a.wide = IbmWide{};
+  if (i < a.ns) ibm_prep_slot<Q, S>(a, r, i);
+  if (r.clear && i < r.nslots) r.fcur[i] = Vec4<A>{A(0), A(0), A(0), A(0)};
+}
+
+template <class S>
+__device__ __forceinline__ void wide_impulse(const IbmArgs& a, const IbmRun<S>& r, int64_t blk) {
+  const int64_t m = blk * IBM_WIDE_BLOCK + threadIdx.x;
+  IbmIndex<8> ix;
+  if (m < a.nm) ix.load(a.st_off, a.st_slot, m);
+  pdl_wait();
+  if (m < a.nm) ibm_first_impulse<8>(a, r, m, ix);
+}
+
+template <class S>
+__device__ __forceinline__ void wide_spread(const IbmArgs& a, const IbmRun<S>& r, int s, int64_t blk) {
+  const int64_t i = blk * IBM_WIDE_BLOCK + threadIdx.x, i0 = i - (i & 31);
+  IbmIndex<8> ix;
+  if (i < a.ns) ix.load(a.cs_off, a.cs_marker, i);
+  pdl_wait();
+  if (a.wide->converged || i0 >= a.ns) return;
+  double ff[3] = {0.0, 0.0, 0.0};
+  if (i < a.ns) ibm_spread_slot<8>(a, r, s, ix, a.brec[i].x, ff);
+  for (int c = 0; c < 3; ++c) {
+    const double v = warp_sum(ff[c]);
+    if ((i & 31) == 0) a.part_spread[3 * (i0 / IBM_CHUNK) + c] = v;
+  }
+}
+
+// nblk: the body's blocks.
+template <class S>
+__device__ __forceinline__ void wide_slip(const IbmArgs& a, const IbmRun<S>& r, int s, int64_t blk, unsigned nblk) {
+  __shared__ double sh[12 * (IBM_WIDE_BLOCK / 32)];
+  __shared__ bool last;
+  const int64_t m = blk * IBM_WIDE_BLOCK + threadIdx.x, m0 = m - (m & 31);
+  const int64_t nc_m = (a.nm + IBM_CHUNK - 1) / IBM_CHUNK, nc_s = (a.ns + IBM_CHUNK - 1) / IBM_CHUNK;
+  double* const px = a.part_diag + 8 * nc_m;
+  IbmIndex<8> ix;
+  if (m < a.nm) ix.load(a.st_off, a.st_slot, m);
+  pdl_wait();
+  IbmWide* const w = a.wide;
+  if (w->converged) return;  // the same in every thread: only the last block sets it, at the end
+  if (m0 < a.nm) {
+    double v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, smax = 0.0;
+    if (m < a.nm) ibm_slip_marker<8>(a, r, s, m, ix, v, smax);
+    smax = warp_max(smax);
+    if ((m & 31) == 0) px[m0 / IBM_CHUNK] = smax;
+    for (int k = 0; k < 8; ++k) {
+      const double y = warp_sum(v[k]);
+      if ((m & 31) == 0) a.part_diag[8 * (m0 / IBM_CHUNK) + k] = y;
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&w->ticket, 1u) == nblk - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // thread t takes chunks t, t + 128, ... in order, then a tree
+  double acc[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0}, amax = 0.0;
+  for (int64_t c = threadIdx.x; c < nc_m; c += IBM_WIDE_BLOCK) {
+    amax = fmax(amax, __ldcg(px + c));
+    for (int k = 0; k < 8; ++k) acc[k] += __ldcg(a.part_diag + 8 * c + k);
+  }
+  for (int64_t c = threadIdx.x; c < nc_s; c += IBM_WIDE_BLOCK)
+    for (int k = 0; k < 3; ++k) acc[8 + k] += __ldcg(a.part_spread + 3 * c + k);
+  amax = warp_max(amax);
+  if ((threadIdx.x & 31) == 0) sh[11 * (IBM_WIDE_BLOCK / 32) + (threadIdx.x >> 5)] = amax;
+  block_sum<11>(acc, sh);
+  if (threadIdx.x != 0) return;
+  for (int k = 0; k < IBM_WIDE_BLOCK / 32; ++k) amax = fmax(amax, sh[11 * (IBM_WIDE_BLOCK / 32) + k]);
+  for (int k = 0; k < 11; ++k) w->run[k] += acc[k];
+  w->slip_max = amax;
+  w->ssq = acc[0];
+  w->wsum = acc[1];
+  w->done = s + 1;
+  w->converged = !r.sv_imp && amax / a.scale <= a.tol;  // the adjoint records a fixed number of sweeps
+  w->ticket = 0;
+}
+
+template <class S>
+__device__ __forceinline__ void wide_commit(const IbmArgs& a, const IbmRun<S>& r, int64_t blk) {
+  pdl_wait();
+  const int64_t i = blk * IBM_WIDE_BLOCK + threadIdx.x;
+  if (i < a.ns) ibm_commit_slot(a, r, i);
+  if (i < 32) {
+    const IbmWide* w = a.wide;
+    ibm_write_diag(a, r, int(i), i < 11 ? w->run[i] : 0.0, w->slip_max, w->ssq, w->wsum, w->done);
+  }
+}
+
+template <int Q, class S>
+__global__ void __launch_bounds__(IBM_WIDE_BLOCK) ibm_wide_prep_kernel(IbmArgs a, IbmRun<S> r) {
+  wide_prep<Q, S>(a, r, blockIdx.x);
+}
+template <class S>
+__global__ void __launch_bounds__(IBM_WIDE_BLOCK) ibm_wide_impulse_kernel(IbmArgs a, IbmRun<S> r) {
+  wide_impulse(a, r, blockIdx.x);
+}
+template <class S>
+__global__ void __launch_bounds__(IBM_WIDE_BLOCK) ibm_wide_spread_kernel(IbmArgs a, IbmRun<S> r, int s) {
+  wide_spread(a, r, s, blockIdx.x);
+}
+template <class S>
+__global__ void __launch_bounds__(IBM_WIDE_BLOCK) ibm_wide_slip_kernel(IbmArgs a, IbmRun<S> r, int s) {
+  wide_slip(a, r, s, blockIdx.x, gridDim.x);
+}
+template <class S>
+__global__ void __launch_bounds__(IBM_WIDE_BLOCK) ibm_wide_commit_kernel(IbmArgs a, IbmRun<S> r) {
+  wide_commit(a, r, blockIdx.x);
 }
 
 }  // namespace lbmb

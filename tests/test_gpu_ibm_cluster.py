@@ -39,6 +39,50 @@ def test_marker_counts_match_oracle(nm, radius, tol):
         assert np.abs(fg - fc).max() <= 1e-12 * np.abs(fc).max()
 
 
+def dense_body(n, nm):
+    """nm markers scattered in a disc of a closed box of n cells: about 8 slots
+    each while they are few."""
+    solid = np.zeros((n, n, n), np.uint8)
+    solid[0] = solid[-1] = 1
+    solid[:, 0] = solid[:, -1] = 1
+    solid[:, :, 0] = solid[:, :, -1] = 1
+    rng = np.random.default_rng(nm)
+    th, r = rng.uniform(0.0, 2.0 * np.pi, nm), rng.uniform(0.1 * n, 0.44 * n, nm)
+    z = 0.5 * n + rng.uniform(-1.0, 1.0, nm) * min(0.44 * n, 0.5 + nm / (0.6 * n * n))
+    pos = np.stack([0.5 * n + r * np.cos(th), 0.5 * n + r * np.sin(th), z], axis=1)
+    return solid.ravel(), lb.RotatingBody([0.5 * n] * 3, [0.0, 0.0, 0.0007], pos, np.full(nm, 0.3))
+
+
+@pytest.mark.parametrize("storage", ["f64", "f16"])
+@pytest.mark.parametrize("nm", [400, 1500, 3000, 6000])
+@pytest.mark.parametrize("tol", [1e-2, 0.0])
+def test_both_forms_give_the_same_bits(nm, tol, storage):
+    # a call on its own leaves the cluster for the full-chip kernels above 4,096
+    # slots, one beside a sweep above 6,000 + cells / 200 (6,460 here): the loop
+    # and the calls one by one then run different forms, and every form sums in
+    # the same order
+    solid, body = dense_body(45, nm)
+    a, b, c = (lb.Solver((45,) * 3, lattice=19, storage=storage, nu=0.03, solid=solid) for _ in range(3))
+    cfg = lb.DirectForcingConfig(3, tol, 1, 1.0)
+    r = a.run_impeller(body, 21, cfg)
+    tq, ff = [], []
+    for k in range(21):
+        b.clear_body_force_field()
+        d = b.apply_rotating_ibm(body, cfg)
+        b.run(1)
+        e = c.runner_step(0, body, cfg)
+        tq.append(-d.torque[2])
+        ff.append(d.fluid_force)
+        assert d.iterations == e.iterations == r["ibm_iterations"][k]
+        for key in ("slip_max", "slip_rms", "momentum_error_rel"):
+            assert getattr(d, key) == getattr(e, key), key
+        assert np.array_equal(d.torque, e.torque) and np.array_equal(d.marker_force, e.marker_force)
+    slots = int(np.count_nonzero(np.any(a.force_field().reshape(-1, 3) != 0.0, axis=1)))
+    assert {400: slots < 4096, 1500: 4096 < slots < 6400}.get(nm, slots > 6500), slots
+    assert np.array_equal(r["torque_lu"], np.array(tq)) and np.array_equal(r["fluid_force"], np.array(ff))
+    assert np.array_equal(a.stage_out(), b.stage_out()) and np.array_equal(a.stage_out(), c.stage_out())
+
+
 # CRC-32 of the force field after two calls from integer-made inputs, as a
 # chain of kernels with plain divisions gave it.
 FIELD_CRC = {(300, 1): 0xa94664c8, (300, 2): 0x0d310867, (5000, 1): 0xcbb8dd4d, (5000, 2): 0xfc32f19a}
