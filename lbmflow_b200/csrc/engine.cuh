@@ -3263,6 +3263,10 @@ struct Batch final : BatchBase {
   DevBuf<BatchCase> cases;
   DevBuf<int32_t> off_cells, off_slots;
   int nb_cells = 0, nb_slots = 0;
+  // cases forced by a cluster, and those in the wide form with their block
+  // offsets (prep, slots, markers)
+  DevBuf<int32_t> cluster_list, wide_list, off_wide[3];
+  int ncluster = 0, nwide = 0, nb_wide[3] = {0, 0, 0};
   DevBuf<double> d_torque;
   DevBuf<int64_t> d_counter;
 
@@ -3304,6 +3308,28 @@ struct Batch final : BatchBase {
     }
     nb_cells = oc.back();
     nb_slots = os.back();
+    int64_t total = 0;
+    for (E* e : eng) total += e->n;
+    std::vector<int32_t> small, big, ow[3] = {{0}, {0}, {0}};
+    for (int k = 0; k < ncase; ++k) {
+      const BodyState& B = *bod[size_t(k)];
+      if (std::max(B.ns, B.nm) <= batch_wide_from(total)) {
+        small.push_back(k);
+        continue;
+      }
+      big.push_back(k);
+      const int64_t count[3] = {std::max(B.ns, eng[k]->nslots), B.ns, B.nm};
+      for (int f = 0; f < 3; ++f)
+        ow[f].push_back(ow[f].back() + int32_t(std::max<int64_t>(1, ceil_div(count[f], IBM_WIDE_BLOCK))));
+    }
+    ncluster = int(small.size());
+    nwide = int(big.size());
+    cluster_list.upload(small, st);
+    wide_list.upload(big, st);
+    for (int f = 0; f < 3; ++f) {
+      off_wide[f].upload(ow[f], st);
+      nb_wide[f] = ow[f].back();
+    }
     off_cells.upload(oc, st);
     off_slots.upload(os, st);
     cases_h.resize(size_t(ncase));
@@ -3359,16 +3385,33 @@ struct Batch final : BatchBase {
 
   // One runner step of every case (runner.rs:1079-1129 per case).
   void one_step() {
-    E::launch_cluster(batch_ibm_kernel<Q, S>, unsigned(ncase), BATCH_IBM_THREADS, st, cases.p, parity,
-                      int(cfg.max_iterations));
+    const int sweeps = int(cfg.max_iterations);
+    if (ncluster)
+      E::launch_cluster(batch_ibm_kernel<Q, S>, unsigned(ncluster), BATCH_IBM_THREADS, st, cases.p, cluster_list.p,
+                        parity, sweeps);
     CK(cudaEventRecord(ev_fork, st));
     CK(cudaStreamWaitEvent(st2, ev_fork, 0));
+    if (nwide) {
+      auto phase = [&](auto kernel, int f, bool dependent, int s) {
+        E::launch_wide(kernel, unsigned(nb_wide[f]), dependent, st2, cases.p, wide_list.p, off_wide[f].p, nwide, parity,
+                       sweeps, s);
+      };
+      phase(batch_wide_kernel<WIDE_PREP, Q, S>, 0, false, 0);
+      phase(batch_wide_kernel<WIDE_IMPULSE, Q, S>, 2, true, 0);
+      for (int s = 0; s < sweeps; ++s) {
+        phase(batch_wide_kernel<WIDE_SPREAD, Q, S>, 1, true, s);
+        phase(batch_wide_kernel<WIDE_SLIP, Q, S>, 2, true, s);
+      }
+      phase(batch_wide_kernel<WIDE_COMMIT, Q, S>, 1, true, 0);
+    }
     if (parity) batch_cells_kernel<Q, S, true><<<unsigned(nb_slots), BATCH_BLOCK, 0, st2>>>(cases.p, off_slots.p, ncase);
     else batch_cells_kernel<Q, S, false><<<unsigned(nb_slots), BATCH_BLOCK, 0, st2>>>(cases.p, off_slots.p, ncase);
     batch_fprev_kernel<<<unsigned(nb_slots), BATCH_BLOCK, 0, st2>>>(cases.p, off_slots.p, ncase);
     CK(cudaGetLastError());
-    {
+    if (ncluster) {
       typename E::BesideIbm beside(*eng[0]);
+      hydro(parity);
+    } else {
       hydro(parity);
     }
     CK(cudaEventRecord(ev_join, st2));

@@ -89,3 +89,27 @@ def test_batch_rejects_mixed_or_unsupported():
     sc.enable_scalar_distribution(1e-3, q=7)
     with pytest.raises(lb.UnsupportedError):
         lb.Batch([sc], [body])
+
+
+def test_batch_of_small_and_large_bodies_equals_each_alone():
+    # bodies on both sides of the line between a cluster per case and the
+    # full-chip phases over the large ones (4,096 + cells / 400), early exits
+    # at different sweeps
+    from test_gpu_ibm_cluster import dense_body
+    cfg = lb.DirectForcingConfig(3, 0.02, 1, 1.0)
+    made = [dense_body(n, nm) + ((n,) * 3,) for n, nm in ((30, 40), (40, 3000), (33, 300), (45, 1200), (36, 2500))]
+    mk = lambda: [lb.Solver(d, lattice=19, storage="f32", nu=0.02 + 0.005 * i, solid=s)  # noqa: E731
+                  for i, (s, _, d) in enumerate(made)]
+    bodies = [b for _, b, _ in made]
+    together, alone = mk(), mk()
+    tq, _ = lb.Batch(together, bodies, cfg).run(37)
+    for k, g in enumerate(alone):
+        g.set_sweep_kernel("lean")
+        r = g.run_impeller(bodies[k], 37, cfg)
+        assert np.array_equal(tq[k], r["torque_lu"]), k
+        assert np.array_equal(g.stage_out(), together[k].stage_out()), k
+    # only large bodies, and only small ones
+    for part in ([1, 4], [0, 2]):
+        g = mk()
+        tq2, _ = lb.Batch([g[k] for k in part], [bodies[k] for k in part], cfg).run(37)
+        assert all(np.array_equal(tq2[j], tq[k]) for j, k in enumerate(part))
