@@ -467,4 +467,29 @@ __global__ void __launch_bounds__(ADJ_IBM_THREADS, 1) adj_ibm_kernel(AdjIbm b, i
   for (int64_t i = tid; i < ns; i += nthr) adj_ibm_fbar<Q, A>(b, lam, pl, i);
 }
 
+// The same phases as one full-chip kernel each, for bodies of more entries
+// (slots or markers) than ADJ_IBM_WIDE. Recomputation and backward pass, us per
+// step, cluster / these: tanks of 64 cells (1,736 slots) 133 / 168, 96 (3,836)
+// 245 / 278, 112 (5,042) 375 / 355, 128 (6,292) 497 / 464, 192 (13,694) 1331 /
+// 1207; a box of 64 cells with 36,122 slots 680 / 225.
+constexpr int64_t ADJ_IBM_WIDE = 4096;
+__device__ __forceinline__ int64_t adj_entry() { return int64_t(blockIdx.x) * ADJ_BLOCK + threadIdx.x; }
+static __global__ void __launch_bounds__(ADJ_BLOCK) adj_ibm_marker_kernel(AdjIbm b, int k) {
+  if (adj_entry() < b.a.nm) adj_ibm_marker(b, k, adj_entry());
+}
+static __global__ void __launch_bounds__(ADJ_BLOCK) adj_ibm_slot_kernel(AdjIbm b, int k) {
+  if (adj_entry() < b.a.ns) adj_ibm_slot(b, k, adj_entry());
+}
+static __global__ void __launch_bounds__(ADJ_BLOCK) adj_ibm_mob_slot_kernel(AdjIbm b) {
+  if (adj_entry() < b.a.ns) adj_ibm_mob_slot(b, adj_entry());
+}
+static __global__ void __launch_bounds__(ADJ_BLOCK) adj_ibm_mob_marker_kernel(AdjIbm b) {
+  const double gO = warp_sum(adj_entry() < b.a.nm ? adj_ibm_mob_marker(b, adj_entry()) : 0.0);
+  if ((threadIdx.x & 31) == 0 && gO != 0.0) atomicAdd(b.grad + 2, gO);
+}
+template <int Q, class A>
+__global__ void __launch_bounds__(ADJ_BLOCK) adj_ibm_fbar_kernel(AdjIbm b, A* lam, int64_t pl) {
+  if (adj_entry() < b.a.ns) adj_ibm_fbar<Q, A>(b, lam, pl, adj_entry());
+}
+
 }  // namespace lbmb

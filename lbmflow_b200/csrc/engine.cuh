@@ -3129,7 +3129,20 @@ struct Engine final : EngineBase {
         ab.xbar = xbar.p;
         ab.grad = grad.p;
         ab.tbar_step = b.tb.p + i;
-        launch_cluster(adj_ibm_kernel<Q, A>, 1, ADJ_IBM_THREADS, sb, ab, nsweep, lam_out, plane);
+        if (std::max(B.ns, B.nm) <= ADJ_IBM_WIDE) {
+          launch_cluster(adj_ibm_kernel<Q, A>, 1, ADJ_IBM_THREADS, sb, ab, nsweep, lam_out, plane);
+          continue;
+        }
+        const unsigned gs = unsigned(ceil_div(std::max<int64_t>(B.ns, 1), ADJ_BLOCK));
+        const unsigned gm = unsigned(ceil_div(std::max<int64_t>(B.nm, 1), ADJ_BLOCK));
+        for (int k = nsweep - 1; k >= 0; --k) {
+          adj_ibm_marker_kernel<<<gm, ADJ_BLOCK, 0, sb>>>(ab, k);
+          adj_ibm_slot_kernel<<<gs, ADJ_BLOCK, 0, sb>>>(ab, k);
+        }
+        adj_ibm_mob_slot_kernel<<<gs, ADJ_BLOCK, 0, sb>>>(ab);
+        adj_ibm_mob_marker_kernel<<<gm, ADJ_BLOCK, 0, sb>>>(ab);
+        adj_ibm_fbar_kernel<Q, A><<<gs, ADJ_BLOCK, 0, sb>>>(ab, lam_out, plane);
+        CK(cudaGetLastError());
       }
     };
     cudaGraphExec_t g_rec[2] = {nullptr, nullptr}, g_bwd[2] = {nullptr, nullptr};

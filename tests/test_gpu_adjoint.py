@@ -122,6 +122,39 @@ def test_adjoint_segments_as_graphs_equal_eager_ones(storage, warm):
         assert np.abs(a["dJ_dpos"] - b["dJ_dpos"]).max() <= 1e-12 * np.abs(a["dJ_dpos"]).max()
 
 
+@pytest.mark.parametrize("nm", [500, 1700])
+def test_adjoint_of_bodies_about_the_wide_line(nm):
+    # on both sides of 4,096 slots (the cluster, and one kernel per phase): the
+    # gradient along random marker directions and in the speed against central
+    # differences of the f64 forward
+    from test_gpu_ibm_cluster import dense_body
+    solid, body = dense_body(38, nm)
+    steps, win = 14, 4
+
+    def run(omega_z, pos):
+        g = lb.Solver((38,) * 3, lattice=19, storage="f64", nu=0.02, solid=solid)
+        b = lb.RotatingBody(body.center, [0.0, 0.0, omega_z], pos, body.weights)
+        t = g.run_impeller(b, steps, CFG)["torque_lu"]
+        slots = int(np.count_nonzero(np.any(g.force_field().reshape(-1, 3) != 0.0, axis=1)))
+        g.close()
+        return float(np.mean(t[win:])), slots
+
+    w, pos = body.omega[2], np.asarray(body.positions).reshape(-1, 3)
+    g = lb.Solver((38,) * 3, lattice=19, storage="f64", nu=0.02, solid=solid)
+    r = g.adjoint_torque(body, steps, win, 6, CFG)
+    J, slots = run(w, pos)
+    assert (slots > 4096) == (nm > 1000), slots
+    assert abs(r["J"] - J) <= 1e-13 * abs(J)
+    h = 1e-4 * w
+    fd = (run(w + h, pos)[0] - run(w - h, pos)[0]) / (2 * h)
+    assert abs(r["dJ_domega_z"] - fd) <= 1e-5 * abs(fd)
+    d = np.random.default_rng(4).normal(size=pos.shape)
+    d /= np.linalg.norm(d)
+    fd = (run(w, pos + 1e-6 * d)[0] - run(w, pos - 1e-6 * d)[0]) / 2e-6
+    ad = float(np.sum(r["dJ_dpos"].reshape(-1, 3) * d))
+    assert abs(ad - fd) <= 1e-5 * max(abs(fd), 1e-12) + 1e-9, (ad, fd)
+
+
 def test_adjoint_rejects_unsupported():
     c, geo = tank()
     g = lb.Solver(c.dims, lattice=27, collision="cm", storage="f32", nu=c.nu, solid=geo["solid"])
