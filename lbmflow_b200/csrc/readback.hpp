@@ -23,55 +23,77 @@
 
 namespace lbmb {
 
-// Pinned blocks of SLOTS slots, shared by the solvers of a process: at most
-// KEEP blocks stay allocated between readbacks, and all go when the last
-// solver does. A block belongs to one readback at a time.
+// Pinned blocks, shared by the solvers of a process: at most KEEP of them, of at
+// most SLOTS slots each, stay allocated between readbacks, and when the last
+// solver goes the largest one (4 MiB at most) stays for the next. Pinning takes
+// 2 to 5 ms whatever the size, which a program that makes one small solver after
+// another would pay for each (moments of a 32^3 grid 1.3 ms in all). A block
+// belongs to one readback at a time.
 class StagePool {
  public:
   static constexpr int SLOTS = 4;
-  static constexpr size_t SLOT_BYTES = size_t(2) << 20;
+  static constexpr size_t SLOT_BYTES = size_t(1) << 20;
   static constexpr size_t KEEP = 2;
+  struct Block {
+    char* p = nullptr;
+    size_t bytes = 0;
+  };
 
+  // The process's pool, held as long as a solver may read (never destroyed: a
+  // solver may go after the statics have).
   static std::shared_ptr<StagePool> get() {
+    static StagePool* const pool = new StagePool();
     static std::mutex mu;
-    static std::weak_ptr<StagePool> one;
+    static std::weak_ptr<StagePool> users;
     std::lock_guard<std::mutex> lk(mu);
-    std::shared_ptr<StagePool> p = one.lock();
-    if (!p) one = p = std::make_shared<StagePool>();
+    std::shared_ptr<StagePool> p = users.lock();
+    if (!p) users = p = std::shared_ptr<StagePool>(pool, [](StagePool* s) { s->shrink(1); });
     return p;
   }
-  ~StagePool() {
-    for (char* b : free_) cudaFreeHost(b);
-  }
-  // null when no pinned memory is left
-  char* take() {
+  // a block of at least `bytes`; null when no pinned memory is left
+  Block take(size_t bytes) {
     {
       std::lock_guard<std::mutex> lk(mu_);
-      if (!free_.empty()) {
-        char* b = free_.back();
-        free_.pop_back();
+      auto best = free_.end();
+      for (auto b = free_.begin(); b != free_.end(); ++b)
+        if (b->bytes >= bytes && (best == free_.end() || b->bytes < best->bytes)) best = b;
+      if (best != free_.end()) {
+        const Block b = *best;
+        free_.erase(best);
         return b;
       }
     }
-    void* b = nullptr;
-    if (cudaHostAlloc(&b, SLOTS * SLOT_BYTES, cudaHostAllocPortable) == cudaSuccess) return static_cast<char*>(b);
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return {static_cast<char*>(p), bytes};
     cudaGetLastError();  // else the next launch check reports this failure
-    return nullptr;
+    return {};
   }
-  void give(char* b) {
+  void give(Block b) {
     {
       std::lock_guard<std::mutex> lk(mu_);
-      if (free_.size() < KEEP) {
-        free_.push_back(b);
-        return;
-      }
+      free_.push_back(b);
     }
-    cudaFreeHost(b);
+    shrink(KEEP);
   }
 
  private:
+  // frees the smallest blocks until `keep` are left
+  void shrink(size_t keep) {
+    for (;;) {
+      Block b;
+      {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (free_.size() <= keep) return;
+        auto least = std::min_element(free_.begin(), free_.end(),
+                                      [](const Block& x, const Block& y) { return x.bytes < y.bytes; });
+        b = *least;
+        free_.erase(least);
+      }
+      cudaFreeHost(b.p);
+    }
+  }
   std::mutex mu_;
-  std::vector<char*> free_;
+  std::vector<Block> free_;
 };
 
 // One output of a readback: `width` consecutive values per cell.
@@ -92,18 +114,20 @@ void read_fields(int device, cudaStream_t s, StagePool& pool, int64_t n, const s
   if (per_cell == 0 || n == 0) return;
   const int64_t chunk = std::max<int64_t>(128, int64_t(StagePool::SLOT_BYTES / per_cell) / 128 * 128);
   const int64_t chunks = (n + chunk - 1) / chunk;
-  struct Held {
-    StagePool& pool;
-    char* p;
-    ~Held() {
-      if (p) pool.give(p);
-    }
-  } held{pool, pool.take()};
-  if (!held.p) check(cudaErrorMemoryAllocation);
   const int workers = int(std::min<int64_t>(
       std::min<int64_t>(chunks, StagePool::SLOTS), std::max<int64_t>(1, int64_t(std::thread::hardware_concurrency()))));
+  constexpr size_t STEP = size_t(64) << 10;
+  const size_t slot_bytes = (size_t(std::min(n, chunk)) * per_cell + STEP - 1) / STEP * STEP;
+  struct Held {
+    StagePool& pool;
+    StagePool::Block b;
+    ~Held() {
+      if (b.p) pool.give(b);
+    }
+  } held{pool, pool.take(size_t(workers) * slot_bytes)};
+  if (!held.b.p) check(cudaErrorMemoryAllocation);
   auto work = [&](int w) {
-    char* const slot = held.p + size_t(w) * StagePool::SLOT_BYTES;
+    char* const slot = held.b.p + size_t(w) * slot_bytes;
     check(cudaSetDevice(device));
     cudaEvent_t done = nullptr;
     check(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));

@@ -184,7 +184,18 @@ int main() {
     thrown = true;
   }
   std::printf("%d %d %d\n", thrown, fake_blocks.load(), fake_events.load());
-  char* const held = pool->take();  // the pool's block is in use, no other to be had
+  // blocks as large as their readback needs, the two largest kept, the
+  // smallest that fits taken
+  {
+    lbmb::StagePool::Block b[3] = {pool->take(100), pool->take(size_t(slot) * 4), pool->take(5000)};
+    for (auto x : b) pool->give(x);
+    auto fit = pool->take(200);
+    std::printf("%d %d %d\n", fake_blocks.load(), int(fit.bytes >= 200 && fit.bytes < size_t(slot) * 4),
+                int(pool->take(size_t(slot) * 4).p == b[1].p));
+    pool->give(fit);
+    pool->give(b[1]);
+  }
+  const auto held = pool->take(size_t(slot) * 4), held2 = pool->take(1);  // all in use, no other to be had
   fake_no_memory = true;
   thrown = false;
   try {
@@ -195,8 +206,14 @@ int main() {
   }
   std::printf("%d %d\n", thrown, cudaGetLastError());
   pool->give(held);
-  pool.reset();
+  pool->give(held2);
+  pool.reset();  // the last user: the largest block stays for the next one
+  fake_no_memory = false;
   std::printf("%d\n", fake_blocks.load());
+  pool = lbmb::StagePool::get();
+  const auto again = pool->take(size_t(slot) * 4);
+  std::printf("%d\n", fake_blocks.load());
+  pool->give(again);
 }
 """, "-pthread", "-I", str(tmp_path))
-    assert out.split() == "0 1 1 0 1 0 0".split()
+    assert out.split() == "0 1 2 0 2 1 1 1 0 1 1".split(), out
