@@ -109,15 +109,19 @@ __device__ __forceinline__ void ibm_target(const IbmArgs& a, int64_t m, double t
 // a load behind a branch per direction the Q loads of a cell follow each
 // other (19 x ~700 cycles in the direct forcing's first phase, measured with
 // the clock register; ~3,000 in all as one batch).
+// 32-bit offsets (Q x plane < 2^31): in 64 bits their registers halve the
+// blocks of a kernel of 27 directions (total mass of a 240^3 D3Q27 grid, the
+// whole call, 0.80 ms against 0.39).
 template <int Q>
-__device__ __forceinline__ int64_t post_stream_offset(int64_t pl, int64_t cell, const Nbr& nb, uint32_t mask, int q) {
+__device__ __forceinline__ uint32_t post_stream_offset(uint32_t pl, uint32_t cell, const Nbr& nb, uint32_t mask,
+                                                       int q) {
   using L = Lat<Q>;
   const int o = opp(q);
   const bool wall = (mask >> o) & 1u;
-  int64_t e = wall ? q * pl + cell : o * pl + nb.at(-L::cx(q), -L::cy(q), -L::cz(q));
+  uint32_t e = wall ? q * pl + cell : o * pl + uint32_t(nb.at(-L::cx(q), -L::cy(q), -L::cz(q)));
   if (slips_in<Q>(q)) {
     const bool slip = wall && (mask & NBR_SLIP) && !((mask >> planar<Q>(o)) & 1u);
-    e = slip ? opp(mirror_z<Q>(q)) * pl + nb.at(-L::cx(q), -L::cy(q), 0) : e;
+    e = slip ? opp(mirror_z<Q>(q)) * pl + uint32_t(nb.at(-L::cx(q), -L::cy(q), 0)) : e;
   }
   return e;
 }
@@ -135,7 +139,8 @@ __device__ __forceinline__ void load_post_stream(const S* fb, int64_t pl, int64_
   } else {
     const Nbr nb(x, y, z, nx, ny, nz);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) f[q] = Codec<S>::ld(fb + post_stream_offset<Q>(pl, cell, nb, mask, q));
+    for (int q = 0; q < Q; ++q)
+      f[q] = Codec<S>::ld(fb + post_stream_offset<Q>(uint32_t(pl), uint32_t(cell), nb, mask, q));
   }
 }
 
