@@ -1523,7 +1523,7 @@ struct Engine final : EngineBase {
     velocity_moments(u3);
     const StrainArgs<S> a = strain_args();
     read({{g9, 9}}, [&](const std::vector<double*>& d, int64_t c0, int64_t c1) {
-      wale_kernel<Q, S><<<unsigned(ceil_div(c1 - c0, 128)), 128, 0, st>>>(
+      wale_kernel<Q, S><<<unsigned(ceil_div(c1 - c0, WALE_BLOCK)), WALE_BLOCK, 0, st>>>(
           a, u3, wall_u.p, cfg.periodic[0], cfg.periodic[1], cfg.periodic[2], A(cfg.nu), 0, A(0), d[0], nullptr,
           nullptr, nullptr, nullptr, c0, c1);
       CK(cudaGetLastError());
@@ -1552,7 +1552,7 @@ struct Engine final : EngineBase {
     if (omega_dev.n != size_t(n)) omega_dev.alloc(size_t(n));
     const StrainArgs<S> a = strain_args();
     auto update = [&](double* nut, int64_t c0, int64_t c1) {
-      wale_kernel<Q, S><<<unsigned(ceil_div(c1 - c0, 128)), 128, 0, st>>>(
+      wale_kernel<Q, S><<<unsigned(ceil_div(c1 - c0, WALE_BLOCK)), WALE_BLOCK, 0, st>>>(
           a, u3, wall_u.p, cfg.periodic[0], cfg.periodic[1], cfg.periodic[2], nu0, clip ? 1 : 0, nu_t_max, nullptr,
           nut, omega_dev.p, cnt, cnt + 1, c0, c1);
       CK(cudaGetLastError());

@@ -241,23 +241,28 @@ __device__ __forceinline__ void vel_grad_cell(const StrainArgs<S>& a, const doub
 // nu_t_max when clip != 0; counts[0] = clipped cells, maxbits = bits of the
 // largest nu_t before clipping (non-negative, so integer order is value
 // order).
+constexpr int WALE_BLOCK = 128;
 template <int Q, class S>
-__global__ void wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typename Codec<S>::A>* wall_u, int per_x,
+__global__ void __launch_bounds__(WALE_BLOCK) wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typename Codec<S>::A>* wall_u, int per_x,
                             int per_y, int per_z, typename Codec<S>::A nu0, int clip,
                             typename Codec<S>::A nu_t_max, double* g9, double* nu_t, typename Codec<S>::A* omega,
                             unsigned long long* counts, unsigned long long* maxbits, int64_t c0, int64_t c1) {
   using A = typename Codec<S>::A;
-  const int64_t cell = c0 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (cell >= c1) return;
+  const int64_t first = c0 + int64_t(blockIdx.x) * WALE_BLOCK, cell = first + threadIdx.x;
   A g[3][3];
-  if (a.flags[cell] & F_SOLID) {
+  if (cell >= c1 || (a.flags[cell] & F_SOLID)) {
     for (int i = 0; i < 9; ++i) g[i / 3][i % 3] = A(0);
   } else {
     vel_grad_cell<Q, S>(a, u3, wall_u, per_x, per_y, per_z, cell, g);
   }
-  if (g9)
-    for (int i = 0; i < 9; ++i) g9[9 * (cell - c0) + i] = double(g[i / 3][i % 3]);
-  if (!omega) return;
+  if (g9) {  // through shared memory: consecutive threads write consecutive values over PCIe
+    __shared__ double sh[9 * WALE_BLOCK];
+    for (int i = 0; i < 9; ++i) sh[9 * threadIdx.x + i] = double(g[i / 3][i % 3]);
+    __syncthreads();
+    const int count = 9 * int(c1 - first < WALE_BLOCK ? c1 - first : WALE_BLOCK);
+    for (int i = threadIdx.x; i < count; i += WALE_BLOCK) g9[9 * (first - c0) + i] = sh[i];
+  }
+  if (!omega || cell >= c1) return;
   A sr[3][3], g2[3][3], sd[3][3];
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) sr[i][j] = A(0.5) * (g[i][j] + g[j][i]);
