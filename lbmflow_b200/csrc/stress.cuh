@@ -243,10 +243,11 @@ __device__ __forceinline__ void vel_grad_cell(const StrainArgs<S>& a, const doub
 // order).
 constexpr int WALE_BLOCK = 128;
 template <int Q, class S>
-__global__ void __launch_bounds__(WALE_BLOCK) wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typename Codec<S>::A>* wall_u, int per_x,
-                            int per_y, int per_z, typename Codec<S>::A nu0, int clip,
-                            typename Codec<S>::A nu_t_max, double* g9, double* nu_t, typename Codec<S>::A* omega,
-                            unsigned long long* counts, unsigned long long* maxbits, int64_t c0, int64_t c1) {
+__global__ void __launch_bounds__(WALE_BLOCK)
+    wale_kernel(StrainArgs<S> a, const double* u3, const Vec4<typename Codec<S>::A>* wall_u, int per_x, int per_y,
+                int per_z, typename Codec<S>::A nu0, int clip, typename Codec<S>::A nu_t_max, double* g9,
+                double* nu_t, typename Codec<S>::A* omega, unsigned long long* counts, unsigned long long* maxbits,
+                int64_t c0, int64_t c1) {
   using A = typename Codec<S>::A;
   const int64_t first = c0 + int64_t(blockIdx.x) * WALE_BLOCK, cell = first + threadIdx.x;
   A g[3][3];
